@@ -376,6 +376,13 @@ int rg_debug_ts_tables(const rg_params* p, const rg_snapshot* s, int n_hist, dou
 int rg_debug_ts_agn_tables(const rg_params* p, const rg_snapshot* s, int n_hist, double x_e_ave,
                            double collapse_fraction, int max_shells, double* agn, double* const_zp);
 
+/* The frequency tables as the device integrates them for rg_compute_Ts (rg_debug_ts_tables and
+   rg_debug_ts_agn_tables give the host engine's):
+     freq[3][3][14][nS]: band (galaxies, AGN soft, AGN hard) x kind (heat, ion, lya) per x_e node,
+                         zero for a band that is off. */
+int rg_debug_ts_device_tables(rg_context* ctx, const rg_params* p, const rg_snapshot* s, int n_hist, double x_e_ave,
+                              double collapse_fraction, int max_shells, double* freq);
+
 /* ---- allocation-free round trip (no counterpart in the reference) ----
    rg_debug_filter_roundtrip without a context and without any device allocation, for
    callers that cannot allocate: one that has given the device's memory to its own pool,

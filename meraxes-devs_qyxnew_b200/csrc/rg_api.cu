@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "rg_fft.cuh"
+#include "rg_freq.h"
 #include "rg_internal.h"
 #include "rg_xray.h"
 
@@ -300,6 +301,13 @@ int rg_create(int device, int grid_dim, rg_context** out) {
     rg_destroy(ctx);
     return RG_ECUDA;
   }
+  // the side stream's few blocks go ahead of the transforms' many
+  int prio_low = 0, prio_high = 0;
+  if (cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high) != cudaSuccess ||
+      cudaStreamCreateWithPriority(&ctx->side_stream, cudaStreamNonBlocking, prio_high) != cudaSuccess) {
+    rg_destroy(ctx);
+    return RG_ECUDA;
+  }
   if (cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
       ctx->num_sms < 1) {
     rg_destroy(ctx);
@@ -318,6 +326,13 @@ int rg_destroy(rg_context* ctx) {
   if (!ctx) return RG_EINVAL;
   cudaSetDevice(ctx->device);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+  if (ctx->side_stream) {
+    cudaStreamSynchronize(ctx->side_stream);
+    cudaStreamDestroy(ctx->side_stream);
+  }
+  if (ctx->freq_xint) cudaFree(ctx->freq_xint);
+  if (ctx->freq_d) cudaFree(ctx->freq_d);
+  if (ctx->freq_h) cudaFreeHost(ctx->freq_h);
   for (auto& e : ctx->twiddles) cudaFree(e.second);
   if (ctx->spec) cudaFree(ctx->spec);
   if (ctx->work) cudaFree(ctx->work);
@@ -824,6 +839,30 @@ int rg_debug_ts_tables(const rg_params* p, const rg_snapshot* s, int n_hist, dou
     shells[5 * nS + r] = freq ? tb.sum_lyn[r] : 0.0;
     for (int k = 0; k < sh.nsrc; ++k) coef[(size_t)r * sh.nsrc + k] = sh.coef[(size_t)r * sh.nsrc + k];
   }
+  return RG_OK;
+}
+
+int rg_debug_ts_device_tables(rg_context* ctx, const rg_params* p, const rg_snapshot* s, int n_hist, double x_e_ave,
+                              double collapse_fraction, int max_shells, double* freq) {
+  if (!ctx || !p || !s || !s->ZZ || !freq || n_hist < 0) return RG_EINVAL;
+  if (s->snapshot < 0 || s->snapshot >= s->n_snapshots) return RG_EINVAL;
+  const int nS = p->TsNumFilterSteps;
+  if (nS < 1 || nS > max_shells || (!s->stored_fcoll && s->snapshot > 0)) return RG_EINVAL;
+  if (p->Flag_IncludeAGNXray < 0 || p->Flag_IncludeAGNXray > 3) return RG_EINVAL;
+  TsShells sh = ts_shells(p, s->ZZ, s->n_snapshots, s->snapshot, n_hist);
+  if (sh.error) return set_error(ctx, RG_EINVAL, sh.msg);
+  cudaSetDevice(ctx->device);
+  int rc = ensure_tables(ctx, p);
+  if (rc) return rc;
+  TsTables tb;
+  const double zp = s->ZZ[s->snapshot];
+  if ((rc = ts_freq_start(ctx, p, sh, zp, x_e_ave, collapse_fraction, s->ZZ, s->stored_fcoll, s->snapshot))) return rc;
+  if ((rc = ts_freq_finish(ctx, p, sh, zp, &tb))) return rc;
+  const std::vector<double>* v[9] = {&tb.heat,      &tb.ion,       &tb.lya,       &tb.agn[0][0], &tb.agn[0][1],
+                                     &tb.agn[0][2], &tb.agn[1][0], &tb.agn[1][1], &tb.agn[1][2]};
+  const size_t per = (size_t)x_int_NXHII * nS;
+  for (int k = 0; k < 9; ++k)
+    for (size_t i = 0; i < per; ++i) freq[k * per + i] = v[k]->empty() ? 0.0 : (*v[k])[i];
   return RG_OK;
 }
 

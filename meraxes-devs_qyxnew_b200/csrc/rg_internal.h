@@ -251,6 +251,14 @@ struct rg_context {
   // host entry points: uploads and early downloads run on copy_stream, ordered by these events
   cudaStream_t copy_stream = nullptr;
   cudaStream_t copy_stream_out = nullptr;   // device-to-host copies that overlap later work
+  // ComputeTs: the frequency integrals run on a stream of their own, ahead of the transforms
+  cudaStream_t side_stream = nullptr;
+  float* freq_xint = nullptr;    // electron tables on the device, from tables.dir == freq_dir
+  std::string freq_dir;
+  double* freq_d = nullptr;      // shell redshifts, nu_tau_one and the tables; freq_h their pinned copy
+  size_t freq_d_elems = 0;
+  double* freq_h = nullptr;
+  size_t freq_h_elems = 0;
   std::vector<cudaEvent_t> stage_events;
   // profiling
   bool prof_on = false;

@@ -3,7 +3,7 @@
 //
 // Inhomogeneous branch, per snapshot:
 //   1. FP64 reductions of the collapse fraction and <x_e> (ComputeTs.c:585-677)
-//   2. host: frequency-integral tables, Lyman-n sums, prefactors (rg_xray.cpp)
+//   2. frequency-integral tables on a side stream (rg_freq.cu); host: Lyman-n sums, prefactors
 //   3. forward r2c of every source grid (this snapshot's sfr / xray_luminosity and the
 //      history slots the shells use); each shell's source is a linear combination of them
 //      (the history re-weighting of :366-478), formed in k-space on load
@@ -23,6 +23,7 @@
 #include <cstring>
 #include <vector>
 
+#include "rg_freq.h"
 #include "rg_internal.h"
 #include "rg_pass.cuh"
 #include "rg_tma.cuh"
@@ -995,6 +996,8 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
   if (!no_light) {
     if (!s->stored_fcoll && s->snapshot > 0)
       return set_error(ctx, RG_EINVAL, "ComputeTs needs stored_fcoll of the previous snapshot");
+    if ((rc = ts_freq_start(ctx, p, sh, zp, x_e_ave, collapse_fraction, s->ZZ, s->stored_fcoll, s->snapshot)))
+      return rc;
     // sources used by any shell
     std::vector<int> slot_of(sh.nsrc, -1), used;
     for (int r = 0; r < nS; ++r)
@@ -1108,12 +1111,9 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
         return rc;
     }
     if ((rc = kick())) return rc;
-    // the frequency tables on the host while the device runs the transforms above
+    // the frequency tables, integrated on the side stream during the transforms above
     TsTables tb;
-    std::string msg;
-    if ((rc = ts_tables(p, ctx->tables, sh, zp, x_e_ave, collapse_fraction, s->ZZ, s->stored_fcoll, s->snapshot, &tb,
-                        &msg)))
-      return set_error(ctx, rc, msg);
+    if ((rc = ts_freq_finish(ctx, p, sh, zp, &tb))) return rc;
 
     // per-shell coefficients.  evolveInt sums over shells R (XRayHeatingFunctions.c:1379-1432):
     //   heat/ion/lya: dt_dzpp dzpp XRAY_R (1+zpp)^-alpha fi_k(x_e)     (times const_zp later)

@@ -9,6 +9,7 @@
 
 #include "rg_gk61.h"
 #include "rg_internal.h"
+#include "rg_xphys.h"
 
 namespace rg {
 
@@ -270,74 +271,6 @@ double Cosmo::ddicke_dz(double z) const {
   return (dicke(z + dz) - dicke(z)) / dz;
 }
 
-// cross sections (XRayHeatingFunctions.c:471-516)
-double HeI_ion_crosssec(double nu) {
-  if (nu < HeI_NUIONIZATION) return 0;
-  const double x = nu / NU_over_EV / 13.61 - 0.4434;
-  const double y = std::sqrt(x * x + std::pow(2.136, 2));
-  return 9.492e-16 * ((x - 1) * (x - 1) + 2.039 * 2.039) * std::pow(y, (0.5 * 3.188 - 5.5)) *
-         std::pow(1.0 + std::sqrt(y / 1.469), -3.188);
-}
-
-double HeII_ion_crosssec(double nu) {
-  const double Z = 2;
-  if (nu < HeII_NUIONIZATION) return 0;
-  if (nu == HeII_NUIONIZATION) nu += TINY;
-  const double epsilon = std::sqrt(nu / HeII_NUIONIZATION - 1);
-  return (6.3e-18) / Z / Z * std::pow(HeII_NUIONIZATION / nu, 4) * std::exp(4 - (4 * std::atan(epsilon) / epsilon)) /
-         (1 - std::exp(-2 * M_PI / epsilon));
-}
-
-double HI_ion_crosssec(double nu) {
-  const double Z = 1;
-  if (nu < NUIONIZATION) return 0;
-  if (nu == NUIONIZATION) nu += TINY;
-  const double epsilon = std::sqrt(nu / NUIONIZATION - 1);
-  return SIGMA_HI / Z / Z * std::pow(NUIONIZATION / nu, 4) * std::exp(4 - (4 * std::atan(epsilon) / epsilon)) /
-         (1 - std::exp(-2 * M_PI / epsilon));
-}
-
-// electron interpolation tables (XRayHeatingFunctions.c:970-1276), float arithmetic as in the C
-static int locate_energy_index(float En) {
-  if (En < 1008.88f) return (int)(std::log((double)En / 10.0) / 1.98026273e-2);
-  return 232 + (int)(std::log((double)En / 1008.88) / 9.53101798e-2);
-}
-
-int locate_xHII_index(const Tables& t, float xHII_call) {
-  int m = x_int_NXHII - 1;
-  while (xHII_call < t.x_int_XHII[m]) m--;
-  return m;
-}
-
-float interp_x_int(const Tables& t, const std::vector<float>& tab, float En, float xHII_call, float below) {
-  const float* E = t.x_int_Energy.data();
-  const float* X = t.x_int_XHII.data();
-  if ((double)En > 0.999 * (double)E[x_int_NENERGY - 1]) {
-    En = (float)((double)E[x_int_NENERGY - 1] * 0.999);
-  } else if (En < E[0]) {
-    return below;
-  }
-  if ((double)xHII_call > (double)X[x_int_NXHII - 1] * 0.999) {
-    xHII_call = (float)((double)X[x_int_NXHII - 1] * 0.999);
-  } else if (xHII_call < X[0]) {
-    xHII_call = (float)(1.001 * (double)X[0]);
-  }
-  const int n_low = locate_energy_index(En), n_high = n_low + 1;
-  const int m_low = locate_xHII_index(t, xHII_call), m_high = m_low + 1;
-  const float* lo = tab.data() + (size_t)m_low * x_int_NENERGY;
-  const float* hi = tab.data() + (size_t)m_high * x_int_NENERGY;
-  float elow = ((lo[n_high] - lo[n_low]) / (E[n_high] - E[n_low]));
-  elow *= (En - E[n_low]);
-  elow += lo[n_low];
-  float ehigh = ((hi[n_high] - hi[n_low]) / (E[n_high] - E[n_low]));
-  ehigh *= (En - E[n_low]);
-  ehigh += hi[n_low];
-  float r = (ehigh - elow) / (X[m_high] - X[m_low]);
-  r *= (xHII_call - X[m_low]);
-  r += elow;
-  return r;
-}
-
 float zmax(float z, int n) {
   const double num = 1 - std::pow(n + 1, -2);
   const double denom = 1 - std::pow(n, -2);
@@ -501,7 +434,6 @@ int ts_tables(const rg_params* p, const Tables& t, const TsShells& sh, double zp
   out->heat.assign((size_t)x_int_NXHII * nS, 0);
   out->ion.assign((size_t)x_int_NXHII * nS, 0);
   out->lya.assign((size_t)x_int_NXHII * nS, 0);
-  out->sum_lyn.assign(nS, 0);
   const double ion_eff = p->ReionEfficiency;
   // interpolate_fcoll (XRayHeatingFunctions.c:2010-2026); stored_fcoll[snapshot] is this step's
   auto fcoll_at = [&](double redshift) {
@@ -542,45 +474,14 @@ int ts_tables(const rg_params* p, const Tables& t, const TsShells& sh, double zp
                       0.02, 100, &st);
   };
   const double thresh = p->NuXrayThreshold;
+  const XInt xi{t.x_int_Energy.data(), t.x_int_XHII.data(), t.fheat.data(), t.n_Lya.data(), t.nion_HI.data(),
+                t.nion_HeI.data(), t.nion_HeII.data()};
   // integrate_over_nu (XRayHeatingFunctions.c:742-856) for the spectral index alpha
   auto integrate_over_nu = [&](double local_x_e, double lo, double hi, int FLAG, double alpha) {
     if (lo >= hi) return 0.0;
-    const float xf = (float)local_x_e;
-    auto pw = [&](double nu) { return std::pow(nu / (thresh * NU_over_EV), -alpha - 1); };
-    std::function<double(double)> f;
-    if (FLAG == 0) {
-      f = [&](double nu) {
-        double s = interp_x_int(t, t.fheat, (float)((nu - NUIONIZATION) / NU_over_EV), xf, 1.0f) * PLANCK *
-                   (nu - NUIONIZATION) * cm.f_H * (1 - local_x_e) * HI_ion_crosssec(nu);
-        s += interp_x_int(t, t.fheat, (float)((nu - HeI_NUIONIZATION) / NU_over_EV), xf, 1.0f) * PLANCK *
-             (nu - HeI_NUIONIZATION) * cm.f_He * (1 - local_x_e) * HeI_ion_crosssec(nu);
-        s += interp_x_int(t, t.fheat, (float)((nu - HeII_NUIONIZATION) / NU_over_EV), xf, 1.0f) * PLANCK *
-             (nu - HeII_NUIONIZATION) * cm.f_He * local_x_e * HeII_ion_crosssec(nu);
-        return s * pw(nu);
-      };
-    } else if (FLAG == 1) {
-      f = [&](double nu) {
-        auto Fi = [&](double e0) {
-          const float en = (float)((nu - e0) / NU_over_EV);
-          return interp_x_int(t, t.nion_HI, en, xf, 0.0f) + interp_x_int(t, t.nion_HeI, en, xf, 0.0f) +
-                 interp_x_int(t, t.nion_HeII, en, xf, 0.0f) + 1;
-        };
-        double s = Fi(NUIONIZATION) * cm.f_H * (1 - local_x_e) * HI_ion_crosssec(nu);
-        s += Fi(HeI_NUIONIZATION) * cm.f_He * (1 - local_x_e) * HeI_ion_crosssec(nu);
-        s += Fi(HeII_NUIONIZATION) * cm.f_He * local_x_e * HeII_ion_crosssec(nu);
-        return s * pw(nu);
-      };
-    } else {
-      f = [&](double nu) {
-        double s = interp_x_int(t, t.n_Lya, (float)((nu - NUIONIZATION) / NU_over_EV), xf, 0.0f) * cm.f_H *
-                   (1 - local_x_e) * HI_ion_crosssec(nu);
-        s += interp_x_int(t, t.n_Lya, (float)((nu - HeI_NUIONIZATION) / NU_over_EV), xf, 0.0f) * cm.f_He *
-             (1 - local_x_e) * HeI_ion_crosssec(nu);
-        s += interp_x_int(t, t.n_Lya, (float)((nu - HeII_NUIONIZATION) / NU_over_EV), xf, 0.0f) * cm.f_He *
-             local_x_e * HeII_ion_crosssec(nu);
-        return s * pw(nu);
-      };
-    }
+    auto f = [&](double nu) {
+      return xray_integrand(xi, cm.f_H, cm.f_He, FLAG, local_x_e, alpha, thresh * NU_over_EV, nu);
+    };
     double result, error;
     const int status = qag61(f, lo, hi, 0, 0.01, 1000, &result, &error);
     if (status != 0) return 0.0;
@@ -641,7 +542,19 @@ int ts_tables(const rg_params* p, const Tables& t, const TsShells& sh, double zp
   out->nu_tau_one_min = *std::min_element(ntone.begin(), ntone.end());
   out->nu_tau_one_max = *std::max_element(ntone.begin(), ntone.end());
 
-  // Lyman-n sums with the kink correction (ComputeTs.c:900-1011), in shell order
+  ts_sum_lyn(t, p, sh, zp, &out->sum_lyn);
+  (void)msg;
+  return RG_OK;
+}
+
+void ts_sum_lyn(const Tables& t, const rg_params* p, const TsShells& sh, double zp, std::vector<double>* sum) {
+  const Cosmo cm(p);
+  const int nS = sh.nS;
+  std::vector<double>& sum_lyn = *sum;
+  sum_lyn.assign(nS, 0);
+  float zm[NSPEC_MAX + 1];   // zmax(zp, n)
+  for (int n_ct = 2; n_ct <= NSPEC_MAX; n_ct++) zm[n_ct] = zmax((float)zp, n_ct);
+  // in shell order
   bool first_radii = true, first_zero = true;
   // the C reuses the history weight variable: without a crossing in the trial loop the
   // correction multiplies by the weight the history loop left behind
@@ -651,13 +564,13 @@ int ts_tables(const rg_params* p, const Tables& t, const TsShells& sh, double zp
     const double prev_zpp = R_ct == 0 ? zp : sh.zpp_edge[R_ct - 1];
     const double prev_R = R_ct == 0 ? 0 : sh.R[R_ct - 1];
     const double zpp = (sh.zpp_edge[R_ct] + prev_zpp) * 0.5;
-    out->sum_lyn[R_ct] = 0;
+    sum_lyn[R_ct] = 0;
     for (int n_ct = NSPEC_MAX; n_ct >= 2; n_ct--) {
-      if (zpp > zmax((float)zp, n_ct)) continue;
+      if (zpp > zm[n_ct]) continue;
       const double nuprime = nu_n(n_ct) * (1 + zpp) / (1.0 + zp);
-      out->sum_lyn[R_ct] += frecycle(n_ct) * spectral_emissivity(t, nuprime);
+      sum_lyn[R_ct] += frecycle(n_ct) * spectral_emissivity(t, nuprime);
     }
-    if (R_ct > 2 && out->sum_lyn[R_ct] == 0.0 && out->sum_lyn[R_ct - 1] > 0. && first_radii) {
+    if (R_ct > 2 && sum_lyn[R_ct] == 0.0 && sum_lyn[R_ct - 1] > 0. && first_radii) {
       const double trial_zpp_max = (prev_zpp - (sh.R[R_ct] - prev_R) * MPC / cm.drdz((float)prev_zpp) + prev_zpp) * 0.5;
       const double trial_zpp_min =
           (sh.zpp_edge[R_ct - 2] - (sh.R[R_ct - 1] - sh.R[R_ct - 2]) * MPC / cm.drdz((float)sh.zpp_edge[R_ct - 2]) +
@@ -668,7 +581,7 @@ int ts_tables(const rg_params* p, const Tables& t, const TsShells& sh, double zp
             trial_zpp_min + (trial_zpp_max - trial_zpp_min) * (float)ii / ((float)n_pts_radii - 1.);
         int counter = 0;
         for (int n_ct = NSPEC_MAX; n_ct >= 2; n_ct--) {
-          if (trial_zpp > zmax((float)zp, n_ct)) continue;
+          if (trial_zpp > zm[n_ct]) continue;
           counter += 1;
         }
         if (counter == 0 && first_zero) {
@@ -676,12 +589,10 @@ int ts_tables(const rg_params* p, const Tables& t, const TsShells& sh, double zp
           weight = (float)ii / (float)n_pts_radii;
         }
       }
-      out->sum_lyn[R_ct] = weight * out->sum_lyn[R_ct - 1];
+      sum_lyn[R_ct] = weight * sum_lyn[R_ct - 1];
       first_radii = false;
     }
   }
-  (void)msg;
-  return RG_OK;
 }
 
 TsPrefactors ts_prefactors(const rg_params* p, double zp) {

@@ -35,11 +35,6 @@ struct Cosmo {
   double ddicke_dz(double z) const;
 };
 
-double HI_ion_crosssec(double nu);
-double HeI_ion_crosssec(double nu);
-double HeII_ion_crosssec(double nu);
-float interp_x_int(const Tables& t, const std::vector<float>& tab, float En, float xHII_call, float below);
-int locate_xHII_index(const Tables& t, float xHII_call);
 float zmax(float z, int n);
 double nu_n(int n);
 double frecycle(int n);
@@ -75,6 +70,9 @@ struct TsTables {
 int ts_tables(const rg_params* p, const Tables& t, const TsShells& sh, double zp, double x_e_ave,
               double collapse_fraction, const double* ZZ, const double* stored_fcoll, int snapshot, TsTables* out,
               std::string* msg);
+
+// The Lyman-n sums of the shells with the kink correction (ComputeTs.c:900-1011).
+void ts_sum_lyn(const Tables& t, const rg_params* p, const TsShells& sh, double zp, std::vector<double>* sum_lyn);
 
 // Per-snapshot prefactors (ComputeTs.c:1014-1109)
 struct TsPrefactors {

@@ -150,6 +150,8 @@ _SIGS = {
                                      C.c_void_p, C.c_void_p, C.c_void_p]),
     "rg_debug_ts_agn_tables": (C.c_int, [_P(rg_params), _P(rg_snapshot), C.c_int, C.c_double, C.c_double, C.c_int,
                                          C.c_void_p, C.c_void_p]),
+    "rg_debug_ts_device_tables": (C.c_int, [C.c_void_p, _P(rg_params), _P(rg_snapshot), C.c_int, C.c_double,
+                                            C.c_double, C.c_int, C.c_void_p]),
     "rg_filter_roundtrip_noalloc": (C.c_int, [_P(rg_params), C.c_void_p, C.c_void_p, C.c_double, C.c_int,
                                               C.c_void_p, C.c_char_p, C.c_size_t]),
 }
