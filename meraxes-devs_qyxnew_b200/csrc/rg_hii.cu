@@ -654,9 +654,9 @@ int launch_forward(rg_context* ctx, const float* const* d_real, int ng, cf* spec
   prof_begin(ctx, "fwd_y_c2c", st);
   RG_CUDA_TRY(ctx, (launch_pass_y<N, false>(spec, stride, ng, tw, st)));
   prof_end(ctx, ng * 16.0 * nzc, st);
-  RG_CUDA_TRY(ctx, prep(k_pass_x_fwd<N>, smem_x<N>()));
+  RG_CUDA_TRY(ctx, prep((k_pass_x<N, false>), smem_x<N>()));
   prof_begin(ctx, "fwd_x_c2c", st);
-  k_pass_x_fwd<N><<<dim3(N / C::BX, C::NZ, ng), C::T * C::BX, smem_x<N>(), st>>>(spec, stride, tw, (float)scale);
+  k_pass_x<N, false><<<dim3(N / C::BX, C::NZ, ng), C::T * C::BX, smem_x<N>(), st>>>(spec, stride, tw, (float)scale);
   prof_end(ctx, ng * 16.0 * nzc, st);
   RG_CUDA_TRY(ctx, cudaGetLastError());
   return RG_OK;

@@ -148,7 +148,7 @@ cudaError_t na_roundtrip(unsigned char* base, const float* in, float* out, doubl
   srcs.p[0] = in;
   k_fwd_z<N><<<dim3(N / (2 * ZFCfg<N>::QF), N, 1), ZFCfg<N>::NTH, na_smem_fz<N>(), st>>>(srcs, spec, nc, tw);
   k_pass_y<N, false><<<dim3(N / YCfg<N>::BY, C::NZ, 1), YCfg<N>::NTH, na_smem_y<N>(), st>>>(spec, nc, tw);
-  k_pass_x_fwd<N><<<dim3(N / C::BX, C::NZ, 1), C::T * C::BX, na_smem_x<N>(), st>>>(
+  k_pass_x<N, false><<<dim3(N / C::BX, C::NZ, 1), C::T * C::BX, na_smem_x<N>(), st>>>(
       spec, nc, tw, (float)(1.0 / ((double)N * N * N)));
   // filter_type < 0: the window is 1 everywhere (no filter)
   k_na_inv_x<N><<<dim3(N / C::BX, C::NZ), C::T * C::BX, na_smem_x<N>(), st>>>(spec, work, tw, 2.0 * M_PI / box, R,

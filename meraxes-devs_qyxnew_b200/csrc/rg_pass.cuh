@@ -4,7 +4,7 @@
 //   k_fwd_z     : r2c along z of padded real grids, two neighbouring rows per complex line,
 //                 split into the two Hermitian halves in shared memory, stored as S[kz][x][y]
 //   k_pass_y    : c2c along y (contiguous lines), in place, over a run of equally spaced grids
-//   k_pass_x_fwd: c2c along x (lines of stride N), in place, scaled on store
+//   k_pass_x    : c2c along x (lines of stride N), in place, scaled on store
 //   zfront      : c2r along z of NG grids for a block of rows; two neighbouring rows of one grid
 //                 share a complex line; the real rows land in shared memory for an epilogue
 //
@@ -224,10 +224,10 @@ inline cudaError_t launch_pass_y(cf* base, size_t stride, int ng, const cf* tw, 
   return cudaGetLastError();
 }
 
-// forward x pass over grids base + z * stride, in place, scaled on store
-template <int N>
+// x pass over grids base + z * stride, in place, scaled on store
+template <int N, bool INV>
 __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::BX, RG_MINB(Cfg<N>::T* Cfg<N>::BX))
-    k_pass_x_fwd(cf* __restrict__ base, size_t stride, const cf* __restrict__ g_tw, float scale) {
+    k_pass_x(cf* __restrict__ base, size_t stride, const cf* __restrict__ g_tw, float scale) {
   constexpr int T = Cfg<N>::T, B = Cfg<N>::BX;
   extern __shared__ cf smem[];
   cf* s_tw = smem;
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::BX, RG_MINB(Cfg<N>::T* Cfg<
   const size_t col = (size_t)kz * N * N + blockIdx.x * B + b;
   load_twiddles<N>(s_tw, g_tw);
   __syncthreads();
-  line_fft<N, false>(
+  line_fft<N, INV>(
       t, xbuf, s_tw, [&](int p, int) { return g[col + (size_t)p * N]; }, [&](int p) { return line_addr<N, B>(p, b); },
       [&](int p, cf v) { g[col + (size_t)p * N] = cf{v.x * scale, v.y * scale}; });
 }

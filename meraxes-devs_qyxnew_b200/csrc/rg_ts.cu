@@ -11,7 +11,12 @@
 //      that turns the grids of every shell (sfr, X-ray, then the AGN soft and / or hard
 //      emissivity) into the four per-cell sums of
 //      evolveInt (X-ray heating, ionisation and Lyman-alpha integrands, stellar Lyman-alpha)
-//      without storing the reference's SMOOTHED_*[nS N^3] arrays
+//      without storing the reference's SMOOTHED_*[nS N^3] arrays.
+//      The X-ray sums are linear in the filtered X-ray grids (they are not clamped) and piecewise
+//      linear in the cell's x_e, so with x_e on few table nodes they are formed in k-space, one
+//      field per node and kind (k_ts_nodes), instead of one X-ray transform per shell.
+//      With the sharp-k window the modes beyond a shell's cut are zero: the x pass skips their
+//      columns, the y pass their lines, and the z pass does not read their planes.
 //   5. per cell, FP64: evolveInt, the Euler step of x_e and T_K, get_Ts, and the FP64 sums
 // Homogeneous branch (zp >= ReionMaxHeatingRedshift): RECFAST x_e and T_K, get_Ts with no
 // Lyman-alpha coupling (:252-331).
@@ -27,6 +32,7 @@
 #include "rg_internal.h"
 #include "rg_pass.cuh"
 #include "rg_tma.cuh"
+#include "rg_xphys.h"
 #include "rg_xray.h"
 
 namespace rg {
@@ -174,13 +180,27 @@ __device__ __forceinline__ void block_sum_dyn(double (&acc)[K], double* out) {
   }
 }
 
-// collapse fraction and <x_e> over the box (ComputeTs.c:585-677)
+// floats as unsigned integers of the same order (and back, on the host)
+__device__ __forceinline__ unsigned float_order(float v) {
+  const unsigned b = __float_as_uint(v);
+  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+static float float_of_order(unsigned o) {
+  const unsigned b = (o & 0x80000000u) ? (o & 0x7fffffffu) : ~o;
+  float v;
+  std::memcpy(&v, &b, sizeof(v));
+  return v;
+}
+
+// collapse fraction, <x_e> and the range of x_e over the box (ComputeTs.c:585-677)
 __global__ void __launch_bounds__(256) k_ts_reduce0(const float* __restrict__ stars, const float* __restrict__ deltax,
                                                     const float* __restrict__ xe, int n, double Mh2,
-                                                    double fourthirds_pi_R3_over_pv, double* partials) {
+                                                    double fourthirds_pi_R3_over_pv, double* partials,
+                                                    unsigned* __restrict__ xe_range) {
   const int padw = 2 * (n / 2 + 1);
   const size_t rows = (size_t)n * n;
   double acc[2] = {0.0, 0.0};
+  unsigned lo = ~0u, hi = 0u;   // range of x_e as ordered integers
   for (size_t row = blockIdx.x; row < rows; row += gridDim.x)
     for (int z = threadIdx.x; z < n; z += blockDim.x) {
       const size_t ip = row * padw + z;
@@ -188,9 +208,30 @@ __global__ void __launch_bounds__(256) k_ts_reduce0(const float* __restrict__ st
       double c = (double)stars[ip] / (Mh2 * density_over_mean) * fourthirds_pi_R3_over_pv;
       if (c > 1.0) c = 1.0;
       acc[0] += c;
-      acc[1] += (double)xe[ip];
+      const float v = xe[ip];
+      acc[1] += (double)v;
+      const unsigned o = float_order(v);
+      lo = min(lo, o);
+      hi = max(hi, o);
     }
   block_sum_dyn<2>(acc, partials + (size_t)blockIdx.x * 2);
+  __shared__ unsigned s_lo, s_hi;
+  if (threadIdx.x == 0) {
+    s_lo = ~0u;
+    s_hi = 0u;
+  }
+  __syncthreads();
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  if ((threadIdx.x & 31) == 0) {
+    atomicMin(&s_lo, lo);
+    atomicMax(&s_hi, hi);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    atomicMin(xe_range, s_lo);
+    atomicMax(xe_range + 1, s_hi);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -203,13 +244,19 @@ struct TsBatch {
   float cs[TS_KB][TS_MAXSRC];
   int filtered[TS_KB];
   int wrow[TS_KB];
-  int ng;             // grids per shell: sfr, X-ray, then 0 to 2 AGN bands
+  int cut[TS_KB];     // last n2 that the shell's window keeps (TS_NOCUT: all)
+  int gs;             // grids per source: sfr, X-ray, then 0 to 2 AGN bands
+  int ng;             // grids per shell: the same, without X-ray where that goes by nodes
+  int skip;           // 1: X-ray goes by nodes
 };
+constexpr int TS_NOCUT = 0x7fffffff;
 
+// Columns beyond a shell's cut hold zeros, which the y pass knows: they are neither read nor written.
+// At 512^3 with 40 sharp-k shells the shells' volumes add up to 4 grids of 40 and their columns to 6.
 template <int N>
 __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::BX, (x_pass_minb<N>()))
     k_ts_x(const cf* __restrict__ spec, size_t stride, cf* __restrict__ work, TsBatch bt,
-           const float* __restrict__ wtab, int wpitch, const int* __restrict__ wcut, const cf* __restrict__ g_tw) {
+           const float* __restrict__ wtab, int wpitch, const cf* __restrict__ g_tw) {
   constexpr int T = Cfg<N>::T, B = Cfg<N>::BX, V = Cfg<N>::V;
   extern __shared__ cf smem[];
   cf* s_tw = smem;
@@ -218,6 +265,10 @@ __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::BX, (x_pass_minb<N>()))
   const int b = threadIdx.x % B, t = threadIdx.x / B;
   const int y = blockIdx.x * B + b;
   const size_t col = (size_t)kz * N * N + y;
+  // the least n2 of the block's columns (|ny| is least at one of its ends)
+  const int ya = blockIdx.x * B, yb = ya + B - 1;
+  const int na = ya > N / 2 ? N - ya : ya, nb = yb > N / 2 ? N - yb : yb;
+  const int n2min = kz * kz + min(na, nb) * min(na, nb);
   load_twiddles<N>(s_tw, g_tw);
   int n2[V];
   const int ny = y > N / 2 ? y - N : y;
@@ -229,26 +280,21 @@ __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::BX, (x_pass_minb<N>()))
   }
   __syncthreads();
   for (int r = 0; r < bt.nr; ++r) {
+    const int cut = bt.cut[r];
+    if (n2min > cut) continue;
     float wv[V];
-    if (!bt.filtered[r]) {
+    if (!bt.filtered[r] || cut != TS_NOCUT) {
 #pragma unroll
-      for (int sl = 0; sl < V; ++sl) wv[sl] = 1.f;
+      for (int sl = 0; sl < V; ++sl) wv[sl] = 1.f;   // sharp-k: the modes beyond the cut are not loaded
     } else {
-      if (wcut) {
-        // sharp-k: the row is the step W = (n2 <= cut), no gathers
-        const int cut = __ldg(wcut + bt.wrow[r]);
+      const float* wr = wtab + (size_t)bt.wrow[r] * wpitch;
 #pragma unroll
-        for (int sl = 0; sl < V; ++sl) wv[sl] = n2[sl] <= cut ? 1.f : 0.f;
-      } else {
-        const float* wr = wtab + (size_t)bt.wrow[r] * wpitch;
-#pragma unroll
-        for (int sl = 0; sl < V; ++sl) wv[sl] = __ldg(wr + n2[sl]);
-      }
+      for (int sl = 0; sl < V; ++sl) wv[sl] = __ldg(wr + n2[sl]);
     }
     const int nk = bt.nk[r];
-    const int G = bt.ng;
-    for (int g = 0; g < G; ++g) {
-      cf* dst = work + ((size_t)r * G + g) * stride;
+    for (int g = 0; g < bt.ng; ++g) {
+      const int gsrc = g > 0 ? g + bt.skip : 0;
+      cf* dst = work + ((size_t)r * bt.ng + g) * stride;
       // the combination sum_i c_i spec_i of this thread's V input positions, source by source:
       // the V loads of a source are independent and in flight together (per element the same
       // fmaf sequence in the order of i)
@@ -257,10 +303,11 @@ __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::BX, (x_pass_minb<N>()))
       for (int sl = 0; sl < V; ++sl) in[sl] = cf{0.f, 0.f};
       for (int i = 0; i < nk; ++i) {
         const float c = bt.cs[r][i];
-        const cf* src = spec + ((size_t)bt.ks[r][i] * G + g) * stride + col;
+        const cf* src = spec + ((size_t)bt.ks[r][i] * bt.gs + gsrc) * stride + col;
         cf v[V];
 #pragma unroll
-        for (int sl = 0; sl < V; ++sl) v[sl] = src[(size_t)stage0_pos<N>(t, sl) * N];
+        for (int sl = 0; sl < V; ++sl)
+          v[sl] = n2[sl] <= cut ? src[(size_t)stage0_pos<N>(t, sl) * N] : cf{0.f, 0.f};
 #pragma unroll
         for (int sl = 0; sl < V; ++sl) {
           in[sl].x = fmaf(c, v[sl].x, in[sl].x);
@@ -271,6 +318,96 @@ __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::BX, (x_pass_minb<N>()))
           t, xbuf, s_tw, [&](int, int sl) { return cf{in[sl].x * wv[sl], in[sl].y * wv[sl]}; },
           [&](int p) { return line_addr<N, B>(p, b); }, [&](int p, cf v) { dst[col + (size_t)p * N] = v; });
     }
+  }
+}
+
+// shell y pass, in place: the columns beyond the cut are zero (the x pass left them unwritten), the
+// planes beyond it are not transformed (the z pass does not read them); gridDim.y covers the
+// batch's planes.  blockIdx.z: shell r, grid g at work + (r ng + g) stride.
+template <int N>
+__global__ void __launch_bounds__(YCfg<N>::NTH, RG_MINB(YCfg<N>::NTH))
+    k_ts_y(cf* __restrict__ work, size_t stride, TsBatch bt, const cf* __restrict__ g_tw) {
+  using Y = YCfg<N>;
+  using PL = typename Y::PL;
+  constexpr int T = Y::T, B = Y::BY;
+  extern __shared__ cf smem[];
+  cf* s_tw = smem;
+  cf* xbuf = smem + N;
+  const int kz = blockIdx.y;
+  const int left = bt.cut[blockIdx.z / bt.ng] - kz * kz;   // ny^2 up to this
+  if (left < 0) return;
+  const int t = threadIdx.x % T, b = threadIdx.x / T;
+  load_twiddles_p<PL>(s_tw, g_tw);
+  __syncthreads();
+  cf* line = work + blockIdx.z * stride + ((size_t)kz * N + blockIdx.x * B + b) * N;
+  line_fft_p<PL, true, true>(
+      t, xbuf, s_tw,
+      [&](int p, int) {
+        const int ny = p > N / 2 ? N - p : p;
+        return ny * ny <= left ? line[p] : cf{0.f, 0.f};
+      },
+      [&](int p) { return pos_addr<N>(b, p); }, [&](int p, cf v, int) { line[p] = v; });
+}
+
+// ---------------------------------------------------------------------------
+// X-ray by nodes: the cell's heating, ionisation and Lyman-alpha sums
+//   sum_r xray_r(cell) (P_rk[lo] + (x_e - X[lo]) Q_rk[lo])
+// are linear in the filtered grids xray_r and, between the table's x_e nodes X[m], linear in x_e:
+//   (1 - t) F_k[lo] + t F_k[lo + 1],  F_k[m] = sum_r f_rk(X[m]) xray_r,  t = (x_e - X[lo]) / (X[lo + 1] - X[lo])
+// so the sum over shells is taken in k-space, once per node that the box uses.  3 M transforms
+// instead of nS (M nodes: two where the whole box lies between neighbouring nodes).  At 512^3, 5
+// nodes and 40 shells, with the sharp-k pruning, ComputeTs went from 76.9 to 47.0 ms; at 256^3, 9
+// nodes, from 8.4 to 6.9 ms.
+
+struct TsNodeShell {
+  int nk;                    // sources of the shell
+  int filtered, cut;         // as in TsBatch
+  int ks[TS_MAXSRC];
+  float cs[TS_MAXSRC];
+  float f[3 * x_int_NXHII];  // coefficient of field 3 j + kind, node m0 + j
+};
+
+// fields [f0, f0 + NF) of nf (f0 = blockIdx.y NF): work[f] = sum_r f_r W_r sum_i c_i spec[k_i][1].
+// One mode a thread; the shells' coefficients are the same for the whole block (read through L1),
+// as are mostly the shells that a warp's modes pass.
+template <int NF>
+__global__ void __launch_bounds__(256) k_ts_nodes(const cf* __restrict__ spec, size_t stride, int gs,
+                                                  cf* __restrict__ work, const TsNodeShell* __restrict__ shells, int nS,
+                                                  int nf, const float* __restrict__ wtab, int wpitch, int log2n) {
+  const int n = 1 << log2n, f0 = blockIdx.y * NF;
+  for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < stride; i += (size_t)gridDim.x * 256) {
+    const int y = (int)(i & (n - 1)), x = (int)((i >> log2n) & (n - 1)), kz = (int)(i >> (2 * log2n));
+    const int ny = y > n / 2 ? y - n : y, nx = x > n / 2 ? x - n : x;
+    const int n2 = nx * nx + ny * ny + kz * kz;
+    cf acc[NF];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) acc[f] = cf{0.f, 0.f};
+    for (int r = 0; r < nS; ++r) {
+      const TsNodeShell& s = shells[r];
+      const int cut = s.cut;
+      if (n2 > cut) continue;
+      cf v{0.f, 0.f};
+      const int nk = s.nk;
+      for (int j = 0; j < nk; ++j) {
+        const float2 a = __ldg(reinterpret_cast<const float2*>(spec + ((size_t)s.ks[j] * gs + 1) * stride + i));
+        v.x = fmaf(s.cs[j], a.x, v.x);
+        v.y = fmaf(s.cs[j], a.y, v.y);
+      }
+      if (s.filtered && cut == TS_NOCUT) {
+        const float w = __ldg(wtab + (size_t)r * wpitch + n2);
+        v.x *= w;
+        v.y *= w;
+      }
+#pragma unroll
+      for (int f = 0; f < NF; ++f) {
+        const float c = s.f[f0 + f];
+        acc[f].x = fmaf(c, v.x, acc[f].x);
+        acc[f].y = fmaf(c, v.y, acc[f].y);
+      }
+    }
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+      if (f0 + f < nf) work[(size_t)(f0 + f) * stride + i] = acc[f];
   }
 }
 
@@ -350,7 +487,8 @@ struct TsShellCoef {
   float P[3][x_int_NXHII];
   float Q[3][x_int_NXHII];
   float cstar;
-  float pad;
+  int kzmax;    // the shell's planes beyond this are zero (and not written)
+  float dX[x_int_NXHII];   // widths of the node intervals
   // AGN units j = 0, 1 (the bands in use, soft first): max(grid, 0) x (PA + dx QA), with the
   // ratio of the band's prefactor to the galaxies' folded in so the terms join the same sums
   float PA[2][3][x_int_NXHII];
@@ -359,6 +497,7 @@ struct TsShellCoef {
 
 struct TsZev {
   int nS;
+  int m0, nm;                     // X-ray by nodes: the nodes m0 .. m0 + nm - 1 (nm 0: by shells)
   float X[x_int_NXHII];           // x_int_XHII (float, as in the reference)
   double inv_scale[4];            // undo the FP32 scaling
 };
@@ -373,49 +512,53 @@ struct TsZ {
   static constexpr int NTH = T * Q;
   static constexpr int MINB = NTH >= 512 ? 1 : 512 / NTH;   // 2 blocks of 256: at most 128 registers
   static constexpr int NZ = N / 2 + 1;
-  // kz rows per tensor box (at most 256): one box, or for N = 512 two of (NZ + 1) / 2 rows at kz 0
-  // and NZ - KZB that overlap in one row, so the second lands on a 128-byte boundary
-  static constexpr int KZB = NZ <= 256 ? NZ : (NZ + 1) / 2;
-  static constexpr int NBOX = NZ <= 256 ? 1 : 2;
+  // A shell's rows come as up to NBOX tensor boxes of KZS + 1 kz rows, KZS apart (they overlap in one
+  // row, so every box lands on a 128-byte boundary and none leaves the spectrum): as many as the
+  // shell's cut needs
+  static constexpr int NBOX = N >= 64 ? 8 : 1;
+  static constexpr int KZS = (N / 2) / NBOX;
   static constexpr int TS = round_up(NZ * Q, 16);            // one shell's rows, a 128-byte multiple
   static constexpr size_t tile_elems() { return (size_t)2 * TS; }   // two shells' rows
-  static constexpr uint32_t SHELL_TX = (uint32_t)(NBOX * KZB * Q * sizeof(cf));
+  static constexpr uint32_t BOX_TX = (uint32_t)((KZS + 1) * Q * sizeof(cf));
   static constexpr int STAGES = 3;           // tiles in flight: units u + 1 and u + 2 load during u
   static constexpr size_t smem() {
     return 128 + sizeof(cf) * (STAGES * tile_elems() + (size_t)line_buf_r0<N, R0, Q>() + N) +
            sizeof(uint64_t) * STAGES;
   }
   static_assert(Q % 2 == 0 && 2 * Q <= 256, "tensor box of 2Q floats, x a 16-byte multiple");
-  static_assert(NBOX == 1 || ((NZ - KZB) * Q * sizeof(cf)) % 128 == 0, "second box off a 128-byte boundary");
+  static_assert(NBOX == 1 || (KZS * Q * sizeof(cf)) % 128 == 0, "boxes off a 128-byte boundary");
 };
 
 constexpr int TS_TMA_WAIT_LIMIT = 1 << 22;   // polls of an mbarrier before a wait gives up
 
-// complex line of row q of the two shells in a tile (shell a real part, shell b imaginary part);
-// the tile holds tile[s][k][j] = (s ? b : a)[k][x][y0 + j], shell b at TS
+// complex line of row q of the two spectra in a tile (a real part, b imaginary part), whose planes
+// beyond ka and kb are zero; the tile holds tile[s][k][j] = (s ? b : a)[k][x][y0 + j], b at TS
 template <int N, int Q>
-__device__ __forceinline__ cf ts_tile_input(const cf* tile, int q, int p) {
+__device__ __forceinline__ cf ts_tile_input(const cf* tile, int q, int p, int ka, int kb) {
   constexpr int TS = TsZ<N>::TS;
   const int k = p <= N / 2 ? p : N - p;
-  const cf A = tile[k * Q + q], B = tile[TS + k * Q + q];
+  const cf A = k <= ka ? tile[k * Q + q] : cf{0.f, 0.f}, B = k <= kb ? tile[TS + k * Q + q] : cf{0.f, 0.f};
   if (p == 0 || p == N / 2) return cf{A.x, B.x};
   if (p < N / 2) return cf{A.x - B.y, A.y + B.x};
   return cf{A.x + B.y, B.x - A.y};
 }
 
-// G grids per shell: 0 sfr, 1 X-ray, 2 and 3 the AGN bands in use (their per-cell heating
-// terms also go to agn_heat, for the AGN heating averages)
-// The shells' Hermitian column tiles arrive by tensor loads (the spectra as the tensor `tmap`:
-// floats y innermost, then x, then kz of spectrum r G + g at (r G + g)(N/2 + 1) + kz), STAGES
-// tiles in flight, one mbarrier each.
-template <int N, int G>
+// Grids per shell: sfr, then with XS (X-ray by shells) the X-ray grid, then NA AGN bands (their
+// per-cell heating terms also go to agn_heat, for the AGN heating averages).  Without XS the X-ray
+// node fields follow the shells: heat, ion, lya of node zv.m0, then of the next node.
+// The Hermitian column tiles arrive by tensor loads (the spectra as the tensor `tmap`: floats y
+// innermost, then x, then kz of spectrum s at s (N/2 + 1) + kz), STAGES tiles in flight, one
+// mbarrier each; a spectrum's planes beyond its cut are not loaded.
+template <int N, bool XS, int NA>
 __global__ void __launch_bounds__(TsZ<N>::NTH, TsZ<N>::MINB)
     k_ts_zsum(const __grid_constant__ CUtensorMap tmap, const cf* __restrict__ g_tw,
               const TsShellCoef* __restrict__ gco, TsZev zv, const float* __restrict__ xe_prev,
               float4* __restrict__ sums, float2* __restrict__ agn_heat, uint32_t* err) {
   using Z = TsZ<N>;
   using PL = typename Z::PL;
-  constexpr int Q = Z::Q, V = Z::V, NZ = Z::NZ, KZB = Z::KZB;
+  constexpr int Q = Z::Q, V = Z::V, NZ = Z::NZ;
+  constexpr int G = 1 + XS + NA;
+  constexpr bool COEF = XS || NA > 0;   // units that read a pair's tables
   constexpr int PADW = 2 * (N / 2 + 1);
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
@@ -423,7 +566,7 @@ __global__ void __launch_bounds__(TsZ<N>::NTH, TsZ<N>::MINB)
   cf* xbuf = tiles + Z::STAGES * Z::tile_elems();
   cf* s_tw = xbuf + line_buf_r0<N, Z::R0, Q>();
   uint64_t* bars = reinterpret_cast<uint64_t*>(s_tw + N);
-  __shared__ TsShellCoef sc[2];
+  __shared__ TsShellCoef sc[COEF ? 2 : 1];
   const int x = blockIdx.y, y = blockIdx.x * Q + threadIdx.x % Q;
   const int t = threadIdx.x / Q;
   if (threadIdx.x == 0) {
@@ -433,7 +576,7 @@ __global__ void __launch_bounds__(TsZ<N>::NTH, TsZ<N>::MINB)
   load_twiddles_p<PL>(s_tw, g_tw);
   const size_t row = (size_t)x * N + y;
   // this thread's cells: z = last_pos(t, s); x_e interpolation node and offset
-  // (ComputeTs.c:1198-1209)
+  // (ComputeTs.c:1198-1209): by shells the offset itself, by nodes its share of the interval
   float dxe[V];
   uint32_t lopack = 0;
 #pragma unroll
@@ -447,69 +590,87 @@ __global__ void __launch_bounds__(TsZ<N>::NTH, TsZ<N>::MINB)
     // parameter bank)
     const float xf = (float)xc;
     int m = 0;
-    float xm = zv.X[0];
+    float xm = zv.X[0], xn = zv.X[1];
 #pragma unroll
     for (int j = 1; j < x_int_NXHII; ++j)
       if (!(xf < zv.X[j])) {
         m = j;
         xm = zv.X[j];
+        xn = zv.X[j + 1 < x_int_NXHII ? j + 1 : j];
       }
     lopack |= (uint32_t)m << (4 * sl);
-    dxe[sl] = (float)(xc - (double)xm);
+    dxe[sl] = XS ? (float)(xc - (double)xm) : (float)((xc - (double)xm) / ((double)xn - (double)xm));
   }
   // every thread's cells each on one x_e node of their own (the common case early in
   // reionization): the coefficient reads leave the per-cell loops.  The choice is the block's, as
   // both paths run transforms with block barriers.
   static_assert(V == 8, "eight x_e node indices in one 32-bit word");
   const uint32_t lo0 = lopack & 15u;
-  const bool uni = __syncthreads_and(lopack == lo0 * 0x11111111u) != 0;
+  bool uni = false;
+  if constexpr (XS) uni = __syncthreads_and(lopack == lo0 * 0x11111111u) != 0;
   float a_heat[V], a_ion[V], a_lya[V], a_star[V];
-  float a_agn0[G > 2 ? V : 1], a_agn1[G > 3 ? V : 1];
+  float a_agn0[NA > 0 ? V : 1], a_agn1[NA > 1 ? V : 1];
 #pragma unroll
   for (int sl = 0; sl < V; ++sl) a_heat[sl] = a_ion[sl] = a_lya[sl] = a_star[sl] = 0.f;
 #pragma unroll
-  for (int sl = 0; sl < (G > 2 ? V : 1); ++sl) a_agn0[sl] = 0.f;
+  for (int sl = 0; sl < (NA > 0 ? V : 1); ++sl) a_agn0[sl] = 0.f;
 #pragma unroll
-  for (int sl = 0; sl < (G > 3 ? V : 1); ++sl) a_agn1[sl] = 0.f;
+  for (int sl = 0; sl < (NA > 1 ? V : 1); ++sl) a_agn1[sl] = 0.f;
   auto addr = [&](int p) { return line_addr_r0<Z::R0, Q>(p, threadIdx.x % Q); };
-  // units u = G (r / 2) + g: the pair of shells (r, r + 1), grid g; the tiles of units u + 1 and
-  // u + 2 load while unit u is transformed (three buffers).  A pair without its second shell (an
-  // odd count) gets zeros there, written by the block.
+  // Units, two spectra each: u = G (r / 2) + g < nsh, the pair of shells (r, r + 1) of grid g; then
+  // without XS one unit (heat, ion) per node, then one (lya, lya) per two nodes.  The tiles of units
+  // u + 1 and u + 2 load while unit u is transformed (three buffers).  A missing second spectrum (an
+  // odd count) reads as zeros.
   constexpr int S = Z::STAGES;
   const int y0 = blockIdx.x * Q, q = threadIdx.x % Q;
-  const int nunits = G * ((zv.nS + 1) / 2);
-  auto has_b = [&](int u) { return 2 * (u / G) + 1 < zv.nS; };
+  const int nsh = G * ((zv.nS + 1) / 2), nm = XS ? 0 : zv.nm;
+  const int nunits = nsh + nm + (nm + 1) / 2;
+  // the spectra of unit u and the last plane of each (-1: there is none)
+  auto unit = [&](int u, int (&sp)[2], int (&kl)[2]) {
+    if (XS || u < nsh) {
+      const int r = 2 * (u / G), g = u % G;
+      const bool two = r + 1 < zv.nS;
+      sp[0] = r * G + g;
+      sp[1] = sp[0] + G;
+      kl[0] = __ldg(&gco[r].kzmax);
+      kl[1] = two ? __ldg(&gco[r + 1].kzmax) : -1;
+    } else {
+      const int v = u - nsh, base = zv.nS * G;
+      const bool la = v >= nm;
+      sp[0] = la ? base + 6 * (v - nm) + 2 : base + 3 * v;
+      sp[1] = la ? sp[0] + 3 : sp[0] + 1;
+      kl[0] = N / 2;
+      kl[1] = !la || 2 * (v - nm) + 1 < nm ? N / 2 : -1;
+    }
+  };
+  auto boxes = [](int k) { return k < 0 ? 0 : k <= Z::KZS ? 1 : (k + Z::KZS - 1) / Z::KZS; };
   // thread 0: tensor loads of unit u into its buffer
   auto issue = [&](int u) {
     const int b = u % S;
-    const bool two = has_b(u);
-    mbar_arrive_expect_tx(&bars[b], (two ? 2u : 1u) * Z::SHELL_TX);
-    for (int sh = 0; sh < (two ? 2 : 1); ++sh) {
-      const int spec = (2 * (u / G) + sh) * G + u % G;
-#pragma unroll
-      for (int k = 0; k < Z::NBOX; ++k) {
-        const int k0 = k ? NZ - KZB : 0;
-        tma_load_3d(tiles + b * Z::tile_elems() + sh * Z::TS + k0 * Q, &tmap, 2 * y0, x, spec * NZ + k0, &bars[b]);
-      }
-    }
-  };
-  auto zero_b = [&](int u) {
-    cf* tb = tiles + (u % S) * Z::tile_elems() + Z::TS;
-    for (int i = threadIdx.x; i < NZ * Q; i += Z::NTH) tb[i] = cf{0.f, 0.f};
+    int sp[2], kl[2];
+    unit(u, sp, kl);
+    mbar_arrive_expect_tx(&bars[b], (uint32_t)(boxes(kl[0]) + boxes(kl[1])) * Z::BOX_TX);
+    for (int sh = 0; sh < 2; ++sh)
+      for (int k = 0; k < boxes(kl[sh]); ++k)
+        tma_load_3d(tiles + b * Z::tile_elems() + sh * Z::TS + k * Z::KZS * Q, &tmap, 2 * y0, x,
+                    sp[sh] * NZ + k * Z::KZS, &bars[b]);
   };
   __syncthreads();   // barriers initialised
   if (threadIdx.x == 0)
     for (int u = 0; u < S - 1 && u < nunits; ++u) issue(u);
-  for (int u = 0; u < S - 1 && u < nunits; ++u)
-    if (!has_b(u)) zero_b(u);
   bool waited = true;
+  // the unit in work
+  const cf* tile = tiles;
+  int sp[2] = {0, 0}, kl[2] = {0, 0};
+  auto input = [&](int p, int) { return ts_tile_input<N, Q>(tile, q, p, kl[0], kl[1]); };
   // an AGN unit j: clamped at 0 (ComputeTs.c:615-630), its own band tables
-  auto agn_unit = [&](const cf* tile, int j, float (&ah)[G > 2 ? V : 1]) {
+  auto agn_unit = [&](int j, float (&ah)[NA > 0 ? V : 1]) {
     line_fft_p<PL, true>(
-        t, xbuf, s_tw, [&](int p, int) { return ts_tile_input<N, Q>(tile, q, p); }, addr,
+        t, xbuf, s_tw, input, addr,
         [&](int, cf v, int sl) {
           const int lo = (int)((lopack >> (4 * sl)) & 15u);
-          const float d = dxe[sl];
+          // by nodes dxe is the share of the interval, which the tables' slopes know as X
+          const float d = XS ? dxe[sl] : dxe[sl] * sc[0].dX[lo];
           const float vx = fmaxf(v.x, 0.f), vy = fmaxf(v.y, 0.f);
           const float h = vx * fmaf(d, sc[0].QA[j][0][lo], sc[0].PA[j][0][lo]) +
                           vy * fmaf(d, sc[1].QA[j][0][lo], sc[1].PA[j][0][lo]);
@@ -521,36 +682,53 @@ __global__ void __launch_bounds__(TsZ<N>::NTH, TsZ<N>::MINB)
                        vy * fmaf(d, sc[1].QA[j][2][lo], sc[1].PA[j][2][lo]);
         });
   };
+  // the share of node m (counted from 0) in this thread's cell sl
+  auto share = [&](int m, int sl) {
+    const int lo = (int)((lopack >> (4 * sl)) & 15u);
+    return lo == m ? 1.f - dxe[sl] : lo + 1 == m ? dxe[sl] : 0.f;
+  };
   for (int u = 0; u < nunits; ++u) {
     const int r = 2 * (u / G), g = u % G;
-    if (g == 0) {
+    if (COEF && g == 0 && u < nsh) {
       __syncthreads();  // readers of the previous pair's coefficients are done
       const bool two = r + 1 < zv.nS;
       const int* src = reinterpret_cast<const int*>(gco + r);
       int* dst = reinterpret_cast<int*>(sc);
       // words per shell: the AGN tables only when there are AGN units
       constexpr int SW = (int)(sizeof(TsShellCoef) / sizeof(int));
-      constexpr int W = G > 2 ? SW : (int)(offsetof(TsShellCoef, PA) / sizeof(int));
+      constexpr int W = NA > 0 ? SW : (int)(offsetof(TsShellCoef, PA) / sizeof(int));
       for (int i = threadIdx.x; i < 2 * W; i += Z::NTH) {
         const int sh = i / W, w = sh * SW + i % W;
         dst[w] = (sh == 0 || two) ? src[w] : 0;
       }
     }
     // buffer (u + 2) % 3 was consumed by unit u - 1 (the barrier at the end of its iteration)
-    if (u + S - 1 < nunits) {
-      if (threadIdx.x == 0) issue(u + S - 1);
-      if (!has_b(u + S - 1)) zero_b(u + S - 1);
-    }
+    if (u + S - 1 < nunits && threadIdx.x == 0) issue(u + S - 1);
     if (!mbar_wait(&bars[u % S], (uint32_t)((u / S) & 1), TS_TMA_WAIT_LIMIT)) waited = false;
-    __syncthreads();  // unit u's tile (and the pair's coefficients) are visible to every thread
-    const cf* tile = tiles + (u % S) * Z::tile_elems();
-    if (g == 0) {
+    if (COEF) __syncthreads();  // the pair's coefficients are visible to every thread
+    tile = tiles + (u % S) * Z::tile_elems();
+    unit(u, sp, kl);
+    if (!XS && u >= nsh) {
+      const int v = u - nsh;
+      if (v < nm) {
+        const int m = zv.m0 + v;
+        line_fft_p<PL, true>(t, xbuf, s_tw, input, addr, [&](int, cf f, int sl) {
+          const float w = share(m, sl);
+          a_heat[sl] = fmaf(w, f.x, a_heat[sl]);
+          a_ion[sl] = fmaf(w, f.y, a_ion[sl]);
+        });
+      } else {
+        const int m = zv.m0 + 2 * (v - nm);
+        line_fft_p<PL, true>(t, xbuf, s_tw, input, addr, [&](int, cf f, int sl) {
+          a_lya[sl] += share(m, sl) * f.x + share(m + 1, sl) * f.y;
+        });
+      }
+    } else if (g == 0) {
       // sfr: stellar Lyman-alpha sum, SFR clamped at 0 (ComputeTs.c:700)
-      const float c0 = sc[0].cstar, c1 = sc[1].cstar;
-      line_fft_p<PL, true>(
-          t, xbuf, s_tw, [&](int p, int) { return ts_tile_input<N, Q>(tile, q, p); }, addr,
-          [&](int, cf v, int sl) { a_star[sl] += fmaxf(v.x, 0.f) * c0 + fmaxf(v.y, 0.f) * c1; });
-    } else if (g == 1) {
+      const float c0 = __ldg(&gco[r].cstar), c1 = kl[1] >= 0 ? __ldg(&gco[r + 1].cstar) : 0.f;
+      line_fft_p<PL, true>(t, xbuf, s_tw, input, addr,
+                           [&](int, cf v, int sl) { a_star[sl] += fmaxf(v.x, 0.f) * c0 + fmaxf(v.y, 0.f) * c1; });
+    } else if (XS && g == 1) {
       // X-ray: heating, ionisation and Lyman-alpha integrands, not clamped
       if (uni) {
         // every cell of this thread on the same x_e node: its twelve coefficients read once
@@ -563,7 +741,7 @@ __global__ void __launch_bounds__(TsZ<N>::NTH, TsZ<N>::MINB)
             c[sh][kd][1] = sc[sh].Q[kd][lo0];
           }
         line_fft_p<PL, true>(
-            t, xbuf, s_tw, [&](int p, int) { return ts_tile_input<N, Q>(tile, q, p); }, addr,
+            t, xbuf, s_tw, input, addr,
             [&](int, cf v, int sl) {
               const float d = dxe[sl];
               a_heat[sl] += v.x * fmaf(d, c[0][0][1], c[0][0][0]) + v.y * fmaf(d, c[1][0][1], c[1][0][0]);
@@ -572,7 +750,7 @@ __global__ void __launch_bounds__(TsZ<N>::NTH, TsZ<N>::MINB)
             });
       } else {
         line_fft_p<PL, true>(
-            t, xbuf, s_tw, [&](int p, int) { return ts_tile_input<N, Q>(tile, q, p); }, addr,
+            t, xbuf, s_tw, input, addr,
             [&](int, cf v, int sl) {
               const int lo = (int)((lopack >> (4 * sl)) & 15u);
               const float d = dxe[sl];
@@ -584,11 +762,11 @@ __global__ void __launch_bounds__(TsZ<N>::NTH, TsZ<N>::MINB)
                   v.x * fmaf(d, sc[0].Q[2][lo], sc[0].P[2][lo]) + v.y * fmaf(d, sc[1].Q[2][lo], sc[1].P[2][lo]);
             });
       }
-    } else if constexpr (G > 2) {
-      if (g == 2) {
-        agn_unit(tile, 0, a_agn0);
-      } else if constexpr (G > 3) {
-        agn_unit(tile, 1, a_agn1);
+    } else if constexpr (NA > 0) {
+      if (g == 1 + XS) {
+        agn_unit(0, a_agn0);
+      } else if constexpr (NA > 1) {
+        agn_unit(1, a_agn1);
       }
     }
     // the tile is consumed (generic reads ordered before the tensor load that refills it)
@@ -600,7 +778,7 @@ __global__ void __launch_bounds__(TsZ<N>::NTH, TsZ<N>::MINB)
   for (int sl = 0; sl < V; ++sl) {
     const size_t ic = row * N + last_pos<PL>(t, sl);
     sums[ic] = make_float4(a_heat[sl], a_ion[sl], a_lya[sl], a_star[sl]);
-    if constexpr (G > 2) agn_heat[ic] = make_float2(a_agn0[sl], G > 3 ? a_agn1[G > 3 ? sl : 0] : 0.f);
+    if constexpr (NA > 0) agn_heat[ic] = make_float2(a_agn0[sl], NA > 1 ? a_agn1[NA > 1 ? sl : 0] : 0.f);
   }
 }
 
@@ -769,60 +947,107 @@ static int ts_combine(rg_context* ctx, int n, cf* spec, size_t stride, int G, co
 // against 43.5 ms for the two passes; the x pass here reads its history spectra mostly from L2.)
 template <int N>
 static int launch_ts_xy(rg_context* ctx, const cf* spec, cf* work_base, size_t stride, const TsBatch& bt,
-                        const float* wtab, int wpitch, const int* wcut, cudaStream_t st) {
+                        const float* wtab, int wpitch, cudaStream_t st) {
   using C = Cfg<N>;
-  const double nzc = (double)C::NZ * N * N;
   const cf* tw;
   int rc = twiddles_for(ctx, N, &tw);
   if (rc) return rc;
+  // planes the batch has, and the modes and columns its shells keep (for the algorithmic bytes)
+  int kzmax = 0;
+  double src_reads = 0, cols = 0, lines = 0;
+  const double full = (double)C::NZ * N * N;
+  for (int r = 0; r < bt.nr; ++r) {
+    const double k = std::sqrt((double)bt.cut[r]);
+    const int kz = std::min(N / 2, (int)k);
+    kzmax = std::max(kzmax, kz);
+    src_reads += bt.nk[r] * std::min(full, 2.0 / 3.0 * M_PI * k * k * k);
+    cols += std::min(full, M_PI / 2 * k * k * N);
+    lines += std::min(full, (kz + 1.0) * N * N);
+  }
   const size_t smx = sizeof(cf) * (N + (size_t)line_buf<N, C::BX>());
   RG_CUDA_TRY(ctx, cudaFuncSetAttribute(k_ts_x<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx));
   prof_begin(ctx, "ts_x_c2c_combine_window", st);
-  k_ts_x<N><<<dim3(N / C::BX, C::NZ), C::T * C::BX, smx, st>>>(spec, stride, work_base, bt, wtab, wpitch, wcut, tw);
-  double src_reads = 0;
-  for (int r = 0; r < bt.nr; ++r) src_reads += bt.nk[r];
-  prof_end(ctx, bt.ng * 8.0 * nzc * (src_reads + bt.nr), st);
+  k_ts_x<N><<<dim3(N / C::BX, kzmax + 1), C::T * C::BX, smx, st>>>(spec, stride, work_base, bt, wtab, wpitch, tw);
+  prof_end(ctx, bt.ng * 8.0 * (src_reads + cols), st);
   RG_CUDA_TRY(ctx, cudaGetLastError());
+  using Y = YCfg<N>;
+  RG_CUDA_TRY(ctx, cudaFuncSetAttribute(k_ts_y<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Y::smem()));
   prof_begin(ctx, "ts_y_c2c", st);
-  RG_CUDA_TRY(ctx, (launch_pass_y<N, true>(work_base, stride, bt.ng * bt.nr, tw, st)));
-  prof_end(ctx, bt.ng * bt.nr * 16.0 * nzc, st);
+  k_ts_y<N><<<dim3(N / Y::BY, kzmax + 1, bt.ng * bt.nr), Y::NTH, Y::smem(), st>>>(work_base, stride, bt, tw);
+  prof_end(ctx, bt.ng * 8.0 * (cols + lines), st);
+  RG_CUDA_TRY(ctx, cudaGetLastError());
   return RG_OK;
 }
 
-// the z pass over all nS shells: per-cell shell sums
-template <int N, int G>
+// the X-ray node fields: their spectra, then the inverse x and y passes in place
+template <int N>
+static int launch_ts_nodes(rg_context* ctx, const cf* spec, cf* fields, size_t stride, int gs,
+                           const TsNodeShell* d_sh, int nS, int nm, const float* wtab, int wpitch, cudaStream_t st) {
+  using C = Cfg<N>;
+  const cf* tw;
+  int rc = twiddles_for(ctx, N, &tw);
+  if (rc) return rc;
+  const int nf = 3 * nm, log2n = __builtin_ctz(N);
+  // fields a thread accumulates: one chunk up to 4 nodes, else as even as 3 or 4 nodes a chunk go
+  const int per = nm <= 2 ? 2 : (nm == 3 || nm == 5 || nm == 6 || nm == 9) ? 3 : 4;
+  const dim3 grid((unsigned)std::min((stride + 255) / 256, (size_t)ctx->num_sms * 64), (nm + per - 1) / per);
+  prof_begin(ctx, "ts_xray_nodes", st);
+  if (per == 2)
+    k_ts_nodes<6><<<grid, 256, 0, st>>>(spec, stride, gs, fields, d_sh, nS, nf, wtab, wpitch, log2n);
+  else if (per == 3)
+    k_ts_nodes<9><<<grid, 256, 0, st>>>(spec, stride, gs, fields, d_sh, nS, nf, wtab, wpitch, log2n);
+  else
+    k_ts_nodes<12><<<grid, 256, 0, st>>>(spec, stride, gs, fields, d_sh, nS, nf, wtab, wpitch, log2n);
+  prof_end(ctx, 8.0 * stride * nf, st);
+  RG_CUDA_TRY(ctx, cudaGetLastError());
+  const size_t smx = sizeof(cf) * (N + (size_t)line_buf<N, C::BX>());
+  RG_CUDA_TRY(ctx, cudaFuncSetAttribute(k_pass_x<N, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx));
+  prof_begin(ctx, "ts_nodes_x_c2c", st);
+  k_pass_x<N, true><<<dim3(N / C::BX, C::NZ, nf), C::T * C::BX, smx, st>>>(fields, stride, tw, 1.f);
+  prof_end(ctx, 16.0 * stride * nf, st);
+  RG_CUDA_TRY(ctx, cudaGetLastError());
+  prof_begin(ctx, "ts_nodes_y_c2c", st);
+  RG_CUDA_TRY(ctx, (launch_pass_y<N, true>(fields, stride, nf, tw, st)));
+  prof_end(ctx, 16.0 * stride * nf, st);
+  return RG_OK;
+}
+
+// the z pass over all nS shells (and the node fields): per-cell shell sums
+template <int N, bool XS, int NA>
 static int launch_ts_zsum_g(rg_context* ctx, const cf* work, size_t stride, const TsShellCoef* d_co, const TsZev& zv,
-                            const float* xe_prev, float4* sums, float2* agn_heat, cudaStream_t st) {
+                            const float* xe_prev, float4* sums, float2* agn_heat, double planes, cudaStream_t st) {
   const cf* tw;
   int rc = twiddles_for(ctx, N, &tw);
   if (rc) return rc;
   using Z = TsZ<N>;
-  const double n3 = (double)N * N * N, nzc = (double)(N / 2 + 1) * N * N;
+  const double n3 = (double)N * N * N;
   if (stride != (size_t)Z::NZ * N * N) return set_error(ctx, RG_EINVAL, "Ts z pass: shell spectra must be contiguous");
-  // every shell's G spectra (S[kz][x][y], one after another) as a 3-D float tensor
+  // every spectrum (S[kz][x][y], one after another) as a 3-D float tensor
   CUtensorMap tmap;
-  const uint64_t dims[3] = {2ull * N, (uint64_t)N, (uint64_t)Z::NZ * zv.nS * G};
+  const uint64_t dims[3] = {2ull * N, (uint64_t)N, (uint64_t)Z::NZ * (zv.nS * (1 + XS + NA) + (XS ? 0 : 3 * zv.nm))};
   const uint64_t strides[2] = {8ull * N, 8ull * N * N};
-  const uint32_t box[3] = {2u * Z::Q, 1u, (uint32_t)Z::KZB};
+  const uint32_t box[3] = {2u * Z::Q, 1u, (uint32_t)Z::KZS + 1u};
   const int mrc = tma_map_3d(&tmap, work, dims, strides, box);
   if (mrc != 0) return set_error(ctx, RG_ECUDA, "cuTensorMapEncodeTiled failed (" + std::to_string(mrc) + ")");
   const size_t smz = Z::smem();
-  RG_CUDA_TRY(ctx, cudaFuncSetAttribute(k_ts_zsum<N, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smz));
+  RG_CUDA_TRY(ctx, cudaFuncSetAttribute(k_ts_zsum<N, XS, NA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smz));
   prof_begin(ctx, "ts_z_c2r_sums", st);
-  k_ts_zsum<N, G><<<dim3(N / Z::Q, N), Z::NTH, smz, st>>>(tmap, tw, d_co, zv, xe_prev, sums, agn_heat, ctx->xy_ctrl);
-  // Hermitian halves of the G grids of every shell, x_e read, four float sums (and the AGN
-  // heating pair) written
-  prof_end(ctx, zv.nS * G * 8.0 * nzc + 4.0 * n3 + 16.0 * n3 + (G > 2 ? 8.0 * n3 : 0.0), st);
+  k_ts_zsum<N, XS, NA><<<dim3(N / Z::Q, N), Z::NTH, smz, st>>>(tmap, tw, d_co, zv, xe_prev, sums, agn_heat,
+                                                                ctx->xy_ctrl);
+  // the planes of the spectra, x_e read, four float sums (and the AGN heating pair) written
+  prof_end(ctx, planes * 8.0 * N * N + 4.0 * n3 + 16.0 * n3 + (NA > 0 ? 8.0 * n3 : 0.0), st);
   RG_CUDA_TRY(ctx, cudaGetLastError());
   return RG_OK;
 }
 
 template <int N>
-static int launch_ts_zsum(rg_context* ctx, const cf* work, size_t stride, int ng, const TsShellCoef* d_co,
-                          const TsZev& zv, const float* xe_prev, float4* sums, float2* agn_heat, cudaStream_t st) {
-  if (ng == 2) return launch_ts_zsum_g<N, 2>(ctx, work, stride, d_co, zv, xe_prev, sums, nullptr, st);
-  if (ng == 3) return launch_ts_zsum_g<N, 3>(ctx, work, stride, d_co, zv, xe_prev, sums, agn_heat, st);
-  return launch_ts_zsum_g<N, 4>(ctx, work, stride, d_co, zv, xe_prev, sums, agn_heat, st);
+static int launch_ts_zsum(rg_context* ctx, const cf* work, size_t stride, int nagn, const TsShellCoef* d_co,
+                          const TsZev& zv, const float* xe_prev, float4* sums, float2* agn_heat, double planes,
+                          cudaStream_t st) {
+#define RG_TS_Z(XS, NA) launch_ts_zsum_g<N, XS, NA>(ctx, work, stride, d_co, zv, xe_prev, sums, agn_heat, planes, st)
+  if (zv.nm) return nagn == 0 ? RG_TS_Z(false, 0) : nagn == 1 ? RG_TS_Z(false, 1) : RG_TS_Z(false, 2);
+  return nagn == 0 ? RG_TS_Z(true, 0) : nagn == 1 ? RG_TS_Z(true, 1) : RG_TS_Z(true, 2);
+#undef RG_TS_Z
 }
 
 #define RG_TS_DISPATCH(n, call)                                                           \
@@ -838,13 +1063,33 @@ static int launch_ts_zsum(rg_context* ctx, const cf* work, size_t stride, int ng
   }
 
 static int ts_xy(rg_context* ctx, int n, const cf* spec, cf* work_base, size_t stride, const TsBatch& bt,
-                 const float* wtab, int wpitch, const int* wcut, cudaStream_t st) {
-  RG_TS_DISPATCH(n, launch_ts_xy<NN>(ctx, spec, work_base, stride, bt, wtab, wpitch, wcut, st));
+                 const float* wtab, int wpitch, cudaStream_t st) {
+  RG_TS_DISPATCH(n, launch_ts_xy<NN>(ctx, spec, work_base, stride, bt, wtab, wpitch, st));
 }
 
-static int ts_zsum(rg_context* ctx, int n, const cf* work, size_t stride, int ng, const TsShellCoef* d_co,
-                   const TsZev& zv, const float* xe_prev, float4* sums, float2* agn_heat, cudaStream_t st) {
-  RG_TS_DISPATCH(n, launch_ts_zsum<NN>(ctx, work, stride, ng, d_co, zv, xe_prev, sums, agn_heat, st));
+static int ts_nodes(rg_context* ctx, int n, const cf* spec, cf* fields, size_t stride, int gs, const TsNodeShell* d_sh,
+                    int nS, int nm, const float* wtab, int wpitch, cudaStream_t st) {
+  RG_TS_DISPATCH(n, launch_ts_nodes<NN>(ctx, spec, fields, stride, gs, d_sh, nS, nm, wtab, wpitch, st));
+}
+
+static int ts_zsum(rg_context* ctx, int n, const cf* work, size_t stride, int nagn, const TsShellCoef* d_co,
+                   const TsZev& zv, const float* xe_prev, float4* sums, float2* agn_heat, double planes,
+                   cudaStream_t st) {
+  RG_TS_DISPATCH(n, launch_ts_zsum<NN>(ctx, work, stride, nagn, d_co, zv, xe_prev, sums, agn_heat, planes, st));
+}
+
+// the last n2 that the sharp-k window of radius R keeps (k R 0.413566994 > 1 drops a mode)
+static int sharpk_cut(double delta_k, double R, int n2max) {
+  auto drops = [&](int n2) { return delta_k * std::sqrt((double)n2) * R * 0.413566994 > 1.0; };
+  int lo = 0, hi = n2max + 1;   // lo is kept; hi is dropped, or past the table
+  while (hi > lo + 1) {
+    const int mid = (lo + hi) / 2;
+    if (drops(mid))
+      hi = mid;
+    else
+      lo = mid;
+  }
+  return lo;
 }
 
 static double pow2_scale(double maxabs) {
@@ -906,17 +1151,22 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
     Z.f_H = cm.f_H;
     Z.f_He = cm.f_He;
   }
-  // device constants, the non-convergence counter and the per-shell coefficients live in one
-  // context buffer: [TsDev][int + pad][TsShellCoef x shells]
+  // device constants, the non-convergence counter, the range of x_e and the per-shell coefficients
+  // live in one context buffer: [TsDev][int, x_e range][TsShellCoef x shells][TsNodeShell x shells]
   const int nS_all = p->TsNumFilterSteps;
   const size_t off_co = (sizeof(TsDev) + 16 + 255) / 256 * 256;
-  if ((rc = ensure_device(ctx, &ctx->ts_const, &ctx->ts_const_elems, off_co + sizeof(TsShellCoef) * (nS_all + 1))))
+  if ((rc = ensure_device(ctx, &ctx->ts_const, &ctx->ts_const_elems,
+                          off_co + (sizeof(TsShellCoef) + sizeof(TsNodeShell)) * (nS_all + 1))))
     return rc;
   TsDev* d_hc = reinterpret_cast<TsDev*>(ctx->ts_const);
   int* d_nonconv = reinterpret_cast<int*>(ctx->ts_const + sizeof(TsDev));
   TsShellCoef* d_co = reinterpret_cast<TsShellCoef*>(ctx->ts_const + off_co);
   RG_CUDA_TRY(ctx, cudaMemcpyAsync(d_hc, &hc, sizeof(TsDev), cudaMemcpyHostToDevice, st));
+  TsNodeShell* d_node = reinterpret_cast<TsNodeShell*>(d_co + nS_all + 1);
+  unsigned* d_range = reinterpret_cast<unsigned*>(d_nonconv + 1);
   RG_CUDA_TRY(ctx, cudaMemsetAsync(d_nonconv, 0, sizeof(int), st));
+  RG_CUDA_TRY(ctx, cudaMemsetAsync(d_range, 0xff, sizeof(unsigned), st));
+  RG_CUDA_TRY(ctx, cudaMemsetAsync(d_range + 1, 0, sizeof(unsigned), st));
   const int nblk = 148 * 8;
   double* partials = ensure_partials(ctx, (size_t)nblk * TS_NSUM);
   if (!partials) return set_error(ctx, RG_ENOMEM, "partials");
@@ -956,14 +1206,18 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
   // collapse fraction and <x_e> (both branches compute the collapse fraction)
   prof_begin(ctx, "ts_reduce0", st);
   if ((rc = stage_wait(ctx, stg->inputs, st))) return rc;
-  k_ts_reduce0<<<nblk, 256, 0, st>>>(g->stars, g->deltax, g->x_e_box_prev, N, Mh2, ftpr3, partials);
+  k_ts_reduce0<<<nblk, 256, 0, st>>>(g->stars, g->deltax, g->x_e_box_prev, N, Mh2, ftpr3, partials, d_range);
   prof_end(ctx, 12.0 * n3, st);
   RG_CUDA_TRY(ctx, cudaGetLastError());
   if ((rc = reduce_partials(ctx, partials, nblk, 2, ctx->d_sums, st))) return rc;
   RG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_sums, ctx->d_sums, sizeof(double) * 2, cudaMemcpyDeviceToHost, st));
+  RG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_sums + 2, d_range, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
   RG_CUDA_TRY(ctx, cudaStreamSynchronize(st));
   const double collapse_fraction = ctx->h_sums[0] / (double)n3;
   const double x_e_ave = ctx->h_sums[1] / (double)n3;
+  unsigned range[2];
+  std::memcpy(range, ctx->h_sums + 2, sizeof(range));
+  const float xe_lo = float_of_order(range[0]), xe_hi = float_of_order(range[1]);
   out->collapse_fraction = collapse_fraction;
   out->x_e_ave = x_e_ave;
 
@@ -1015,10 +1269,26 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
       wide = wide || nk > TS_MAXSRC;
     }
     const int nused = std::max(1, (int)used.size());
+    // X-ray by nodes where 3 fields per node are fewer than the shells: the nodes m0 .. m0 + nm - 1
+    // around the box's x_e (clamped as each cell's is).  A shell with its combination in a spare
+    // slot, which later batches overwrite, and a NaN in x_e keep the shells.
+    auto node = [&](float v) {
+      const float* X = ctx->tables.x_int_XHII.data();
+      const double top = (double)X[x_int_NXHII - 1] * 0.999;
+      const double xc = (double)v > top ? top : (double)v < (double)X[0] ? 1.001 * (double)X[0] : (double)v;
+      return locate_xHII_index(X, (float)xc);
+    };
+    if (!wide && !std::isnan(xe_lo) && !std::isnan(xe_hi)) {
+      zv.m0 = node(xe_lo);
+      zv.nm = node(xe_hi) + 2 - zv.m0;
+      if (3 * zv.nm >= nS) zv.nm = 0;
+    }
+    const int xs = zv.nm == 0;              // X-ray grids per shell
+    const int Gs = 1 + xs + nagn;           // grids per shell
     const size_t slots = (size_t)nused + (wide ? TS_KB : 0);
     if ((rc = ensure_device(ctx, &ctx->spec, &ctx->spec_elems, nc * G * slots))) return rc;
     // every shell's filtered grids stay in HBM until the fused z pass (G nS spectra)
-    if ((rc = ensure_device(ctx, &ctx->work, &ctx->work_elems, nc * G * nS))) return rc;
+    if ((rc = ensure_device(ctx, &ctx->work, &ctx->work_elems, nc * ((size_t)Gs * nS + 3 * zv.nm)))) return rc;
     // source grid `which` (0 sfr, 1 xray, 2 + j AGN band bands[j]) of source k, on the device
     // (the AGN histories are re-weighted like the sfr ones, load_reion_bh_grids)
     const rg_grids* sg = src_host ? src_host : g;
@@ -1037,14 +1307,21 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
     };
     // window rows for the shells (filter() takes BoxSize in Mpc/h and R in Mpc, ComputeTs.c:532)
     const int n2max = 3 * (N / 2) * (N / 2);
-    if ((rc = ensure_device(ctx, &ctx->d_radii, &ctx->d_radii_elems, (size_t)nS))) return rc;
-    RG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->d_radii, sh.R.data(), sizeof(double) * nS, cudaMemcpyHostToDevice, st));
-    if ((rc = ensure_device(ctx, &ctx->wtab, &ctx->wtab_elems, (size_t)nS * (n2max + 1)))) return rc;
-    if ((rc = ensure_device(ctx, &ctx->wcut, &ctx->wcut_elems, (size_t)nS))) return rc;
-    if ((rc = window_table(ctx, p->BoxSize, ctx->d_radii, nS, p->TsHeatingFilterType, ctx->wtab, n2max, st,
-                           ctx->wcut)))
-      return rc;
-    const int* wcut = p->TsHeatingFilterType == 1 ? ctx->wcut : nullptr;
+    // (the sharp-k rows are steps: their ends are all the passes need)
+    const bool sharp = p->TsHeatingFilterType == 1;
+    std::vector<int> cut(nS, TS_NOCUT);   // no filter on the first shell (ComputeTs.c:529)
+    if (sharp) {
+      for (int r = 1; r < nS; ++r) cut[r] = sharpk_cut(2.0 * M_PI / p->BoxSize, sh.R[r], n2max);
+    } else {
+      if ((rc = ensure_device(ctx, &ctx->d_radii, &ctx->d_radii_elems, (size_t)nS))) return rc;
+      RG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->d_radii, sh.R.data(), sizeof(double) * nS, cudaMemcpyHostToDevice, st));
+      if ((rc = ensure_device(ctx, &ctx->wtab, &ctx->wtab_elems, (size_t)nS * (n2max + 1)))) return rc;
+      if ((rc = window_table(ctx, p->BoxSize, ctx->d_radii, nS, p->TsHeatingFilterType, ctx->wtab, n2max, st)))
+        return rc;
+    }
+    auto kzmax = [&](int r) { return std::min(N / 2, (int)std::sqrt((double)cut[r])); };
+    std::vector<TsNodeShell> nodes(nS);
+    std::memset(nodes.data(), 0, sizeof(TsNodeShell) * nodes.size());
 
     // Batches of TS_KB shells: the forward transforms of the sources a batch uses first (`used`
     // is in order of first use), then its x and y passes into work[r][g].  From host arrays,
@@ -1079,7 +1356,9 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
       TsBatch bt;
       std::memset(&bt, 0, sizeof(bt));
       bt.nr = cnt;
-      bt.ng = G;
+      bt.gs = G;
+      bt.ng = Gs;
+      bt.skip = !xs;
       for (int j = 0; j < cnt; ++j) {
         const int r = r0 + j;
         std::vector<int> ks;
@@ -1104,10 +1383,16 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
           bt.cs[j][i] = cs[i];
         }
         bt.nk[j] = nk;
-        bt.filtered[j] = r > 0;  // no filter on the first shell (ComputeTs.c:529)
+        bt.filtered[j] = r > 0;
         bt.wrow[j] = r;
+        bt.cut[j] = cut[r];
+        nodes[r].nk = nk;
+        nodes[r].filtered = r > 0;
+        nodes[r].cut = cut[r];
+        std::copy(bt.ks[j], bt.ks[j] + nk, nodes[r].ks);
+        std::copy(bt.cs[j], bt.cs[j] + nk, nodes[r].cs);
       }
-      if ((rc = ts_xy(ctx, N, ctx->spec, ctx->work + (size_t)r0 * G * nc, nc, bt, ctx->wtab, n2max + 1, wcut, st)))
+      if ((rc = ts_xy(ctx, N, ctx->spec, ctx->work + (size_t)r0 * Gs * nc, nc, bt, ctx->wtab, n2max + 1, st)))
         return rc;
     }
     if ((rc = kick())) return rc;
@@ -1185,6 +1470,12 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
           hco[r].Q[kind][m] = (float)(Qd[((size_t)r * 3 + kind) * x_int_NXHII + m] * scale[kind]);
         }
       hco[r].cstar = (float)(cs[r] * scale[3]);
+      hco[r].kzmax = kzmax(r);
+      for (int m = 0; m + 1 < x_int_NXHII; ++m) hco[r].dX[m] = (float)((double)X[m + 1] - (double)X[m]);
+      for (int m = 0; m < zv.nm; ++m)
+        for (int kind = 0; kind < 3; ++kind)
+          nodes[r].f[3 * m + kind] =
+              (float)(Pd[((size_t)r * 3 + kind) * x_int_NXHII + zv.m0 + m] * scale[kind]);
       for (int j = 0; j < nagn; ++j)
         for (int kind = 0; kind < 3; ++kind)
           for (int m = 0; m < x_int_NXHII; ++m) {
@@ -1195,11 +1486,19 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
     }
     RG_CUDA_TRY(ctx, cudaMemcpyAsync(d_co, hco.data(), sizeof(TsShellCoef) * (nS + 1), cudaMemcpyHostToDevice, st));
     zv.nS = nS;
+    if (zv.nm) {
+      RG_CUDA_TRY(ctx, cudaMemcpyAsync(d_node, nodes.data(), sizeof(TsNodeShell) * nS, cudaMemcpyHostToDevice, st));
+      if ((rc = ts_nodes(ctx, N, ctx->spec, ctx->work + (size_t)nS * Gs * nc, nc, G, d_node, nS, zv.nm, ctx->wtab,
+                         n2max + 1, st)))
+        return rc;
+    }
+    double planes = 3.0 * zv.nm * (N / 2 + 1);
+    for (int r = 0; r < nS; ++r) planes += Gs * (kzmax(r) + 1.0);
     if ((rc = ensure_device(ctx, &ctx->ts_sums, &ctx->ts_sums_elems, n3))) return rc;
     if (nagn && (rc = ensure_device(ctx, &ctx->ts_agn, &ctx->ts_agn_elems, n3))) return rc;
     if ((rc = xy_ctrl_reset(ctx, 0, st))) return rc;   // the error word of the tile waits
-    if ((rc = ts_zsum(ctx, N, ctx->work, nc, G, d_co, zv, g->x_e_box_prev, ctx->ts_sums, nagn ? ctx->ts_agn : nullptr,
-                      st)))
+    if ((rc = ts_zsum(ctx, N, ctx->work, nc, nagn, d_co, zv, g->x_e_box_prev, ctx->ts_sums,
+                      nagn ? ctx->ts_agn : nullptr, planes, st)))
       return rc;
     RG_CUDA_TRY(ctx, cudaStreamSynchronize(st));  // hco outlives the copy
     if ((rc = xy_ctrl_check(ctx, st))) return rc;
