@@ -192,8 +192,9 @@ typedef struct rg_context rg_context;
 int rg_create(int device, int grid_dim, rg_context** out);
 int rg_destroy(rg_context* ctx);
 int rg_set_mode(rg_context* ctx, int mode);
-/* Radii per batch of the fused mode's x/y and z passes: 0 = the default, 8; larger values are
-   cut to 16 (the tuner in autotune.py picks one per workload shape). */
+/* Radii per batch of the fused mode's x/y and z passes: 0 = the default, 16 where the windowed
+   spectra of a batch take at most 6 GB, else 8; larger values are cut to 16 (the tuner in
+   autotune.py picks one per workload shape). */
 int rg_set_radius_batch(rg_context* ctx, int radii_per_batch);
 /* cudaStream_t to launch on (NULL = the context's own stream). */
 int rg_set_stream(rg_context* ctx, void* stream);
@@ -230,8 +231,8 @@ int rg_find_HII_bubbles(rg_context* ctx, const rg_params* p, const rg_snapshot* 
 /* find_HII_bubbles for n_units independent snapshots of one ReionGridDim on device grids, in one
    call (arrays p[n_units], s[n_units], g[n_units], out[n_units]): the forward transforms of all
    their grids and, for every batch of radii, the windowed inverse x/y passes of all of them run
-   as shared launches; the z passes (the barrier test) run per snapshot; the host synchronises
-   once.  Each unit gets exactly what rg_find_HII_bubbles gives it.  The units must share
+   as shared launches; the z passes (the barrier test) take several snapshots a launch up to
+   128^3 and one above; the host synchronises once.  Each unit gets exactly what rg_find_HII_bubbles gives it.  The units must share
    ReionGridDim (= the context's), BoxSize, ReionFilterType, the feature flags and the radius
    schedule (RG_EINVAL otherwise).  With recombinations, Pop III sources or RG_MODE_PLAIN the
    units run one after another.  Device memory grows with the units: n_units x (live grids) x

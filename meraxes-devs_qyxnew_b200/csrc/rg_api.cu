@@ -338,6 +338,7 @@ int rg_destroy(rg_context* ctx) {
   if (ctx->work) cudaFree(ctx->work);
   if (ctx->bits) cudaFree(ctx->bits);
   if (ctx->wtab) cudaFree(ctx->wtab);
+  if (ctx->wplanes) cudaFree(ctx->wplanes);
   if (ctx->wcut) cudaFree(ctx->wcut);
   if (ctx->ps_pad) cudaFree(ctx->ps_pad);
   if (ctx->ps_stage) cudaFree(ctx->ps_stage);

@@ -144,7 +144,8 @@ __device__ __forceinline__ void dft_small(cf* v) {
 }
 
 // ---------------------------------------------------------------------------
-// radix plans: length NN, stages R[0..S) and threads per line T (T divides every N / R[s])
+// radix plans: length NN, stages R[0..S) and threads per line T (T divides every N / R[s], except in
+// PlanZ)
 
 #define RG_PLAN(name, n, t, ...)                      \
   template <>                                         \
@@ -181,6 +182,17 @@ RG_PLAN(Plan8, 64, 8, 8, 8)
 RG_PLAN(Plan8, 128, 16, 8, 4, 4)
 RG_PLAN(Plan8, 256, 32, 8, 8, 4)
 RG_PLAN(Plan8, 512, 64, 8, 8, 8)
+
+// the z pass of find_HII_bubbles, which keeps every grid's values of a thread in registers: the
+// default plans' stages (the same arithmetic), over more threads where 3 divides N, so that a thread
+// ends with 6 values instead of 24.  A quarter of the threads idle in the radix-8 stages.
+template <int N>
+struct PlanZ : Plan<N> {};
+RG_PLAN(PlanZ, 24, 4, 8, 3)
+RG_PLAN(PlanZ, 48, 8, 8, 2, 3)
+RG_PLAN(PlanZ, 96, 16, 8, 4, 3)
+RG_PLAN(PlanZ, 192, 32, 8, 8, 3)
+RG_PLAN(PlanZ, 384, 64, 8, 8, 2, 3)
 #undef RG_PLAN
 
 template <class PL, int s>
@@ -213,6 +225,24 @@ __host__ __device__ constexpr int tw_offset(int s) {
   return off;
 }
 
+// Butterflies of stage s that a thread owns at most.  Where T does not divide the N / R[s] butterflies
+// (PlanZ) the threads beyond them sit the last round out.
+template <class PL, int s>
+__host__ __device__ constexpr int stage_rounds() {
+  return (PL::NN / PL::R[s] + PL::T - 1) / PL::T;
+}
+// values a thread holds at most, and after the last stage
+template <class PL, int s = 0>
+__host__ __device__ constexpr int plan_values() {
+  constexpr int here = stage_rounds<PL, s>() * PL::R[s];
+  if constexpr (s + 1 < PL::S) return here > plan_values<PL, s + 1>() ? here : plan_values<PL, s + 1>();
+  return here;
+}
+template <class PL>
+__host__ __device__ constexpr int last_values() {
+  return stage_rounds<PL, PL::S - 1>() * PL::R[PL::S - 1];
+}
+
 // Stage-0 input position of register slot `slot` (0 <= slot < N/T) of thread t.
 template <class PL>
 __device__ __forceinline__ int stage0_pos(int t, int slot) {
@@ -229,11 +259,13 @@ __device__ __forceinline__ void stage_compute(cf* v, int t, const cf* __restrict
   constexpr int T = PL::T;
   constexpr int R = PL::R[s];
   constexpr int NS = StageNS<PL, s>::value;
-  constexpr int K = (N / R) / T;
-  static_assert((N / R) % T == 0, "T must divide N/R");
+  constexpr int K = stage_rounds<PL, s>();
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     const int j = t + k * T;
+    if constexpr ((N / R) % T != 0) {
+      if (j >= N / R) continue;
+    }
 #pragma unroll
     for (int r = 0; r < R; ++r) v[k * R + r] = load(j + r * (N / R), k * R + r);
     if constexpr (NS > 1) {
@@ -257,10 +289,13 @@ __device__ __forceinline__ void stage_emit(const cf* v, int t, Put&& put) {
   constexpr int N = PL::NN;
   constexpr int R = PL::R[s];
   constexpr int NS = StageNS<PL, s>::value;
-  constexpr int K = (N / R) / T;
+  constexpr int K = stage_rounds<PL, s>();
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     const int j = t + k * T;
+    if constexpr ((N / R) % T != 0) {
+      if (j >= N / R) continue;
+    }
     const int idxD = (j / NS) * NS * R + (j % NS);
 #pragma unroll
     for (int r = 0; r < R; ++r) put(idxD + r * NS, v[k * R + r], k * R + r);
@@ -310,8 +345,7 @@ template <class PL, bool INV, bool WS = false, class Load, class Addr, class Sto
 __device__ __forceinline__ void line_fft_p(int t, cf* xbuf, const cf* tw, Load&& load, Addr&& addr, Store&& store) {
   static_assert(plan_product<PL>() == PL::NN, "radix plan does not multiply to N");
   static_assert(!WS || (PL::T <= 32 && 32 % PL::T == 0), "warp barriers need a line within a warp");
-  constexpr int V = PL::NN / PL::T;
-  cf v[V];
+  cf v[plan_values<PL>()];
   stage_compute<PL, 0, INV>(v, t, tw, load);
   stages_from<PL, 0, INV, WS>(v, t, xbuf, addr, tw, store);
 }

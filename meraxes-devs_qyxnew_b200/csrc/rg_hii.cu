@@ -2,11 +2,10 @@
 //
 // Per snapshot: one forward r2c of each grid the barrier test reads (deltax, stars, [x_e],
 // [effective_bhm]); then the filter radii in batches of KB:
-//   x pass : each block loads its spectrum tile once and writes KB windowed, x-transformed
-//            copies (one per radius of the batch)
-//   y pass : in place over the KB x G work grids
-//   z pass : per block of rows, for each radius of the batch in order: c2r of the G grids into
-//            shared memory, then the aliasing clamp and the barrier test per cell.
+//   x and y passes (rg_hii_xy.cu) into KB x G work grids
+//   z pass : per block of rows, for each radius of the batch in order: c2r of the G grids, then the
+//            aliasing clamp and the barrier test per cell (k_hii_zr in rg_hii_z.cuh; here the
+//            row-buffer form for Pop III sources, k_hii_z).
 // Until the last radius the per-cell state is two bits (ionized this snapshot; z_at_ionization
 // still < 0), kept in registers within a batch and in one byte per cell between batches;
 // z_at_ionization and J_21 are written only where a cell first ionizes.  The last radius also
@@ -21,10 +20,9 @@
 #include <utility>
 #include <vector>
 
+#include "rg_hii_z.cuh"
 #include "rg_internal.h"
 #include "rg_pass.cuh"
-#include "rg_tma.cuh"
-#include "rg_xyf.cuh"
 
 namespace rg {
 
@@ -62,64 +60,27 @@ __global__ void k_window_table(float* wtab, int n2max, const double* __restrict_
   }
 }
 
-
-// ---------------------------------------------------------------------------
-// inverse x pass with the window and a batch of radii: grid g of spec (spec + g * stride) is
-// read once per block; radius r of the batch is written to work + (r * ng + g) * stride.
-// Radius r uses window row wrows + r * wpitch, or none when r == unfiltered.
-
-template <int N>
-__global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::BX, (x_pass_minb<N>()))
-    k_hii_x(const cf* __restrict__ spec, size_t stride, int ng, cf* __restrict__ work, int nr,
-            const float* __restrict__ wrows, int wpitch, int unfiltered, const cf* __restrict__ g_tw) {
-  constexpr int T = Cfg<N>::T, B = Cfg<N>::BX, V = Cfg<N>::V;
-  extern __shared__ cf smem[];
-  cf* s_tw = smem;
-  cf* xbuf = smem + N;
-  const int kz = blockIdx.y;
-  const int b = threadIdx.x % B, t = threadIdx.x / B;
-  const int y = blockIdx.x * B + b;
-  const size_t col = (size_t)kz * N * N + y;
-  load_twiddles<N>(s_tw, g_tw);
-  // |k|^2 index of each register slot: nx from the position, ny from the column
-  int n2[V];
-  const int ny = y > N / 2 ? y - N : y;
-#pragma unroll
-  for (int sl = 0; sl < V; ++sl) {
-    const int p = stage0_pos<N>(t, sl);
-    const int nx = p > N / 2 ? p - N : p;
-    n2[sl] = nx * nx + ny * ny + kz * kz;
-  }
-  __syncthreads();
-  // Radius outer, grid inner: the window gathers (scattered 4-byte reads of the table) are
-  // shared by all grids; a grid's spectrum tile is read from HBM at the first radius and
-  // from L1/L2 after that.
-  for (int r = 0; r < nr; ++r) {
-    float wv[V];
-    if (r == unfiltered) {
-#pragma unroll
-      for (int sl = 0; sl < V; ++sl) wv[sl] = 1.f;
-    } else {
-      const float* wr = wrows + (size_t)r * wpitch;
-#pragma unroll
-      for (int sl = 0; sl < V; ++sl) wv[sl] = __ldg(wr + n2[sl]);
+// The windows of the radii blockIdx.y on the octant of modes.  The x pass of a radius reads each value
+// up to four times per grid, and from a row W[n2] its lanes, at consecutive ny, would gather 32
+// different sectors: the planes are read in runs.  One gather fills a mode and its mirror across
+// kz = |nx|.  With planes instead of gathers the x/y passes of a 512^3 snapshot (61 radii, 3 grids)
+// went from 72.9 to 65.5 ms, of a 256^3 one (42 radii, 2 grids) from 3.69 to 3.35 ms; the planes take
+// 2.4 and 0.19 ms.
+__global__ void __launch_bounds__(256) k_window_planes(const float* __restrict__ rows, int n2max, int n,
+                                                       float* __restrict__ planes) {
+  const int h = n / 2 + 1, wp = wplane_pitch(n), kz = blockIdx.x;
+  const float* row = rows + (size_t)blockIdx.y * (n2max + 1) + kz * kz;
+  float* out = planes + blockIdx.y * wplane_size(n);
+  for (int nx = kz + threadIdx.x / 32; nx < h; nx += 8)
+    for (int ny = threadIdx.x % 32; ny < h; ny += 32) {
+      const float w = __ldg(row + nx * nx + ny * ny);
+      out[((size_t)kz * h + nx) * wp + ny] = w;
+      out[((size_t)nx * h + kz) * wp + ny] = w;
     }
-    for (int g = 0; g < ng; ++g) {
-      const cf* src = spec + g * stride;
-      cf* dst = work + ((size_t)r * ng + g) * stride;
-      line_fft<N, true>(
-          t, xbuf, s_tw,
-          [&](int p, int sl) {
-            const cf v = src[col + (size_t)p * N];
-            return cf{v.x * wv[sl], v.y * wv[sl]};
-          },
-          [&](int p) { return line_addr<N, B>(p, b); }, [&](int p, cf v) { dst[col + (size_t)p * N] = v; });
-    }
-  }
 }
 
 // ---------------------------------------------------------------------------
-// the barrier test
+// temperatures
 
 __device__ __forceinline__ float partial_T(float t_hi, float res_xh) {
   // ComputePartiallyIoinizedTemperature (find_HII_bubbles.c:76-84)
@@ -128,23 +89,30 @@ __device__ __forceinline__ float partial_T(float t_hi, float res_xh) {
   return (float)((double)(t_hi * res_xh) + T_RE * (1.0 - (double)res_xh));
 }
 
-__device__ float fully_ionized_T(float z_re, float z, float delta) {
-  // ComputeFullyIoinizedTemperature (find_HII_bubbles.c:48-74), with its float/double mix
+// ComputeFullyIoinizedTemperature (find_HII_bubbles.c:48-74), with its float/double mix.  The powers
+// of constants and of the redshift alone come from the host (HiiConst); the per-cell ones are
+// exp(c log(x)), within 1e-13 of x^c for the arguments here (|c log x| < 40), at a third of
+// pow's instructions: five pow a cell bounded the closing pass of a mostly ionised box.
+__device__ __forceinline__ double pow_pos(double x, double c) { return exp(c * log(x)); }
+
+__device__ __forceinline__ float fully_ionized_T(float z_re, float delta, const HiiConst& k) {
+  const float z = k.redshift;
   float result, delta_re;
   if (fabs((double)(z - z_re)) < 1e-4) {
     result = 1.f;
   } else {
+    const double ratio = (1.0 + (double)z) / (1.0 + (double)z_re);
     delta_re = (float)((double)delta * (1.0 + (double)z) / (1.0 + (double)z_re));
     if (delta_re <= -1.f) delta_re = (float)(-1.0 + (double)ABS_TOL);
     if (delta <= -1.f) delta = (float)(-1.0 + (double)ABS_TOL);
-    result = (float)pow((1.0 + (double)delta) / (1.0 + (double)delta_re), 1.1333);
-    result = (float)((double)result * pow((1.0 + (double)z) / (1.0 + (double)z_re), 3.4));
-    result *= expf((float)(pow((1.0 + (double)z) / 7.1, 2.5) - pow((1.0 + (double)z_re) / 7.1, 2.5)));
+    result = (float)pow_pos((1.0 + (double)delta) / (1.0 + (double)delta_re), 1.1333);
+    result = (float)((double)result * pow_pos(ratio, 3.4));
+    const double b = (1.0 + (double)z_re) / 7.1;
+    result *= expf((float)(k.z_25 - b * b * sqrt(b)));
   }
-  result = (float)((double)result * pow(T_RE, 1.7));
-  result = (float)((double)result + pow(1e4 * ((1.0 + (double)z) / 4.0), 1.7) * (double)(1.f + delta));
-  result = (float)pow((double)result, 0.5882);
-  return result;
+  result = (float)((double)result * k.t_17);
+  result = (float)((double)result + k.z_17 * (double)(1.f + delta));
+  return (float)pow_pos((double)result, 0.5882);
 }
 
 // Block sum of K doubles per thread into out[0..K), deterministic order.
@@ -179,44 +147,70 @@ __device__ __forceinline__ void block_sum(double (&acc)[K], double* out) {
   }
 }
 
-struct HiiBatch {
-  int nr;             // radii in this batch
-  int first;          // the batch starts the snapshot (state comes from z_at_ionization)
-  int ng;             // grids per radius (read by the instantiation for 5 to 7 grids)
-  double fcoll_pref[KB_MAX];
-  float J_aux[KB_MAX], J_aux_bh[KB_MAX];
-  float G_pref[KB_MAX], G_pref_bh[KB_MAX], R[KB_MAX];   // recombination branch
-  double fcoll_prefIII[KB_MAX];                          // Pop III (mini-halos)
-  float J_auxIII[KB_MAX], G_prefIII[KB_MAX];
-};
+// ---------------------------------------------------------------------------
+// closing pass (find_HII_bubbles.c:577-645): one cell a thread in memory order, so every access is
+// coalesced (in the z pass, whose threads hold a few cells of many rows, it took 5 ms of a 512^3
+// snapshot).  In: xH with the sign of "neutral at every radius" (the z pass).  A partly ionised
+// cell's temperature, ComputePartiallyIoinizedTemperature of the neutral gas's T at residual xH 1,
+// is that T: Tk_box with the spin temperature, else the adiabatic T; the floor is the same T.
+constexpr int CLOSE_NT = 256;
 
-struct HiiState {
-  float* xH;
-  float* z_in;
-  float* J21;
-  float* temp;
-  const float* Tk_box;
-  const float* deltax_unf;   // padded
-  const float* wsfr;         // padded
-  const float* bhar;         // padded, may be null
-  const float* wsfrIII;      // padded, Pop III only
-  float* Gamma12;            // recombination branch: written at a cell's first crossing
-  float* r_bubble;
-  uint8_t* st8;              // per cell between radius batches: bit 0 = z_at_ionization still < 0,
-                             // bit 1 = ionised at a radius of this snapshot
-  double* partials;          // [nblocks][HII_NSUM]
-};
+template <int N>
+__global__ void __launch_bounds__(CLOSE_NT) k_hii_close(HiiConst c, HiiState s, double* __restrict__ partials) {
+  constexpr int PADW = 2 * (N / 2 + 1);
+  const size_t n3 = (size_t)N * N * N;
+  double acc[HII_NSUM];
+#pragma unroll
+  for (int k = 0; k < HII_NSUM; ++k) acc[k] = 0.0;
+  for (size_t ir = (size_t)blockIdx.x * CLOSE_NT + threadIdx.x; ir < n3; ir += (size_t)gridDim.x * CLOSE_NT) {
+    const size_t ip = ir / N * PADW + ir % N;
+    const float xs = s.xH[ir], du = s.deltax_unf[ip], zin = s.z_in[ir], told = s.temp[ir], ws = s.wsfr[ip];
+    const bool neutral = signbit(xs);
+    const float xH = fabsf(xs);
+    const float tn = c.spin ? s.Tk_box[ir] : (float)((double)c.TK * (1.0 + (double)(c.cT_ad * du)));
+    float temp = neutral ? tn : told;
+    if (xH < REL_TOL && zin > 0.f) temp = fully_ionized_T(zin, du, c);
+    if (temp < tn) temp = tn;
+    if (neutral) s.xH[ir] = xH;
+    s.temp[ir] = temp;
+    const double domu = 1.0 + (double)du;
+    acc[0] += (double)xH;
+    // acc[1] and acc[6]: r_bubble is written only on the recombination branch
+    // (find_HII_bubbles.c:490-508); its sums come from k_hii_recomb.
+    acc[2] += (double)ws;
+    if (s.bhar != nullptr) acc[3] += (double)s.bhar[ip];
+    if (s.wsfrIII != nullptr) acc[9] += (double)s.wsfrIII[ip];
+    acc[4] += (double)temp;
+    acc[5] += (double)xH * domu;
+    acc[7] += (double)temp * domu;
+    acc[8] += domu;
+  }
+  block_sum<CLOSE_NT, HII_NSUM>(acc, partials + (size_t)blockIdx.x * HII_NSUM);
+}
 
-// Shared-memory plan of the z pass: ZB tile buffers of TB complex each; the buffer of the unit
+template <int N>
+int launch_hii_close(rg_context* ctx, const HiiConst& c, const HiiState& s, double* partials, int nblocks,
+                     cudaStream_t st) {
+  prof_begin(ctx, "hii_close", st);
+  k_hii_close<N><<<nblocks, CLOSE_NT, 0, st>>>(c, s, partials);
+  // xH, deltax, z_at_ionization, temperature, weighted_sfr (and Tk_box, ...) read, xH and temperature written
+  prof_end(ctx, 4.0 * N * N * N * (7 + c.spin + (s.bhar != nullptr) + (s.wsfrIII != nullptr)), st);
+  RG_CUDA_TRY(ctx, cudaGetLastError());
+  return RG_OK;
+}
+
+// ---------------------------------------------------------------------------
+// the z pass with Pop III sources, and of the boxes below 64^3: up to 9 grids a radius, in row buffers
+//
+// Shared-memory plan: ZB tile buffers of TB complex each; the buffer of the unit
 // being transformed is also its FFT exchange buffer (the tile is consumed by the first stage).
-// Two buffers let the next grid's tile arrive while this one is transformed.  At 512^3 the
-// batches before the last use one buffer instead, which brings a block to 72 KB and 77 registers
-// and the SM to three blocks (measured: 46.0 -> 44.0 ms over 7 batches; the closing batch, with
-// more registers, keeps two buffers).
-template <int N, bool FINAL>
+// Two buffers let the next grid's tile arrive while this one is transformed.  At 512^3 one buffer
+// brings a block to 72 KB and the SM to three blocks instead (46.0 -> 44.0 ms over 7 batches of 8
+// radii and 3 grids).
+template <int N>
 struct HiiZ {
   static constexpr int NTH = Cfg<N>::T * Cfg<N>::QZ;
-  static constexpr bool WIDE = N == 512 && !FINAL;
+  static constexpr bool WIDE = N == 512;
   static constexpr int ZB = WIDE ? 1 : 2;
   static constexpr int TB = round_up(cmax((int)ztile_elems<N>(), line_buf<N, Cfg<N>::QZ>()), 2);
   static constexpr int MINB = WIDE ? 3 : RG_MINB(NTH);
@@ -226,15 +220,14 @@ struct HiiZ {
   }
 };
 
-// z pass of a batch.  FINAL: the batch ends with the snapshot's last (unfiltered) radius.
+// z pass of a batch.
 // Grids in rt: 0 deltax, 1 stars, then x_e (spin temperature), then effective_bhm (BH), then
 // starsIII (Pop III), then with recombinations N_rec, weighted_sfr, effective_bhar (BH) and
-// weighted_sfrIII (Pop III).  NG is the number of grids; the EXT instantiation (recombinations or
-// Pop III) takes any count up to NG from bt.ng.
-template <int N, int NG, bool FINAL, bool EXT>
-__global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::QZ, (HiiZ<N, FINAL>::MINB))
-    k_hii_z(const cf* __restrict__ work, size_t stride, const cf* __restrict__ g_tw, HiiBatch bt, HiiConst c,
-            HiiState s) {
+// weighted_sfrIII (Pop III); bt.ng of them.
+template <int N>
+__global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::QZ, (HiiZ<N>::MINB))
+    k_hii_z(const cf* __restrict__ work, size_t stride, const cf* __restrict__ g_tw, HiiBatch bt, HiiBatchIII b3,
+            HiiConst c, HiiState s) {
   constexpr int T = Cfg<N>::T, Q = Cfg<N>::QZ, NTH = T * Q, ROWS = 2 * Q, RP = Cfg<N>::RT_PITCH;
   constexpr int PADW = 2 * (N / 2 + 1);
   constexpr int IT = ROWS * N / NTH;   // cells per thread
@@ -242,20 +235,19 @@ __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::QZ, (HiiZ<N, FINAL>::MINB))
   static_assert(ROWS * N % NTH == 0, "whole rows per block");
   extern __shared__ __align__(16) unsigned char smem_raw[];  // 16-byte aligned for cp.async
   cf* smem = reinterpret_cast<cf*>(smem_raw);
-  constexpr int ZB = HiiZ<N, FINAL>::ZB, TB = HiiZ<N, FINAL>::TB;
+  constexpr int ZB = HiiZ<N>::ZB, TB = HiiZ<N>::TB;
   cf* s_tw = smem;
   float* rt = reinterpret_cast<float*>(smem + N);
   // ZB shared tiles (with two, grid u + 1 is copied while grid u is transformed); the tile of
   // unit u is the exchange buffer of its transform
-  // (the EXT instantiation lays the tiles out after the row buffers of the grids it has)
-  cf* tiles = reinterpret_cast<cf*>(rt + round_up((EXT ? bt.ng : NG) * ROWS * RP, 4));
+  // (after the row buffers of the grids there are)
+  cf* tiles = reinterpret_cast<cf*>(rt + round_up(bt.ng * ROWS * RP, 4));
   const int x = blockIdx.y, y0 = blockIdx.x * ROWS;
-  const size_t blk = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
   load_twiddles<N>(s_tw, g_tw);
 
   // per-cell state bits: A = z_at_ionization still < 0, I = ionized at a radius of this snapshot.
   // Cell it of this thread is block cell threadIdx.x + it * NTH, bit it % 32 of word it / 32;
-  // between batches the state is one byte per cell (s.st8, bit 0 = A, bit 1 = I).
+  // between batches the state is one byte per cell (s.state, bit 0 = A, bit 1 = I).
   uint32_t A[W], I[W];
 #pragma unroll
   for (int w = 0; w < W; ++w) {
@@ -268,7 +260,7 @@ __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::QZ, (HiiZ<N, FINAL>::MINB))
       if (bt.first) {
         if (s.z_in[ir] < 0.f) a |= 1u << bb;
       } else {
-        const uint32_t v = s.st8[ir];
+        const uint32_t v = s.state[ir];
         a |= (v & 1u) << bb;
         iv |= ((v >> 1) & 1u) << bb;
       }
@@ -276,10 +268,8 @@ __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::QZ, (HiiZ<N, FINAL>::MINB))
     A[w] = a;
     I[w] = iv;
   }
-  // the Pop III and recombination grids (only the 9-grid instantiation runs with them, so the
-  // others compile without those branches)
-  const int ng = EXT ? bt.ng : NG;
-  const bool rec = EXT && c.rec, mini = EXT && c.mini;
+  const int ng = bt.ng;
+  const bool rec = c.rec, mini = c.mini;
   int gi = 2;
   const int gx = c.spin ? gi++ : -1;
   const int gb = c.bh ? gi++ : -1;
@@ -288,9 +278,6 @@ __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::QZ, (HiiZ<N, FINAL>::MINB))
   const int gw = rec ? gi++ : -1;                  // weighted_sfr
   const int gr = rec && c.bh ? gi++ : -1;          // effective_bhar
   const int gw3 = rec && mini ? gi++ : -1;         // weighted_sfrIII
-  double acc[FINAL ? HII_NSUM : 1];
-#pragma unroll
-  for (int k = 0; k < (FINAL ? HII_NSUM : 1); ++k) acc[k] = 0.0;
 
   const int nunits = bt.nr * ng;   // (radius, grid) pairs, unit u = r * ng + g
   ztile_issue<N, Q>(tiles, work, x, y0, NTH);
@@ -324,7 +311,7 @@ __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::QZ, (HiiZ<N, FINAL>::MINB))
         cp_async_commit();
       }
     }
-    const bool last = FINAL && r == bt.nr - 1;
+    const bool last = bt.last && r == bt.nr - 1;
     const double pref = bt.fcoll_pref[r];
 #pragma unroll
     for (int w = 0; w < W; ++w) {
@@ -364,13 +351,12 @@ __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::QZ, (HiiZ<N, FINAL>::MINB))
         // (f_bh + f_stars) * prefactor > nf (1 + rec) with f = grid / dom, tested with both
         // sides times dom: the two forms differ only within a few FP64 ulps of the barrier
         const double num = c.bh ? (double)bhm + (double)st : (double)st;
-        const double prefIII = gm >= 0 ? bt.fcoll_prefIII[r] : 0.0;
+        const double prefIII = gm >= 0 ? b3.fcoll_pref[r] : 0.0;
         const double lhs_dom = gm >= 0 ? num * pref + (double)stIII * prefIII : num * pref;
         const bool ion = lhs_dom > nf * (1.0 + rec) * dom;
         float xH = (iw & bit) ? 0.f : 1.f;   // so far: 0 once ionized at a radius, else 1
         const size_t cellrow = (size_t)x * N + y0 + row;
         const size_t ir = cellrow * N + z;
-        float temp_new = -1.f;               // >= 0: partial temperature written this radius
         if (ion) {
           if (gn >= 0 && !(iw & bit)) {
             // first crossing of the snapshot (find_HII_bubbles.c:488-508)
@@ -380,7 +366,7 @@ __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::QZ, (HiiZ<N, FINAL>::MINB))
             if (gw3 >= 0) {
               float w3 = fmaxf(rt[(gw3 * ROWS + row) * RP + z], 0.f);
               if (w3 < ABS_TOL) w3 = 0.f;
-              G = __fadd_rn(G, __fmul_rn(w3, bt.G_prefIII[r]));
+              G = __fadd_rn(G, __fmul_rn(w3, b3.G_pref[r]));
             }
             if (gr >= 0) {
               float bhr = fmaxf(rt[(gr * ROWS + row) * RP + z], 0.f);
@@ -391,7 +377,7 @@ __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::QZ, (HiiZ<N, FINAL>::MINB))
             s.r_bubble[ir] = bt.R[r];
             if (c.uvb == 2) {
               float j = __fmul_rn(st, bt.J_aux[r]);
-              if (gm >= 0) j = __fadd_rn(j, __fmul_rn(stIII, bt.J_auxIII[r]));
+              if (gm >= 0) j = __fadd_rn(j, __fmul_rn(stIII, b3.J_aux[r]));
               if (c.bh) j = __fadd_rn(j, __fmul_rn(bhm, bt.J_aux_bh[r]));
               s.J21[ir] = j;
             }
@@ -399,15 +385,7 @@ __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::QZ, (HiiZ<N, FINAL>::MINB))
           xH = 0.f;
           iw |= bit;
         } else if (last && xH > REL_TOL) {
-          // partially ionized: temperature of the neutral gas, xH = nf - f_coll prefactor
-          float thi;
-          if (c.spin) {
-            thi = s.Tk_box[ir];
-          } else {
-            const float du = s.deltax_unf[cellrow * PADW + z];
-            thi = (float)((double)c.TK * (1.0 + (double)(c.cT_ad * du)));
-          }
-          temp_new = partial_T(thi, xH);
+          // partially ionized: xH = nf - f_coll prefactor
           const double fcs = (double)st / dom;
           const double fbh = c.bh ? (double)bhm / dom : 0.0;
           const double lhs = (fbh + fcs) * pref;
@@ -415,56 +393,25 @@ __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::QZ, (HiiZ<N, FINAL>::MINB))
           if (gm >= 0) v -= (float)((double)stIII / dom * prefIII);   // a float subtraction in the C
           xH = v < 0.f ? 0.f : (v > 1.f ? 1.f : v);
         }
-        float zin_new = -1.f;                // > -1: set this radius
         if (xH < REL_TOL && (a & bit)) {
           // new ionization (find_HII_bubbles.c:531-543)
           a &= ~bit;
-          zin_new = c.redshift;
-          s.z_in[ir] = zin_new;
+          s.z_in[ir] = c.redshift;
           if (c.uvb == 1) {
             float j = st * bt.J_aux[r];
-            if (gm >= 0) j = __fadd_rn(j, __fmul_rn(stIII, bt.J_auxIII[r]));
+            if (gm >= 0) j = __fadd_rn(j, __fmul_rn(stIII, b3.J_aux[r]));
             if (c.bh) j += bhm * bt.J_aux_bh[r];
             s.J21[ir] = j;
           }
         }
-        if (FINAL && last) {
-          // closing pass (find_HII_bubbles.c:577-645)
-          const size_t ip = cellrow * PADW + z;
-          s.xH[ir] = xH;
-          const float du = s.deltax_unf[ip];
-          const double domu = 1.0 + (double)du;
-          float temp = temp_new >= 0.f ? temp_new : s.temp[ir];
-          if (xH < REL_TOL) {
-            const float zin = zin_new > -1.f ? zin_new : s.z_in[ir];
-            if (zin > 0.f) temp = fully_ionized_T(zin, c.redshift, du);
-          }
-          if (c.spin) {
-            const float tk = s.Tk_box[ir];
-            if (temp < tk) temp = tk;
-          } else {
-            const float thistk = (float)((double)c.TK * (1.0 + (double)(c.cT_ad * du)));
-            if (temp < thistk) temp = thistk;
-          }
-          s.temp[ir] = temp;
-          acc[0] += (double)xH;
-          // acc[1] and acc[6]: r_bubble is written only on the recombination branch
-          // (find_HII_bubbles.c:490-508); its sums come from k_hii_recomb.
-          acc[2] += (double)s.wsfr[ip];
-          if (s.bhar != nullptr) acc[3] += (double)s.bhar[ip];
-          if (s.wsfrIII != nullptr) acc[9] += (double)s.wsfrIII[ip];
-          acc[4] += (double)temp;
-          acc[5] += (double)xH * domu;
-          acc[7] += (double)temp * domu;
-          acc[8] += domu;
-        }
+        if (last) s.xH[ir] = (iw & bit) ? 0.f : -xH;   // the sign: neutral at every radius (k_hii_close)
       }
       A[w] = a;
       I[w] = iw;
     }
   }
 
-  if constexpr (!FINAL) {
+  if (!bt.last) {
 #pragma unroll
     for (int w = 0; w < W; ++w) {
       const int nb = IT - 32 * w < 32 ? IT - 32 * w : 32;
@@ -472,29 +419,28 @@ __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::QZ, (HiiZ<N, FINAL>::MINB))
       for (int bb = 0; bb < nb; ++bb) {
         const int i = threadIdx.x + (32 * w + bb) * NTH;
         const size_t ir = ((size_t)x * N + y0 + i / N) * N + i % N;
-        s.st8[ir] = (uint8_t)(((A[w] >> bb) & 1u) | (((I[w] >> bb) & 1u) << 1));
+        s.state[ir] = (uint8_t)(((A[w] >> bb) & 1u) | (((I[w] >> bb) & 1u) << 1));
       }
     }
-  } else {
-    block_sum<NTH, HII_NSUM>(acc, s.partials + blk * HII_NSUM);
   }
 }
 
-// deterministic second stage: one block sums the per-block partials in a fixed order
-__global__ void k_reduce_partials(const double* __restrict__ partials, int nblocks, int nsum, double* out) {
+// deterministic second stage: block (i, u) sums sum i of the per-block partials of set u in a fixed
+// order (one block for all the sums took 11 to 28 us)
+__global__ void __launch_bounds__(256) k_reduce_partials(const double* __restrict__ partials, int nblocks, int nsum,
+                                                         double* out, size_t set_pitch, int out_pitch) {
   __shared__ double sh[256];
-  for (int i = 0; i < nsum; ++i) {
-    double v = 0.0;
-    for (int b = threadIdx.x; b < nblocks; b += 256) v += partials[(size_t)b * nsum + i];
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-      if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) out[i] = sh[0];
+  const int i = blockIdx.x;
+  partials += blockIdx.y * set_pitch;
+  double v = 0.0;
+  for (int b = threadIdx.x; b < nblocks; b += 256) v += partials[(size_t)b * nsum + i];
+  sh[threadIdx.x] = v;
+  __syncthreads();
+  for (int w = 128; w > 0; w >>= 1) {
+    if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
     __syncthreads();
   }
+  if (threadIdx.x == 0) out[blockIdx.y * out_pitch + i] = sh[0];
 }
 
 // ---------------------------------------------------------------------------
@@ -632,465 +578,64 @@ static cudaError_t prep(K kernel, size_t smem) {
   return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
-template <int N>
-constexpr size_t smem_x() { return sizeof(cf) * (N + (size_t)line_buf<N, Cfg<N>::BX>()); }
-
-template <int N>
-int launch_forward(rg_context* ctx, const float* const* d_real, int ng, cf* spec, size_t stride, double scale,
-                   cudaStream_t st) {
-  const cf* tw;
-  int rc = twiddles_for(ctx, N, &tw);
-  if (rc) return rc;
-  using C = Cfg<N>;
-  GridPtrs src{};
-  for (int g = 0; g < ng; ++g) src.p[g] = d_real[g];
-  const double nzc = (double)C::NZ * N * N;
-  using ZF = ZFCfg<N>;
-  RG_CUDA_TRY(ctx, prep(k_fwd_z<N>, ZF::smem()));
-  prof_begin(ctx, "fwd_z_r2c", st);
-  k_fwd_z<N><<<dim3(N / (2 * ZF::QF), N, ng), ZF::NTH, ZF::smem(), st>>>(src, spec, stride, tw);
-  prof_end(ctx, ng * (4.0 * N * N * N + 8.0 * nzc), st);
-  RG_CUDA_TRY(ctx, cudaGetLastError());
-  prof_begin(ctx, "fwd_y_c2c", st);
-  RG_CUDA_TRY(ctx, (launch_pass_y<N, false>(spec, stride, ng, tw, st)));
-  prof_end(ctx, ng * 16.0 * nzc, st);
-  RG_CUDA_TRY(ctx, prep((k_pass_x<N, false>), smem_x<N>()));
-  prof_begin(ctx, "fwd_x_c2c", st);
-  k_pass_x<N, false><<<dim3(N / C::BX, C::NZ, ng), C::T * C::BX, smem_x<N>(), st>>>(spec, stride, tw, (float)scale);
-  prof_end(ctx, ng * 16.0 * nzc, st);
-  RG_CUDA_TRY(ctx, cudaGetLastError());
-  return RG_OK;
-}
-
-
-// f(std::integral_constant<int, I>{}) for I in the sequence, in order
-template <class F, int... I>
-__device__ __forceinline__ void for_each_index(std::integer_sequence<int, I...>, F&& f) {
-  (f(std::integral_constant<int, I>{}), ...);
-}
-
-// ---------------------------------------------------------------------------
-// z pass of a batch before the last one (no recombination or Pop III grid), with the tiles staged
-// by TMA and the barrier test on the transforms' registers.
-//
-// The block owns rows [y0, y0 + 2Q) of plane x.  For every (radius, grid) unit u of the batch, the
-// Hermitian half column tile (all kz, those rows) arrives in shared memory by tensor loads (ZB
-// tiles in flight, one mbarrier each); the c2r of its row pairs leaves each thread the same cells
-// of every grid (the transform's output positions do not depend on the grid), so the previous
-// grids' values are kept in registers and the clamp and barrier test run as the last grid's
-// values come out of the transform: no row buffer in shared memory.  The state of a cell
-// (z_at_ionization still < 0; ionised at a radius of this snapshot) is two bits in registers
-// within the batch and one byte per cell between batches.
-template <int N>
-struct HiiZR {
-  static constexpr int T = Cfg<N>::T, Q = Cfg<N>::QZ, NTH = T * Q, V = N / T;
-  static constexpr int NZ = N / 2 + 1;
-  // kz rows per tensor box (box dimensions are at most 256): one box, or for N = 512 two boxes of
-  // (NZ + 1) / 2 rows at kz 0 and kz NZ - KZB that overlap in one row, so the second box lands on
-  // a 128-byte boundary of the tile and no row lies outside the tensor
-  static constexpr int KZB = NZ <= 256 ? NZ : (NZ + 1) / 2;
-  static constexpr int NBOX = NZ <= 256 ? 1 : 2;
-  static constexpr int TB = round_up(cmax(NZ * 2 * Q, line_buf<N, Q>()), 16);   // 128-byte multiple
-  static constexpr int ZB = 3;                                 // tiles in flight
-  static constexpr uint32_t TX = (uint32_t)(NBOX * KZB * 2 * Q * sizeof(cf));   // bytes the boxes deliver
-  static_assert(NBOX == 1 || ((NZ - KZB) * 2 * Q * sizeof(cf)) % 128 == 0, "second box off a 128-byte boundary");
-  static constexpr size_t smem() { return 128 + sizeof(cf) * ((size_t)ZB * TB + N) + sizeof(uint64_t) * ZB; }
-  // resident blocks: register room for the kept grids (up to 3 x 2V floats) without spills; the
-  // closing batch also holds ten FP64 sums (three blocks still fit at 512^3)
-  template <bool FINAL>
-  static constexpr int minb() { return FINAL ? (NTH >= 256 ? 1 : (N >= 512 ? 3 : 2)) : (NTH >= 256 ? 2 : 3); }
-  // the sizes it serves: power-of-two grids of 64^3 and up (at most 16 values per thread)
-  static constexpr bool USED = (N == 64 || N == 128 || N == 256 || N == 512);
-  static_assert(2 * V <= 64, "two state bits per cell in 64-bit masks");
-};
-
-constexpr int TMA_WAIT_LIMIT = 1 << 22;   // polls of an mbarrier before a wait gives up
-
-// FINAL: the batch ends with the snapshot's last (unfiltered) radius: the partial xH of the
-// never-ionised cells, and the closing pass (temperatures, xH, FP64 sums into partials) as in
-// k_hii_z.
-template <int N, bool SPIN, bool BH, bool FINAL>
-__global__ void __launch_bounds__(HiiZR<N>::NTH, (HiiZR<N>::template minb<FINAL>()))
-    k_hii_zr(const __grid_constant__ CUtensorMap tmap, const cf* __restrict__ g_tw, HiiBatch bt, HiiConst c,
-             HiiState s, uint32_t* err) {
-  using Z = HiiZR<N>;
-  using PL = Plan<N>;
-  constexpr int Q = Z::Q, V = Z::V, ZB = Z::ZB, TB = Z::TB, NZ = Z::NZ, KZB = Z::KZB, NBOX = Z::NBOX;
-  constexpr int PADW = 2 * (N / 2 + 1);
-  constexpr int NG = 2 + SPIN + BH;          // deltax, stars, [x_e], [effective_bhm]
-  constexpr int GX = 2, GB = 2 + SPIN;       // grid indices of x_e and effective_bhm
-  extern __shared__ unsigned char smem_raw[];
-  unsigned char* sm = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
-  cf* tiles = reinterpret_cast<cf*>(sm);
-  cf* s_tw = tiles + ZB * TB;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_tw + N);
-  const int x = blockIdx.y, y0 = blockIdx.x * 2 * Q;
-  const int q = threadIdx.x % Q, tq = threadIdx.x / Q;
-  const int nunits = bt.nr * NG;
-
-  if (threadIdx.x == 0) {
-    for (int b = 0; b < ZB; ++b) mbar_init(&bars[b], 1);
-    mbar_init_fence();
-  }
-  load_twiddles<N>(s_tw, g_tw);
-  __syncthreads();
-  // thread 0: tensor loads of unit u into tile u % ZB (tensor coordinates: y in floats, x, kz of
-  // the unit's spectrum stacked after the previous units)
-  auto issue = [&](int u) {
-    const int b = u % ZB;
-    mbar_arrive_expect_tx(&bars[b], Z::TX);
-#pragma unroll
-    for (int k = 0; k < NBOX; ++k) {
-      const int k0 = k ? NZ - KZB : 0;
-      tma_load_3d(tiles + b * TB + k0 * 2 * Q, &tmap, 2 * y0, x, u * NZ + k0, &bars[b]);
-    }
-  };
-  if (threadIdx.x == 0)
-    for (int u = 0; u < ZB && u < nunits; ++u) issue(u);
-
-  // state of this thread's 2V cells: cell 2 slot + h is row y0 + 2q + h at z = last_pos(tq, slot)
-  uint64_t A = 0, I = 0, P = 0;   // P: partly ionised at the closing radius
-#pragma unroll
-  for (int slot = 0; slot < V; ++slot) {
-    const int z = last_pos<PL>(tq, slot);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const size_t ir = ((size_t)x * N + y0 + 2 * q + h) * N + z;
-      const uint64_t bit = 1ull << (2 * slot + h);
-      if (bt.first) {
-        if (s.z_in[ir] < 0.f) A |= bit;
-      } else {
-        const uint32_t v = s.st8[ir];
-        if (v & 1u) A |= bit;
-        if (v & 2u) I |= bit;
-      }
-    }
-  }
-
-  const uint64_t A0 = A;
-  float vals[NG - 1][2 * V];   // the transformed grids before the last one, for the radius in work
-  double acc[FINAL ? HII_NSUM : 1];
-#pragma unroll
-  for (int k = 0; k < (FINAL ? HII_NSUM : 1); ++k) acc[k] = 0.0;
-  bool waited = true;
-  int u = 0;
-  for (int r = 0; r < bt.nr; ++r) {
-    const double pref = bt.fcoll_pref[r];
-    const float jaux = bt.J_aux[r], jaux_bh = bt.J_aux_bh[r];
-    const bool lastr = FINAL && r == bt.nr - 1;
-    // one (radius, grid) unit; the grid index is a compile-time constant (register arrays)
-    auto unit = [&](auto gconst) {
-      constexpr int g = decltype(gconst)::value;
-      const int b = u % ZB;
-      cf* tile = tiles + b * TB;
-      if (!mbar_wait(&bars[b], (uint32_t)((u / ZB) & 1), TMA_WAIT_LIMIT)) waited = false;
-      line_fft_p<PL, true>(
-          tq, tile, s_tw, [&](int p, int) { return ztile_c2r_input<N, Q>(tile, q, p); },
-          [&](int p) { return line_addr<N, Q>(p, q); },
-          [&](int z, cf v, int slot) {
-            if constexpr (g < NG - 1) {
-              vals[g][2 * slot] = v.x;
-              vals[g][2 * slot + 1] = v.y;
-            } else {
-#pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                const float last = h ? v.y : v.x;
-                auto val = [&](auto gi) -> float {
-                  constexpr int gg = decltype(gi)::value;
-                  if constexpr (gg == NG - 1) return last;
-                  else return vals[gg][2 * slot + h];
-                };
-                // the aliasing clamp (find_HII_bubbles.c:373-422) and the barrier test of
-                // k_hii_z without recombinations or Pop III
-                const float dx = fmaxf(val(std::integral_constant<int, 0>{}), -1.f + REL_TOL);
-                float st = fmaxf(val(std::integral_constant<int, 1>{}), 0.f);
-                if (st < ABS_TOL) st = 0.f;
-                float xe = 0.f, bhm = 0.f;
-                if constexpr (SPIN) {
-                  xe = fmaxf(val(std::integral_constant<int, GX>{}), 0.f);
-                  if (xe < ABS_TOL) xe = 0.f;
-                  xe = fminf(xe, 0.999f);
-                }
-                if constexpr (BH) {
-                  bhm = fmaxf(val(std::integral_constant<int, GB>{}), 0.f);
-                  if (bhm < ABS_TOL) bhm = 0.f;
-                }
-                const double dom = 1.0 + (double)dx;
-                const double nf = SPIN ? 1.0 - (double)xe : 1.0;
-                const double num = BH ? (double)bhm + (double)st : (double)st;
-                const bool ion = num * pref > nf * (1.0 + 0.0) * dom;
-                const uint64_t bit = 1ull << (2 * slot + h);
-                const size_t cellrow = (size_t)x * N + y0 + 2 * q + h;
-                const size_t ir = cellrow * N + z;
-                float xH = (I & bit) ? 0.f : 1.f;   // so far: 0 once ionized at a radius, else 1
-                if (ion) {
-                  I |= bit;
-                  xH = 0.f;
-                } else if (lastr && xH > REL_TOL) {
-                  // partially ionized: xH = nf - f_coll prefactor; its temperature is that of the
-                  // neutral gas (the closing pass below)
-                  P |= bit;
-                  const double fcs = (double)st / dom;
-                  const double fbh = BH ? (double)bhm / dom : 0.0;
-                  const float v = (float)(nf - (fbh + fcs) * pref);
-                  xH = v < 0.f ? 0.f : (v > 1.f ? 1.f : v);
-                }
-                if (xH < REL_TOL && (A & bit)) {
-                  // new ionization (find_HII_bubbles.c:531-543)
-                  A &= ~bit;
-                  s.z_in[ir] = c.redshift;
-                  if (c.uvb == 1) {
-                    float j = st * jaux;
-                    if (BH) j += bhm * jaux_bh;
-                    s.J21[ir] = j;
-                  }
-                }
-                // the cell's deltax is used: its register keeps the final xH for the closing pass
-                if constexpr (FINAL) {
-                  if (lastr) vals[0][2 * slot + h] = xH;
-                }
-              }
-            }
-          });
-      // every thread is done with tile b (read by the first stage, exchange buffer after that):
-      // order those generic accesses before the tensor load that refills it
-      fence_proxy_async_smem();
-      __syncthreads();
-      if (threadIdx.x == 0 && u + ZB < nunits) issue(u + ZB);
-      ++u;
-    };
-    for_each_index(std::make_integer_sequence<int, NG>{}, unit);
-  }
-  if (!waited && threadIdx.x % 32 == 0) atomicExch(err, 1u);
-  if constexpr (FINAL) {
-    // closing pass (find_HII_bubbles.c:577-645) of this thread's cells, four slots at a time with
-    // their loads issued together.  z_at_ionization is this snapshot's redshift where this batch
-    // set it (A0 & ~A), else it is read (not written by this kernel).  A partly ionised cell's
-    // temperature, ComputePartiallyIoinizedTemperature of the neutral gas's T at residual xH 1,
-    // is that T: Tk_box with the spin temperature, else the adiabatic T; the floor is the same T.
-    constexpr int CH = 4;
-#pragma unroll
-    for (int s0 = 0; s0 < V; s0 += CH) {
-      float du[2 * CH], tk[2 * CH], tp[2 * CH], zi[2 * CH], ws[2 * CH], bh[2 * CH];
-#pragma unroll
-      for (int j = 0; j < 2 * CH; ++j) {
-        const int slot = s0 + j / 2, h = j % 2;
-        const uint64_t bit = 1ull << (2 * slot + h);
-        const size_t cellrow = (size_t)x * N + y0 + 2 * q + h;
-        const int z = last_pos<PL>(tq, slot);
-        const size_t ir = cellrow * N + z, ip = cellrow * PADW + z;
-        const float xH = vals[0][2 * slot + h];
-        du[j] = s.deltax_unf[ip];
-        ws[j] = s.wsfr[ip];
-        bh[j] = s.bhar != nullptr ? s.bhar[ip] : 0.f;
-        tk[j] = SPIN ? s.Tk_box[ir] : 0.f;
-        tp[j] = (P & bit) ? 0.f : s.temp[ir];
-        zi[j] = (xH < REL_TOL && !((A0 & ~A) & bit)) ? s.z_in[ir] : c.redshift;
-      }
-#pragma unroll
-      for (int j = 0; j < 2 * CH; ++j) {
-        const int slot = s0 + j / 2, h = j % 2;
-        const uint64_t bit = 1ull << (2 * slot + h);
-        const size_t cellrow = (size_t)x * N + y0 + 2 * q + h;
-        const size_t ir = cellrow * N + last_pos<PL>(tq, slot);
-        const float xH = vals[0][2 * slot + h];
-        const float tn = SPIN ? tk[j] : (float)((double)c.TK * (1.0 + (double)(c.cT_ad * du[j])));
-        float temp = (P & bit) ? tn : tp[j];
-        if (xH < REL_TOL && zi[j] > 0.f) temp = fully_ionized_T(zi[j], c.redshift, du[j]);
-        if (temp < tn) temp = tn;
-        s.xH[ir] = xH;
-        s.temp[ir] = temp;
-        const double domu = 1.0 + (double)du[j];
-        acc[0] += (double)xH;
-        acc[2] += (double)ws[j];
-        acc[3] += (double)bh[j];
-        acc[4] += (double)temp;
-        acc[5] += (double)xH * domu;
-        acc[7] += (double)temp * domu;
-        acc[8] += domu;
-      }
-    }
-    block_sum<Z::NTH, HII_NSUM>(acc, s.partials + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * HII_NSUM);
-  } else {
-#pragma unroll
-    for (int slot = 0; slot < V; ++slot) {
-      const int z = last_pos<PL>(tq, slot);
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const size_t ir = ((size_t)x * N + y0 + 2 * q + h) * N + z;
-        const int sh = 2 * slot + h;
-        s.st8[ir] = (uint8_t)(((A >> sh) & 1ull) | (((I >> sh) & 1ull) << 1));
-      }
-    }
-  }
-}
-
-// the batch of the fused x/y pass: grid g of spec windowed for radius r into work (r ng + g)
-// The grids may be several snapshots' (ngu grids each, the same radii): the work buffer holds
-// snapshot u's block [radius][its grids] at u nr ngu (one snapshot: [radius][grid]).
-struct HiiXOp {
-  const cf* spec;
-  size_t stride;
-  int ng;
-  int ngu;           // grids per snapshot
-  int nr;            // radii of the batch
-  cf* work;
-  const float* wrows;
-  int wpitch;
-  int unfiltered;
-  const int* wcut;   // sharp-k step ends per radius, or null (window rows are read)
-  __device__ int grids() const { return ng; }
-  __device__ bool filtered(int r) const { return r != unfiltered; }
-  __device__ const float* wrow(int r) const { return wrows + (size_t)r * wpitch; }
-  __device__ int cutoff(int r) const { return wcut ? __ldg(wcut + r) : -2; }
-  __device__ cf* out(int r, int g) const {
-    const int u = g / ngu;
-    return work + (((size_t)u * nr + r) * ngu + (g - u * ngu)) * stride;
-  }
-};
-
-// inverse x (window, batch of nr radii) and y passes: one fused kernel, or (plain mode) the two
-// passes as separate kernels
-template <int N>
-int launch_inverse_xy(rg_context* ctx, const cf* spec, int ng, int ngu, cf* work, size_t stride, int nr,
-                      const float* wrows, int wpitch, int unfiltered, cudaStream_t st, const int* wcut = nullptr) {
-  using C = Cfg<N>;
-  const double nzc = (double)C::NZ * N * N;
-  if (ctx->mode == RG_MODE_FUSED) {
-    const HiiXOp op{spec, stride, ng, ngu, nr, work, wrows, wpitch, unfiltered, wcut};
-    if (stride != (size_t)C::NZ * N * N) return set_error(ctx, RG_EINVAL, "fused x/y pass: spectra must be contiguous");
-    return launch_xy_fused<N>(ctx, op, spec, ng, nr, "inv_xy_c2c_window", ng * 8.0 * nzc * (1 + nr), st);
-  }
-  if (ngu != ng) return set_error(ctx, RG_EINVAL, "several snapshots in one pass need the fused mode");
-  const cf* tw;
-  int rc = twiddles_for(ctx, N, &tw);
-  if (rc) return rc;
-  RG_CUDA_TRY(ctx, prep(k_hii_x<N>, smem_x<N>()));
-  prof_begin(ctx, "inv_x_c2c_window", st);
-  k_hii_x<N><<<dim3(N / C::BX, C::NZ), C::T * C::BX, smem_x<N>(), st>>>(spec, stride, ng, work, nr, wrows, wpitch,
-                                                                        unfiltered, tw);
-  prof_end(ctx, ng * 8.0 * nzc * (1 + nr), st);
-  RG_CUDA_TRY(ctx, cudaGetLastError());
-  prof_begin(ctx, "inv_y_c2c", st);
-  RG_CUDA_TRY(ctx, (launch_pass_y<N, true>(work, stride, ng * nr, tw, st)));
-  prof_end(ctx, ng * nr * 16.0 * nzc, st);
-  return RG_OK;
-}
-
-// grids one EXT z pass can hold at this size: the most, up to 9, whose row buffers fit the
+// grids k_hii_z can hold at this size: the most, up to 9, whose row buffers fit the
 // 227 KB of shared memory a block may use (7 at 384^3, 8 at 192^3)
 template <int N>
 constexpr int hii_ngx() {
   int ng = 9;
-  while (ng > 4 && HiiZ<N, true>::smem(ng) > 227 * 1024) --ng;
+  while (ng > 4 && HiiZ<N>::smem(ng) > 227 * 1024) --ng;
   return ng;
 }
 
-template <int N, int NG, bool FINAL, bool EXT = false>
-int launch_hii_z3(rg_context* ctx, const cf* work, size_t stride, const HiiBatch& bt, const HiiConst& c,
-                  const HiiState& s, cudaStream_t st, int* nblocks) {
+template <int N>
+int launch_hii_zrow(rg_context* ctx, const cf* work, size_t stride, const HiiZUnit& u, const HiiBatchIII& b3,
+                    cudaStream_t st) {
   const cf* tw;
   int rc = twiddles_for(ctx, N, &tw);
   if (rc) return rc;
   using C = Cfg<N>;
-  static_assert(HiiZ<N, FINAL>::smem(NG) <= 227 * 1024, "z pass shared memory above the per-block limit");
-  // the EXT instantiation takes the shared memory of the grids it has, not of its maximum
-  const size_t sm = HiiZ<N, FINAL>::smem(EXT ? bt.ng : NG);
-  RG_CUDA_TRY(ctx, prep(k_hii_z<N, NG, FINAL, EXT>, HiiZ<N, FINAL>::smem(NG)));
+  const HiiBatch& bt = u.bt;
+  if (bt.ng > hii_ngx<N>())
+    return set_error(ctx, RG_EUNSUPPORTED,
+                     "this combination of grids (recombinations, Pop III, BH feedback, spin temperature) needs "
+                     "more row buffers than one z pass holds at this ReionGridDim");
+  static_assert(HiiZ<N>::smem(hii_ngx<N>()) <= 227 * 1024, "z pass shared memory above the per-block limit");
+  // the shared memory of the grids there are, not of the maximum
+  const size_t sm = HiiZ<N>::smem(bt.ng);
+  RG_CUDA_TRY(ctx, prep(k_hii_z<N>, HiiZ<N>::smem(hii_ngx<N>())));
   const dim3 grid(N / (2 * C::QZ), N);
-  // algorithmic bytes: the Hermitian halves of NG grids per radius, z_at_ionization on the
-  // first batch; the closing pass writes xH and temperature and reads deltax, weighted_sfr,
-  // [effective_bhar], [Tk_box]
+  // algorithmic bytes: the Hermitian halves of the grids per radius, z_at_ionization on the
+  // first batch, xH at the end
   const double n3 = (double)N * N * N, nzc = (double)C::NZ * N * N;
-  double bytes = bt.nr * (EXT ? bt.ng : NG) * 8.0 * nzc + (bt.first ? 4.0 * n3 : 0.0);
-  if (FINAL) bytes += 4.0 * n3 * (2 + 2 + (s.bhar != nullptr) + (s.Tk_box != nullptr));
-  prof_begin(ctx, FINAL ? "inv_z_c2r_test_final" : "inv_z_c2r_test", st);
-  k_hii_z<N, NG, FINAL, EXT><<<grid, C::T * C::QZ, sm, st>>>(work, stride, tw, bt, c, s);
-  prof_end(ctx, bytes, st);
+  prof_begin(ctx, bt.last ? "inv_z_c2r_test_final" : "inv_z_c2r_test", st);
+  k_hii_z<N><<<grid, C::T * C::QZ, sm, st>>>(work, stride, tw, bt, b3, u.c, u.s);
+  prof_end(ctx, bt.nr * bt.ng * 8.0 * nzc + (bt.first || bt.last ? 4.0 * n3 : 2.0 * n3), st);
   RG_CUDA_TRY(ctx, cudaGetLastError());
-  if (nblocks) *nblocks = (int)(grid.x * grid.y);
   return RG_OK;
 }
 
-template <int N, bool SPIN, bool BH, bool FINAL>
-int launch_hii_zr3(rg_context* ctx, const cf* work, const HiiBatch& bt, const HiiConst& c, const HiiState& s,
-                   cudaStream_t st, int* nblocks) {
-  using Z = HiiZR<N>;
-  constexpr int NG = 2 + SPIN + BH;
-  const cf* tw;
-  int rc = twiddles_for(ctx, N, &tw);
-  if (rc) return rc;
-  // the batch's units as one 3-D float tensor: y (2N floats), x (N), kz of unit u at u NZ + kz
-  CUtensorMap map;
-  const uint64_t dims[3] = {2ull * N, (uint64_t)N, (uint64_t)Z::NZ * bt.nr * NG};
-  const uint64_t strides[2] = {8ull * N, 8ull * N * N};
-  const uint32_t box[3] = {4u * Z::Q, 1u, (uint32_t)Z::KZB};
-  const int mrc = tma_map_3d(&map, work, dims, strides, box);
-  if (mrc != 0) return set_error(ctx, RG_ECUDA, "cuTensorMapEncodeTiled failed (" + std::to_string(mrc) + ")");
-  auto kern = k_hii_zr<N, SPIN, BH, FINAL>;
-  RG_CUDA_TRY(ctx, prep(kern, Z::smem()));
-  const dim3 grid(N / (2 * Z::Q), N);
-  const double n3 = (double)N * N * N, nzc = (double)Z::NZ * N * N;
-  // algorithmic bytes: the Hermitian halves of NG grids per radius, the state (z_at_ionization on
-  // the first batch, one byte per cell read otherwise, one written before the closing batch); the
-  // closing pass writes xH and temperature and reads deltax, weighted_sfr, [effective_bhar], the
-  // temperature and [Tk_box]
-  double bytes = bt.nr * NG * 8.0 * nzc + (bt.first ? 4.0 * n3 : 1.0 * n3) + (FINAL ? 0.0 : 1.0 * n3);
-  if (FINAL) bytes += 4.0 * n3 * (2 + 3 + (s.bhar != nullptr) + SPIN);
-  prof_begin(ctx, FINAL ? "inv_z_c2r_test_final" : "inv_z_c2r_test", st);
-  kern<<<grid, Z::NTH, Z::smem(), st>>>(map, tw, bt, c, s, ctx->xy_ctrl);
-  prof_end(ctx, bytes, st);
-  RG_CUDA_TRY(ctx, cudaGetLastError());
-  if (nblocks) *nblocks = (int)(grid.x * grid.y);
-  return RG_OK;
-}
-
+// the z pass of one batch for nu snapshots (one with Pop III sources: b3), whose windowed spectra lie
+// one after another in work
 template <int N>
-int launch_hii_z(rg_context* ctx, const cf* work, size_t stride, int ng, const HiiBatch& bt, const HiiConst& c,
-                 const HiiState& s, bool fin, cudaStream_t st, int* nblocks) {
-  // without recombinations or Pop III: TMA tiles, registers
+int launch_hii_z(rg_context* ctx, const cf* work, size_t stride, int ng, int nu, const HiiZUnits& us,
+                 const HiiBatchIII& b3, cudaStream_t st) {
   if constexpr (HiiZR<N>::USED) {
-    if (!c.rec && !c.mini) {
-      if (fin) {
-        if (c.spin && c.bh) return launch_hii_zr3<N, true, true, true>(ctx, work, bt, c, s, st, nblocks);
-        if (c.spin) return launch_hii_zr3<N, true, false, true>(ctx, work, bt, c, s, st, nblocks);
-        if (c.bh) return launch_hii_zr3<N, false, true, true>(ctx, work, bt, c, s, st, nblocks);
-        return launch_hii_zr3<N, false, false, true>(ctx, work, bt, c, s, st, nblocks);
-      }
-      if (c.spin && c.bh) return launch_hii_zr3<N, true, true, false>(ctx, work, bt, c, s, st, nblocks);
-      if (c.spin) return launch_hii_zr3<N, true, false, false>(ctx, work, bt, c, s, st, nblocks);
-      if (c.bh) return launch_hii_zr3<N, false, true, false>(ctx, work, bt, c, s, st, nblocks);
-      return launch_hii_zr3<N, false, false, false>(ctx, work, bt, c, s, st, nblocks);
-    }
+    if (!us.u[0].c.mini) return launch_hii_zr<N>(ctx, work, nu, us, st);
   }
-  // with recombinations or Pop III (up to 9 grids) one instantiation reads the count from the
-  // batch
-  if (c.rec || c.mini) {
-    constexpr int NGX = hii_ngx<N>();
-    if (ng > NGX)
-      return set_error(ctx, RG_EUNSUPPORTED,
-                       "this combination of grids (recombinations, Pop III, BH feedback, spin temperature) needs "
-                       "more row buffers than one z pass holds at this ReionGridDim");
-    return fin ? launch_hii_z3<N, NGX, true, true>(ctx, work, stride, bt, c, s, st, nblocks)
-               : launch_hii_z3<N, NGX, false, true>(ctx, work, stride, bt, c, s, st, nblocks);
+  for (int k = 0; k < nu; ++k) {
+    const int rc =
+        launch_hii_zrow<N>(ctx, work + (size_t)k * us.u[k].bt.nr * ng * stride, stride, us.u[k], b3, st);
+    if (rc) return rc;
   }
-  if (ng == 2)
-    return fin ? launch_hii_z3<N, 2, true>(ctx, work, stride, bt, c, s, st, nblocks)
-               : launch_hii_z3<N, 2, false>(ctx, work, stride, bt, c, s, st, nblocks);
-  if (ng == 3)
-    return fin ? launch_hii_z3<N, 3, true>(ctx, work, stride, bt, c, s, st, nblocks)
-               : launch_hii_z3<N, 3, false>(ctx, work, stride, bt, c, s, st, nblocks);
-  return fin ? launch_hii_z3<N, 4, true>(ctx, work, stride, bt, c, s, st, nblocks)
-             : launch_hii_z3<N, 4, false>(ctx, work, stride, bt, c, s, st, nblocks);
+  return RG_OK;
 }
 
-
 template <int N>
-int launch_debug_inverse(rg_context* ctx, const cf* spec, cf* work, const float* wrow, float* out, cudaStream_t st) {
+int launch_debug_inverse(rg_context* ctx, const cf* spec, cf* work, const float* wplane, float* out, cudaStream_t st) {
   const size_t stride = (size_t)Cfg<N>::NZ * N * N;
   int rc = xy_ctrl_reset(ctx, Cfg<N>::NZ, st);
   if (rc) return rc;
-  rc = launch_inverse_xy<N>(ctx, spec, 1, 1, work, stride, 1, wrow, 0, wrow ? -1 : 0, st);
+  rc = inverse_xy(ctx, N, spec, 1, 1, work, stride, 1, wplane, wplane ? -1 : 0, st, nullptr);
   if (rc) return rc;
   const cf* tw;
   if ((rc = twiddles_for(ctx, N, &tw))) return rc;
@@ -1102,56 +647,18 @@ int launch_debug_inverse(rg_context* ctx, const cf* spec, cf* work, const float*
   return RG_OK;
 }
 
-#define RG_DISPATCH_N(n, call)                                                   \
-  switch (n) {                                                                   \
-    case 8: { constexpr int NN = 8; return call; }                               \
-    case 16: { constexpr int NN = 16; return call; }                             \
-    case 24: { constexpr int NN = 24; return call; }                             \
-    case 32: { constexpr int NN = 32; return call; }                             \
-    case 48: { constexpr int NN = 48; return call; }                             \
-    case 64: { constexpr int NN = 64; return call; }                             \
-    case 96: { constexpr int NN = 96; return call; }                             \
-    case 128: { constexpr int NN = 128; return call; }                           \
-    case 192: { constexpr int NN = 192; return call; }                           \
-    case 256: { constexpr int NN = 256; return call; }                           \
-    case 384: { constexpr int NN = 384; return call; }                           \
-    case 512: { constexpr int NN = 512; return call; }                           \
-    default: return set_error(ctx, RG_EUNSUPPORTED, "ReionGridDim not in {8,16,24,32,48,64,96,128,192,256,384,512}"); \
-  }
-
-#define RG_DISPATCH_N_VAL(n, call, dflt)       \
-  switch (n) {                                 \
-    case 8: { constexpr int NN = 8; return call; } \
-    case 16: { constexpr int NN = 16; return call; } \
-    case 24: { constexpr int NN = 24; return call; } \
-    case 32: { constexpr int NN = 32; return call; } \
-    case 48: { constexpr int NN = 48; return call; } \
-    case 64: { constexpr int NN = 64; return call; } \
-    case 96: { constexpr int NN = 96; return call; } \
-    case 128: { constexpr int NN = 128; return call; } \
-    case 192: { constexpr int NN = 192; return call; } \
-    case 256: { constexpr int NN = 256; return call; } \
-    case 384: { constexpr int NN = 384; return call; } \
-    case 512: { constexpr int NN = 512; return call; } \
-    default: return dflt;                      \
-  }
-
-int fft_forward(rg_context* ctx, int n, const float* const* d_real, int ng, cf* spec, size_t stride, double scale,
-                cudaStream_t st) {
-  if (ng > MAXG) return set_error(ctx, RG_EINVAL, "too many grids in one forward launch");
-  RG_DISPATCH_N(n, launch_forward<NN>(ctx, d_real, ng, spec, stride, scale, st));
+static int hii_z(rg_context* ctx, int n, const cf* work, size_t stride, int ng, int nu, const HiiZUnits& us,
+                 const HiiBatchIII& b3, cudaStream_t st) {
+  RG_DISPATCH_N(n, launch_hii_z<NN>(ctx, work, stride, ng, nu, us, b3, st));
 }
 
-static int inverse_xy(rg_context* ctx, int n, const cf* spec, int ng, int ngu, cf* work, size_t stride, int nr,
-                      const float* wrows, int wpitch, int unfiltered, cudaStream_t st, const int* wcut) {
-  RG_DISPATCH_N(n, launch_inverse_xy<NN>(ctx, spec, ng, ngu, work, stride, nr, wrows, wpitch, unfiltered, st, wcut));
-}
+// snapshots one z launch takes at this size
+static int hii_z_units(int n) { return n <= 128 ? HII_ZU : 1; }
 
-static int hii_z(rg_context* ctx, int n, const cf* work, size_t stride, int ng, const HiiBatch& bt, const HiiConst& c,
-                 const HiiState& s, bool fin, cudaStream_t st, int* nblocks) {
-  RG_DISPATCH_N(n, launch_hii_z<NN>(ctx, work, stride, ng, bt, c, s, fin, st, nblocks));
+static int hii_close(rg_context* ctx, int n, const HiiConst& c, const HiiState& s, double* partials, int nblocks,
+                     cudaStream_t st) {
+  RG_DISPATCH_N(n, launch_hii_close<NN>(ctx, c, s, partials, nblocks, st));
 }
-
 
 static int hii_recomb(rg_context* ctx, int n, const RecTables& tab, const RecConst& c, const RecState& s,
                       double* partials, int nblocks, cudaStream_t st) {
@@ -1170,10 +677,20 @@ int window_table(rg_context* ctx, double box, const double* d_radii, int nr, int
   return RG_OK;
 }
 
-int reduce_partials(rg_context* ctx, const double* partials, int nblocks, int nsum, double* d_out, cudaStream_t st) {
+int window_planes(rg_context* ctx, int n, const float* wrows, int nr, float* planes, cudaStream_t st) {
+  const int n2max = 3 * (n / 2) * (n / 2);
+  prof_begin(ctx, "window_planes", st);
+  k_window_planes<<<dim3(n / 2 + 1, nr), 256, 0, st>>>(wrows, n2max, n, planes);
+  prof_end(ctx, 4.0 * wplane_size(n) * nr, st);
+  RG_CUDA_TRY(ctx, cudaGetLastError());
+  return RG_OK;
+}
+
+int reduce_partials(rg_context* ctx, const double* partials, int nblocks, int nsum, double* d_out, cudaStream_t st,
+                    int sets, size_t set_pitch, int out_pitch) {
   prof_begin(ctx, "reduce_partials", st);
-  k_reduce_partials<<<1, 256, 0, st>>>(partials, nblocks, nsum, d_out);
-  prof_end(ctx, 8.0 * nblocks * nsum, st);
+  k_reduce_partials<<<dim3(nsum, sets), 256, 0, st>>>(partials, nblocks, nsum, d_out, set_pitch, out_pitch);
+  prof_end(ctx, 8.0 * nblocks * nsum * sets, st);
   RG_CUDA_TRY(ctx, cudaGetLastError());
   return RG_OK;
 }
@@ -1211,12 +728,16 @@ static int hii_const(rg_context* ctx, const rg_params* p, double redshift, HiiCo
   c->bh = p->Flag_BHFeedback != 0;
   c->rec = p->Flag_IncludeRecombinations != 0;
   c->mini = p->UseMiniHalos != 0;
+  const double opz = 1.0 + (double)c->redshift;
+  c->t_17 = std::pow(T_RE, 1.7);
+  c->z_17 = std::pow(1e4 * (opz / 4.0), 1.7);
+  c->z_25 = std::pow(opz / 7.1, 2.5);
   return RG_OK;
 }
 
 // the per-radius prefactors of radii [r0, r0 + cnt) (find_HII_bubbles.c:430-450)
 static void hii_batch_radii(const rg_params* p, double redshift, const std::vector<std::pair<double, bool>>& sched,
-                            int r0, int cnt, int ntest, HiiBatch* bt) {
+                            int r0, int cnt, int ntest, HiiBatch* bt, HiiBatchIII* b3) {
   const int N = p->ReionGridDim;
   const double pixel_volume = std::pow(p->BoxSize / (double)N, 3);
   const Units u = make_units(p);
@@ -1224,6 +745,7 @@ static void hii_batch_radii(const rg_params* p, double redshift, const std::vect
   std::memset(bt, 0, sizeof(*bt));
   bt->nr = cnt;
   bt->first = (r0 == 0);
+  bt->last = (r0 + cnt == (int)sched.size());
   bt->ng = ntest;
   for (int k = 0; k < cnt; ++k) {
     const double R = sched[r0 + k].first;
@@ -1242,9 +764,9 @@ static void hii_batch_radii(const rg_params* p, double redshift, const std::vect
     bt->R[k] = (float)R;
     bt->fcoll_pref[k] = p->ReionEfficiency * (4.0 / 3.0) * M_PI / pixel_volume / M_mean * R * R * R;
     // Pop III (find_HII_bubbles.c:443-450): photons per baryon and efficiency of their own
-    bt->J_auxIII[k] = bt->J_aux[k] * (float)(p->ReionNionPhotPerBaryIII / p->ReionNionPhotPerBary);
-    bt->G_prefIII[k] = (float)(Gamma_R_prefactor * p->ReionNionPhotPerBaryIII / p->ReionNionPhotPerBary);
-    bt->fcoll_prefIII[k] = bt->fcoll_pref[k] / p->ReionEfficiency * p->ReionEfficiencyIII;
+    b3->J_aux[k] = bt->J_aux[k] * (float)(p->ReionNionPhotPerBaryIII / p->ReionNionPhotPerBary);
+    b3->G_pref[k] = (float)(Gamma_R_prefactor * p->ReionNionPhotPerBaryIII / p->ReionNionPhotPerBary);
+    b3->fcoll_pref[k] = bt->fcoll_pref[k] / p->ReionEfficiency * p->ReionEfficiencyIII;
   }
 }
 
@@ -1272,7 +794,7 @@ static int hii_sources(const rg_params* p, const rg_grids* g, bool plain, const 
   return ng;
 }
 
-static HiiState hii_state(const rg_params* p, const rg_grids* g, uint8_t* st8, double* partials) {
+static HiiState hii_state(const rg_params* p, const rg_grids* g, uint8_t* state) {
   const bool bh = p->Flag_BHFeedback != 0, mini = p->UseMiniHalos != 0;
   HiiState hs;
   hs.xH = g->xH;
@@ -1286,8 +808,7 @@ static HiiState hii_state(const rg_params* p, const rg_grids* g, uint8_t* st8, d
   hs.wsfrIII = mini ? g->weighted_sfrIII : nullptr;
   hs.Gamma12 = g->Gamma12;
   hs.r_bubble = g->r_bubble;
-  hs.st8 = st8;
-  hs.partials = partials;
+  hs.state = state;
   return hs;
 }
 
@@ -1338,6 +859,37 @@ static int hii_windows(rg_context* ctx, const rg_params* p, const std::vector<st
   return window_table(ctx, p->BoxSize, ctx->d_radii, nr, p->ReionFilterType, ctx->wtab, n2max, st, ctx->wcut);
 }
 
+// blocks of the closing pass: enough to fill the chip, at least four cells a thread
+static int hii_close_blocks(const rg_context* ctx, int n) {
+  return (int)std::max<size_t>(1, std::min((size_t)n * n * n / (4 * CLOSE_NT), (size_t)8 * ctx->num_sms));
+}
+
+// radii per batch of the fused mode: the caller's, or 16 where their windowed spectra take at most 6 GB
+// and 8 above (fewer launches and less state between batches: 0.34 -> 0.31 ms at 64^3, 4.74 -> 4.53 at
+// 192^3, no gain at 512^3)
+static int radius_batch(const rg_context* ctx, size_t nc, int ng, int nr) {
+  int kb = ctx->radius_batch > 0 ? ctx->radius_batch : nc * ng * 16 * sizeof(cf) <= ((size_t)6 << 30) ? 16 : 8;
+  return std::max(1, std::min({kb, KB_MAX, nr}));
+}
+
+// the work buffer of kb radii; *kb is halved down to 8 where the device has no room for the default 16
+static int ensure_work(rg_context* ctx, size_t nc, int ng, int* kb) {
+  int rc = ensure_device(ctx, &ctx->work, &ctx->work_elems, nc * ng * *kb);
+  if (rc == RG_ENOMEM && ctx->radius_batch == 0 && *kb > 8) {
+    cudaGetLastError();   // the failed allocation is dealt with
+    *kb = 8;
+    rc = ensure_device(ctx, &ctx->work, &ctx->work_elems, nc * ng * *kb);
+  }
+  return rc;
+}
+
+// radii whose window planes are formed at a time: whole batches, at most 256 MB where that is more
+// than one
+static int plane_radii(int n, int kb, int nr) {
+  const int fit = (int)((256u << 20) / (sizeof(float) * wplane_size(n))) / kb * kb;
+  return std::min(nr, std::max(kb, fit));
+}
+
 int hii_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const rg_grids* g, rg_hii_scalars* out,
                  const Staging* stg) {
   const Staging none;
@@ -1358,11 +910,9 @@ int hii_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, cons
   const size_t nc = (size_t)(N / 2 + 1) * N * N;
   auto sched = radius_schedule(p, redshift);
   const int nr = (int)sched.size();
-  int kb = plain ? 1 : (ctx->radius_batch > 0 ? ctx->radius_batch : 8);
-  if (kb > KB_MAX) kb = KB_MAX;
-  if (kb > nr) kb = nr;
+  int kb = plain ? 1 : radius_batch(ctx, nc, ng, nr);
   if ((rc = ensure_device(ctx, &ctx->spec, &ctx->spec_elems, nc * ng))) return rc;
-  if ((rc = ensure_device(ctx, &ctx->work, &ctx->work_elems, nc * ng * kb))) return rc;
+  if ((rc = ensure_work(ctx, nc, ng, &kb))) return rc;
   // one state byte per cell between radius batches (in words of four)
   if ((rc = ensure_device(ctx, &ctx->bits, &ctx->bits_elems, ((size_t)N * N * N + 3) / 4))) return rc;
   if ((rc = stage_wait(ctx, stg->inputs, st))) return rc;
@@ -1374,6 +924,8 @@ int hii_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, cons
   if ((rc = hii_windows(ctx, p, sched, st))) return rc;
   const int n2max = 3 * (N / 2) * (N / 2);
   const int* wcut = p->ReionFilterType == 1 ? ctx->wcut : nullptr;
+  const int npl = plane_radii(N, kb, nr);
+  if ((rc = ensure_device(ctx, &ctx->wplanes, &ctx->wplanes_elems, wcut ? 1 : npl * wplane_size(N)))) return rc;
 
   // r_bubble is only written on the recombination branch: zero it once
   RG_CUDA_TRY(ctx, cudaMemsetAsync(g->r_bubble, 0, sizeof(float) * (size_t)N * N * N, st));
@@ -1385,28 +937,34 @@ int hii_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, cons
     RG_CUDA_TRY(ctx, cudaMemcpyAsync(stg->host_r_bubble, g->r_bubble, sizeof(float) * (size_t)N * N * N,
                                      cudaMemcpyDeviceToHost, ctx->copy_stream));
   }
-  double* partials =
-      ensure_partials(ctx, std::max((size_t)N * N * HII_NSUM, (size_t)4 * ctx->num_sms * REC_NSUM));
+  const int cb = hii_close_blocks(ctx, N);
+  double* partials = ensure_partials(ctx, std::max((size_t)cb * HII_NSUM, (size_t)4 * ctx->num_sms * REC_NSUM));
   if (!partials) return set_error(ctx, RG_ENOMEM, "partials");
-  const HiiState hs = hii_state(p, g, reinterpret_cast<uint8_t*>(ctx->bits), partials);
+  const HiiState hs = hii_state(p, g, reinterpret_cast<uint8_t*>(ctx->bits));
 
   if ((rc = xy_ctrl_reset(ctx, (size_t)(N / 2 + 1) * kb, st))) return rc;
-  int nblocks = 0;
   for (int r0 = 0; r0 < nr; r0 += kb) {
     const int cnt = std::min(kb, nr - r0);
     const bool fin = (r0 + cnt == nr);
-    HiiBatch bt;
-    hii_batch_radii(p, redshift, sched, r0, cnt, ntest, &bt);
+    HiiZUnits us;
+    HiiBatchIII b3;
+    hii_batch_radii(p, redshift, sched, r0, cnt, ntest, &us.u[0].bt, &b3);
+    us.u[0].c = c;
+    us.u[0].s = hs;
     // the snapshot's last radius is unfiltered (find_HII_bubbles.c:313)
     const int unf = fin ? cnt - 1 : -1;
-    if ((rc = inverse_xy(ctx, N, ctx->spec, ng, ng, ctx->work, nc, cnt, ctx->wtab + (size_t)r0 * (n2max + 1),
-                         n2max + 1, unf, st, wcut ? wcut + r0 : nullptr)))
+    if (!wcut && r0 % npl == 0 &&
+        (rc = window_planes(ctx, N, ctx->wtab + (size_t)r0 * (n2max + 1), std::min(npl, nr - r0), ctx->wplanes, st)))
+      return rc;
+    if ((rc = inverse_xy(ctx, N, ctx->spec, ng, ng, ctx->work, nc, cnt, ctx->wplanes + (r0 % npl) * wplane_size(N),
+                         unf, st, wcut ? wcut + r0 : nullptr)))
       return rc;
     if (r0 == 0 && (rc = stage_wait(ctx, stg->state, st))) return rc;
-    if (fin && (rc = stage_wait(ctx, stg->closing, st))) return rc;
-    if ((rc = hii_z(ctx, N, ctx->work, nc, ntest, bt, c, hs, fin, st, &nblocks))) return rc;
+    if ((rc = hii_z(ctx, N, ctx->work, nc, ntest, 1, us, b3, st))) return rc;
   }
-  if ((rc = reduce_partials(ctx, partials, nblocks, HII_NSUM, ctx->d_sums, st))) return rc;
+  if ((rc = stage_wait(ctx, stg->closing, st))) return rc;
+  if ((rc = hii_close(ctx, N, c, hs, partials, cb, st))) return rc;
+  if ((rc = reduce_partials(ctx, partials, cb, HII_NSUM, ctx->d_sums, st))) return rc;
   if (rec) {
     RecTables tab;
     tab.knots = ctx->rec_knots;
@@ -1475,11 +1033,9 @@ int hii_batch(rg_context* ctx, int nu, const rg_params* p, const rg_snapshot* s,
   const int ng = nu * ngu;
   const size_t nc = (size_t)(N / 2 + 1) * N * N, n3 = (size_t)N * N * N;
   const int nr = (int)sched.size();
-  int kb = ctx->radius_batch > 0 ? ctx->radius_batch : 8;
-  if (kb > KB_MAX) kb = KB_MAX;
-  if (kb > nr) kb = nr;
+  int kb = radius_batch(ctx, nc, ng, nr);
   if ((rc = ensure_device(ctx, &ctx->spec, &ctx->spec_elems, nc * ng))) return rc;
-  if ((rc = ensure_device(ctx, &ctx->work, &ctx->work_elems, nc * ng * kb))) return rc;
+  if ((rc = ensure_work(ctx, nc, ng, &kb))) return rc;
   // one state byte per cell of every unit
   if ((rc = ensure_device(ctx, &ctx->bits, &ctx->bits_elems, (n3 * nu + 3) / 4))) return rc;
   if ((rc = ensure_device(ctx, &ctx->batch_sums, &ctx->batch_sums_elems, (size_t)32 * nu))) return rc;
@@ -1498,33 +1054,49 @@ int hii_batch(rg_context* ctx, int nu, const rg_params* p, const rg_snapshot* s,
   if ((rc = hii_windows(ctx, &p[0], sched, st))) return rc;
   const int n2max = 3 * (N / 2) * (N / 2);
   const int* wcut = p[0].ReionFilterType == 1 ? ctx->wcut : nullptr;
+  const int npl = plane_radii(N, kb, nr);
+  if ((rc = ensure_device(ctx, &ctx->wplanes, &ctx->wplanes_elems, wcut ? 1 : npl * wplane_size(N)))) return rc;
   for (int u = 0; u < nu; ++u)
     RG_CUDA_TRY(ctx, cudaMemsetAsync(g[u].r_bubble, 0, sizeof(float) * n3, st));
-  double* partials = ensure_partials(ctx, (size_t)N * N * HII_NSUM);
+  const int cb = hii_close_blocks(ctx, N);
+  double* partials = ensure_partials(ctx, (size_t)nu * cb * HII_NSUM);
   if (!partials) return set_error(ctx, RG_ENOMEM, "partials");
   std::vector<HiiState> hs(nu);
   for (int u = 0; u < nu; ++u)
-    hs[u] = hii_state(&p[u], &g[u], reinterpret_cast<uint8_t*>(ctx->bits) + n3 * u, partials);
+    hs[u] = hii_state(&p[u], &g[u], reinterpret_cast<uint8_t*>(ctx->bits) + n3 * u);
 
   if ((rc = xy_ctrl_reset(ctx, (size_t)(N / 2 + 1) * kb, st))) return rc;
+  const int zu = hii_z_units(N);
   for (int r0 = 0; r0 < nr; r0 += kb) {
     const int cnt = std::min(kb, nr - r0);
     const bool fin = (r0 + cnt == nr);
     const int unf = fin ? cnt - 1 : -1;
     // the windowed inverse x/y passes of every unit's grids in one launch; unit u's block of
     // the work buffer is [radius][its grids], as a single snapshot's
-    if ((rc = inverse_xy(ctx, N, ctx->spec, ng, ngu, ctx->work, nc, cnt, ctx->wtab + (size_t)r0 * (n2max + 1),
-                         n2max + 1, unf, st, wcut ? wcut + r0 : nullptr)))
+    if (!wcut && r0 % npl == 0 &&
+        (rc = window_planes(ctx, N, ctx->wtab + (size_t)r0 * (n2max + 1), std::min(npl, nr - r0), ctx->wplanes, st)))
       return rc;
-    for (int u = 0; u < nu; ++u) {
-      HiiBatch bt;
-      hii_batch_radii(&p[u], s[u].ZZ[s[u].snapshot], sched, r0, cnt, ntest, &bt);
-      int nblocks = 0;
-      if ((rc = hii_z(ctx, N, ctx->work + (size_t)u * cnt * ngu * nc, nc, ntest, bt, cs[u], hs[u], fin, st, &nblocks)))
+    if ((rc = inverse_xy(ctx, N, ctx->spec, ng, ngu, ctx->work, nc, cnt, ctx->wplanes + (r0 % npl) * wplane_size(N),
+                         unf, st, wcut ? wcut + r0 : nullptr)))
+      return rc;
+    // the z passes, zu snapshots a launch (a 96^3 box alone fills a fifth of the chip)
+    for (int u0 = 0; u0 < nu; u0 += zu) {
+      const int cu = std::min(zu, nu - u0);
+      HiiZUnits us;
+      HiiBatchIII b3;
+      for (int k = 0; k < cu; ++k) {
+        const int u = u0 + k;
+        hii_batch_radii(&p[u], s[u].ZZ[s[u].snapshot], sched, r0, cnt, ntest, &us.u[k].bt, &b3);
+        us.u[k].c = cs[u];
+        us.u[k].s = hs[u];
+      }
+      if ((rc = hii_z(ctx, N, ctx->work + (size_t)u0 * cnt * ngu * nc, nc, ntest, cu, us, b3, st)))
         return rc;
-      if (fin && (rc = reduce_partials(ctx, partials, nblocks, HII_NSUM, ctx->batch_sums + 32 * u, st))) return rc;
     }
   }
+  for (int u = 0; u < nu; ++u)
+    if ((rc = hii_close(ctx, N, cs[u], hs[u], partials + (size_t)u * cb * HII_NSUM, cb, st))) return rc;
+  if ((rc = reduce_partials(ctx, partials, cb, HII_NSUM, ctx->batch_sums, st, nu, (size_t)cb * HII_NSUM, 32))) return rc;
   RG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_batch_sums, ctx->batch_sums, sizeof(double) * 32 * nu,
                                    cudaMemcpyDeviceToHost, st));
   RG_CUDA_TRY(ctx, cudaStreamSynchronize(st));
@@ -1534,8 +1106,8 @@ int hii_batch(rg_context* ctx, int nu, const rg_params* p, const rg_snapshot* s,
   return RG_OK;
 }
 
-static int debug_inverse(rg_context* ctx, int n, const float* wrow, float* d_out, cudaStream_t st) {
-  RG_DISPATCH_N(n, launch_debug_inverse<NN>(ctx, ctx->spec, ctx->work, wrow, d_out, st));
+static int debug_inverse(rg_context* ctx, int n, const float* wplane, float* d_out, cudaStream_t st) {
+  RG_DISPATCH_N(n, launch_debug_inverse<NN>(ctx, ctx->spec, ctx->work, wplane, d_out, st));
 }
 
 int spectrum_to_padded(rg_context* ctx, float* d_out, cudaStream_t st) {
@@ -1554,16 +1126,18 @@ int debug_roundtrip(rg_context* ctx, const rg_params* p, const float* d_in, floa
   if ((rc = ensure_device(ctx, &ctx->work, &ctx->work_elems, nc))) return rc;
   const float* srcs[1] = {d_in};
   if ((rc = fft_forward(ctx, N, srcs, 1, ctx->spec, nc, 1.0 / std::pow((double)N, 3), st))) return rc;
-  const float* wrow = nullptr;
+  const float* wplane = nullptr;
   if (ftype >= 0) {
     const int n2max = 3 * (N / 2) * (N / 2);
     if ((rc = ensure_device(ctx, &ctx->d_radii, &ctx->d_radii_elems, 1))) return rc;
     RG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->d_radii, &R, sizeof(double), cudaMemcpyHostToDevice, st));
     if ((rc = ensure_device(ctx, &ctx->wtab, &ctx->wtab_elems, (size_t)(n2max + 1)))) return rc;
     if ((rc = window_table(ctx, p->BoxSize, ctx->d_radii, 1, ftype, ctx->wtab, n2max, st))) return rc;
-    wrow = ctx->wtab;
+    if ((rc = ensure_device(ctx, &ctx->wplanes, &ctx->wplanes_elems, wplane_size(N)))) return rc;
+    if ((rc = window_planes(ctx, N, ctx->wtab, 1, ctx->wplanes, st))) return rc;
+    wplane = ctx->wplanes;
   }
-  if ((rc = debug_inverse(ctx, N, wrow, d_out, st))) return rc;
+  if ((rc = debug_inverse(ctx, N, wplane, d_out, st))) return rc;
   return xy_ctrl_check(ctx, st);
 }
 

@@ -1,0 +1,6 @@
+// k_hii_zr at 384 (one translation unit per size: they compile in parallel).
+#include "rg_hii_z.cuh"
+
+namespace rg {
+template int launch_hii_zr<384>(rg_context*, const cf*, int, const HiiZUnits&, cudaStream_t);
+}  // namespace rg

@@ -97,6 +97,8 @@ int ensure_device(rg_context* ctx, T** ptr, size_t* have, size_t need) {
 struct HiiConst {
   float redshift, TK, cT_ad;
   int uvb, spin, bh, rec, mini;
+  // powers of the ionised gas temperature: T_re^1.7, (1e4 (1 + z) / 4)^1.7, ((1 + z) / 7.1)^2.5
+  double t_17, z_17, z_25;
 };
 
 // Recombination tables on the device (splined_recombination, recombinations.c:35-84).
@@ -114,6 +116,13 @@ constexpr int KB_MAX = 16;    // radii per batch
 // Forward r2c of ng padded real grids into spectra spec_base + g * stride, scaled.
 int fft_forward(rg_context* ctx, int n, const float* const* d_real, int ng, cf* spec_base, size_t stride,
                 double scale, cudaStream_t st);
+// Windowed inverse x and y passes of nr radii of the ng spectra at spec (ngu per snapshot) into
+// work; radius r's window in wplanes (window_planes; none for r == unfiltered), or the sharp-k steps wcut.
+int inverse_xy(rg_context* ctx, int n, const cf* spec, int ng, int ngu, cf* work, size_t stride, int nr,
+               const float* wplanes, int unfiltered, cudaStream_t st, const int* wcut);
+// the windows of nr radii on the octant of modes (W[kz][|nx|][|ny|], wplane_size(n) floats each) from
+// the rows W[n2] of window_table
+int window_planes(rg_context* ctx, int n, const float* wrows, int nr, float* planes, cudaStream_t st);
 // W[r][n2] for the radii in d_radii (filter() closed forms, double precision); for the sharp-k
 // filter also d_wcut[r] (when given), the last n2 of the step, so W[r][n2] == (n2 <= d_wcut[r])
 int window_table(rg_context* ctx, double box, const double* d_radii, int nr, int ftype, float* d_wtab, int n2max,
@@ -141,7 +150,7 @@ int hii_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, cons
                  const Staging* stg = nullptr);
 // find_HII_bubbles for nu snapshots of this size with the same radii, device grids, fused mode:
 // the forward transforms and every radius batch's x/y passes of all of them in shared launches,
-// the z passes per snapshot, one host synchronisation.
+// the z passes of up to 8 snapshots a launch, one host synchronisation.
 int hii_batch(rg_context* ctx, int nu, const rg_params* p, const rg_snapshot* s, const rg_grids* g,
               rg_hii_scalars* out);
 // The spin-temperature step on device grids (rg_ts.cu).  With src_host, the sfr /
@@ -155,7 +164,10 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
 int spectrum_to_padded(rg_context* ctx, float* d_out, cudaStream_t st);
 // Forward + (windowed) inverse of one padded grid, for tests.
 int debug_roundtrip(rg_context* ctx, const rg_params* p, const float* d_in, float* d_out, double R, int ftype);
-int reduce_partials(rg_context* ctx, const double* partials, int nblocks, int nsum, double* d_out, cudaStream_t st);
+// the nsum sums over nblocks partials (deterministic); of `sets` sets, set u at partials + u set_pitch
+// into d_out + u out_pitch
+int reduce_partials(rg_context* ctx, const double* partials, int nblocks, int nsum, double* d_out, cudaStream_t st,
+                    int sets = 1, size_t set_pitch = 0, int out_pitch = 0);
 double* ensure_partials(rg_context* ctx, size_t n);
 int ensure_tables(rg_context* ctx, const rg_params* p);
 int validate_common(rg_context* ctx, const rg_params* p);
@@ -196,6 +208,8 @@ struct rg_context {
   size_t bits_elems = 0;
   float* wtab = nullptr;         // window table [nR][n2max+1]
   size_t wtab_elems = 0;
+  float* wplanes = nullptr;      // the windows of some radii on the octant of modes
+  size_t wplanes_elems = 0;
   int* wcut = nullptr;           // sharp-k window: last n2 of each row's step
   size_t wcut_elems = 0;
   float* ps_pad = nullptr;       // power spectrum: padded real input of the transform

@@ -125,6 +125,31 @@ __host__ __device__ constexpr int line_buf_r0() {
   return N * B + (B < 16 ? B * (N / R0 + 1) : 0);
 }
 
+// A radius's window on the modes of one octant, W[kz][|nx|][|ny|] with rows of wplane_pitch(N) values:
+// what the windowed x passes read, in runs over |ny|
+__host__ __device__ constexpr int wplane_pitch(int n) { return round_up(n / 2 + 1, 8); }
+__host__ __device__ constexpr size_t wplane_size(int n) {
+  return (size_t)(n / 2 + 1) * (n / 2 + 1) * wplane_pitch(n);
+}
+
+// call with NN = n for the sizes there are plans for
+#define RG_DISPATCH_N(n, call)                                                   \
+  switch (n) {                                                                   \
+    case 8: { constexpr int NN = 8; return call; }                               \
+    case 16: { constexpr int NN = 16; return call; }                             \
+    case 24: { constexpr int NN = 24; return call; }                             \
+    case 32: { constexpr int NN = 32; return call; }                             \
+    case 48: { constexpr int NN = 48; return call; }                             \
+    case 64: { constexpr int NN = 64; return call; }                             \
+    case 96: { constexpr int NN = 96; return call; }                             \
+    case 128: { constexpr int NN = 128; return call; }                           \
+    case 192: { constexpr int NN = 192; return call; }                           \
+    case 256: { constexpr int NN = 256; return call; }                           \
+    case 384: { constexpr int NN = 384; return call; }                           \
+    case 512: { constexpr int NN = 512; return call; }                           \
+    default: return set_error(ctx, RG_EUNSUPPORTED, "ReionGridDim not in {8,16,24,32,48,64,96,128,192,256,384,512}"); \
+  }
+
 // ---------------------------------------------------------------------------
 
 // the forward z pass's launch shape: QF row pairs per block, one line of T threads each (the

@@ -47,6 +47,7 @@ struct XYSched {
   uint32_t* done;    // [J] finished X items per job (zero at launch)
   uint32_t* err;     // set to 1 when a wait runs out
   int max_polls;     // polls of a Y item's wait before it gives up
+  int stream;        // Y stores evict first
   int signal;        // X items signal their job (0 only in the forced-timeout test)
 };
 
@@ -86,13 +87,15 @@ __device__ __forceinline__ void xy_wait(const XYSched& s, int job) {
 // The fused pass's plans (PlanW): at 512, 8 x 16 x 4 over 32 threads a line measured faster than
 // 8 x 8 x 8 over 64 (77.2 against 81.3 ms for the 61 radii of a 512^3 snapshot; 16 x 16 x 2 took
 // 78.5 ms, and 16 columns an item instead of 8 took 85-87 ms), and its Y lines are warp-local.
-template <int N>
+template <int N, class Plan_>
 struct XYF {
-  using PL = PlanW<N>;
+  using PL = Plan_;
   static constexpr int T = PL::T;
-  static constexpr int V = N / T;
-  static constexpr int B = Cfg<N>::BX;   // columns per X item, lines per Y item
-  static constexpr int MINB = N != 512 ? x_pass_minb<N>() : 2;
+  static constexpr int V = stage_rounds<PL, 0>() * PL::R[0];   // inputs of a thread
+  static constexpr int B = pow2_div(N, cmax(256 / T, 8));      // columns per X item, lines per Y item
+  // three blocks an SM at 256 (2.95 against 3.17 ms for the 42 radii of a 256^3 snapshot), two where
+  // a block's registers or the planes in flight do not leave room for the third (512^3: 65.6, 67.9)
+  static constexpr int MINB = T * B >= 512 ? 1 : N == 256 ? 3 : RG_MINB(T * B);
   static constexpr int NTH = T * B;
   static constexpr int M = N / B;
   static constexpr int XROWS = N <= 256 ? N : N / 2;   // x rows per tensor box (box dimensions <= 256)
@@ -112,25 +115,24 @@ __device__ __forceinline__ cf ldcg_cf(const cf* p) {
 
 // release the finished X item: the block barrier before it orders the block's stores
 __device__ __forceinline__ void xy_signal(uint32_t* p) {
-  __threadfence();
-  atomicAdd(p, 1u);
+  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory");
 }
 
 // Op (by value) describes the batch:
 //   int grids() const                         grids per job
 //   bool filtered(int r) const                radius r is windowed
-//   const float* wrow(int r) const            its window row W[n2]
-//   int cutoff(int r) const                   >= -1: the row is the step W = (n2 <= cutoff), read
-//                                             without gathers (sharp-k); < -1: read the row
+//   const float* wplane(int r) const          its window on the octant (wplane_pitch)
+//   int cutoff(int r) const                   >= -1: the window is the step W = (n2 <= cutoff)
+//                                             (sharp-k); < -1: read the planes
 //   cf* out(int r, int g) const               output grid (plane kz at kz N^2)
 // The X input of grid g is W(k) * spectrum_g(k); the spectra are the tensor `smap` (floats, y
 // innermost, then x, then kz of grid g at g (N/2 + 1) + kz).
-template <int N, class Op>
-__global__ void __launch_bounds__(XYF<N>::NTH, XYF<N>::MINB)
+template <int N, class PL_, class Op>
+__global__ void __launch_bounds__(XYF<N, PL_>::NTH, XYF<N, PL_>::MINB)
     k_xy_fused(XYSched sch, Op op, const __grid_constant__ CUtensorMap smap, const cf* __restrict__ g_tw) {
-  using F = XYF<N>;
-  using PL = typename F::PL;
-  constexpr int T = F::T, B = F::B, V = F::V, TB = F::TB, NZ = N / 2 + 1;
+  using F = XYF<N, PL_>;
+  using PL = PL_;
+  constexpr int T = F::T, B = F::B, V = F::V, TB = F::TB, NZ = N / 2 + 1, R0 = PL::R[0];
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
   cf* bufs = reinterpret_cast<cf*>(sm);
@@ -172,9 +174,16 @@ __global__ void __launch_bounds__(XYF<N>::NTH, XYF<N>::MINB)
   int item = s_item[0];
   uint32_t xu = 0;          // X units (item, grid) this block has started: unit u uses buffer u & 1
   bool waited = true;
+  int owed = -1;   // job of the X item this block has finished and not signalled yet (thread 0)
   while (item < sch.total) {
     int nxt = 0;
-    if (threadIdx.x == 0) nxt = (int)atomicAdd(sch.ctr, 1u);   // the next item, fetched early
+    if (threadIdx.x == 0) {
+      // the signal waits for the item's stores to reach L2; here, at the start of the next item (before
+      // that can wait on anything), the wait overlaps the other warps' loads
+      if (owed >= 0) xy_signal(sch.done + owed);
+      owed = -1;
+      nxt = (int)atomicAdd(sch.ctr, 1u);   // the next item, fetched early
+    }
     const bool pref = s_pref[it & 1] != 0;
     const int seg = item / sch.M, k = item - seg * sch.M;
     bool is_y;
@@ -191,15 +200,15 @@ __global__ void __launch_bounds__(XYF<N>::NTH, XYF<N>::MINB)
 #pragma unroll
       for (int sl = 0; sl < V; ++sl) wv[sl] = 1.f;
       if (op.filtered(r)) {
-        const float* wr = op.wrow(r);
         const int cut = op.cutoff(r);
-        const int ny = y > N / 2 ? y - N : y;
+        const int ny = y > N / 2 ? N - y : y;
+        constexpr int WP = wplane_pitch(N);
+        const float* wp = op.wplane(r) + (size_t)kz * (N / 2 + 1) * WP + ny;
 #pragma unroll
         for (int sl = 0; sl < V; ++sl) {
           const int p = stage0_pos<PL>(t, sl);
-          const int nx = p > N / 2 ? p - N : p;
-          const int n2 = nx * nx + ny * ny + kz * kz;
-          wv[sl] = cut >= -1 ? (n2 <= cut ? 1.f : 0.f) : __ldg(wr + n2);
+          const int nx = p > N / 2 ? N - p : p;
+          if ((N / R0) % T == 0 || t + (sl / R0) * T < N / R0) wv[sl] = cut >= -1 ? (nx * nx + ny * ny + kz * kz <= cut ? 1.f : 0.f) : __ldg(wp + nx * WP);
         }
       }
       for (int g = 0; g < ng; ++g, ++xu) {
@@ -228,7 +237,7 @@ __global__ void __launch_bounds__(XYF<N>::NTH, XYF<N>::MINB)
         fence_proxy_async_smem();
         __syncthreads();   // every store of the unit is issued; its buffer may be refilled
       }
-      if (threadIdx.x == 0 && sch.signal) xy_signal(sch.done + job);
+      if (sch.signal) owed = job;
     } else {
       if (threadIdx.x == 0) xy_wait(sch, job);
       __syncthreads();
@@ -239,7 +248,10 @@ __global__ void __launch_bounds__(XYF<N>::NTH, XYF<N>::MINB)
         cf* line = op.out(r, g) + row;
         line_fft_p<PL, true, (T <= 32)>(
             t, bufs, s_tw, [&](int p, int) { return ldcg_cf(line + p); }, [&](int p) { return pos_addr<N>(b, p); },
-            [&](int p, cf v, int) { line[p] = v; });
+            [&](int p, cf v, int) {
+              if (sch.stream) __stcs(reinterpret_cast<float2*>(line + p), make_float2(v.x, v.y));
+              else line[p] = v;
+            });
       }
       fence_proxy_async_smem();   // the exchange buffer is a tile buffer of later X items
     }
@@ -251,15 +263,16 @@ __global__ void __launch_bounds__(XYF<N>::NTH, XYF<N>::MINB)
     ++it;
     item = s_item[it & 1];
   }
+  if (threadIdx.x == 0 && owed >= 0) xy_signal(sch.done + owed);
   if (!waited && threadIdx.x % 32 == 0) atomicExch(sch.err, 1u);
 }
 
 // Launch the fused pass of one batch of nr radii (or shells); the control words must have been
 // sized by xy_ctrl_reset for at least (N/2 + 1) nr jobs.
-template <int N, class Op>
+template <int N, class PL, class Op>
 int launch_xy_fused(rg_context* ctx, const Op& op, const cf* spec, int nspec, int nr, const char* name,
                     double alg_bytes, cudaStream_t st) {
-  using F = XYF<N>;
+  using F = XYF<N, PL>;
   const cf* tw;
   int rc = twiddles_for(ctx, N, &tw);
   if (rc) return rc;
@@ -272,7 +285,7 @@ int launch_xy_fused(rg_context* ctx, const Op& op, const cf* spec, int nspec, in
   if (mrc != 0) return set_error(ctx, RG_ECUDA, "cuTensorMapEncodeTiled failed (" + std::to_string(mrc) + ")");
   const int J = Cfg<N>::NZ * nr;
   if (nr < 1 || (size_t)J + 2 > ctx->xy_ctrl_elems) return set_error(ctx, RG_EINVAL, "fused x/y pass: batch too large");
-  auto kern = k_xy_fused<N, Op>;
+  auto kern = k_xy_fused<N, PL, Op>;
   RG_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F::smem()));
   int per_sm = 0;
   RG_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, F::NTH, F::smem()));
@@ -281,9 +294,17 @@ int launch_xy_fused(rg_context* ctx, const Op& op, const cf* spec, int nspec, in
   s.nr = nr;
   s.M = F::M;
   s.J = J;
-  // Y(j) is handed out (2L + 1) M items after X(j) starts; with `grid` blocks in flight that is
-  // about when X(j) completes for L = grid / (2M), one more for slack
-  s.L = std::min(J, (grid + 2 * F::M - 1) / (2 * F::M) + 1);
+  // Y(j) is handed out (2L + 1) M items after X(j) starts.  With `grid` blocks in flight that is about
+  // when X(j) completes for L = grid / (2M); twice that keeps the Y items from waiting, as long as
+  // the 2L planes written in between (64 MB of them: a plane is written by X, read and written by Y)
+  // stay in L2.  Measured (ms of a snapshot's passes) at L = grid / (2M), 1.5, 2 and 3 times that:
+  // 192^3 3.50, 2.83, 2.91, 3.29; 256^3 3.47, 3.04, 2.95, 3.03; 512^3 65.6, 65.8, 66.7, 70.4.
+  const int base = (grid + 2 * F::M - 1) / (2 * F::M);
+  const size_t job_bytes = sizeof(cf) * (size_t)N * N * op.ng;
+  s.L = std::min(J, std::max(base + 1, std::min(2 * base + 1, (int)((64u << 20) / (2 * job_bytes)))));
+  // a batch that does not stay in L2 until its z pass leaves by evict-first stores: its finished planes
+  // go before the ones that Y items still read (192^3: 3.31 -> 2.83 ms)
+  s.stream = (size_t)J * job_bytes > (48u << 20);
   s.total = 2 * J * F::M;
   s.err = ctx->xy_ctrl;
   s.max_polls = ctx->xy_poll_limit;
