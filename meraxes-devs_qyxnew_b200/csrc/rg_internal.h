@@ -220,7 +220,7 @@ struct rg_context {
   size_t vel_work_elems = 0;
   float* vel_stage = nullptr;    // rg_delta_T_host: device copy of the caller's velocity grid
   size_t vel_stage_elems = 0;
-  int* ngp_bad = nullptr;        // rg_deposit_ngp: count of galaxies below the box
+  int* ngp_bad = nullptr;        // rg_deposit_ngp: galaxies below the box; properties with values below 0
   size_t ngp_bad_elems = 0;
   float2* ts_agn = nullptr;       // ComputeTs: per-cell AGN heating sums of the two AGN units
   size_t ts_agn_elems = 0;
