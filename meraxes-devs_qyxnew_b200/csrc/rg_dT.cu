@@ -3,6 +3,7 @@
 // over the cells, with the FP64 volume average reduced in the same kernel.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 
 #include "rg_internal.h"
@@ -15,40 +16,63 @@ constexpr int DT_NT = 256;
 constexpr int N_RSD_STEPS = 50;      // reionization.h:34
 constexpr float MAX_DVDR = 0.2f;     // reionization.h:45
 
+// FP64 block sum in a fixed order -> partials[blockIdx.x]
+__device__ __forceinline__ void dt_block_sum(double acc, double* __restrict__ partials) {
+  __shared__ double sh[DT_NT / 32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
+  if (threadIdx.x % 32 == 0) sh[threadIdx.x / 32] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double v = 0.0;
+#pragma unroll
+    for (int w = 0; w < DT_NT / 32; ++w) v += sh[w];
+    partials[blockIdx.x] = v;
+  }
+}
+
+// f(cell, padded cell) over the box, DT_U cells of a thread in a row of the loop so that their loads are
+// in flight together (one at a time a pass over 256^3 cells reached 2.5 of 6.5 TB/s)
+constexpr int DT_U = 4;
+__device__ __forceinline__ size_t dt_padded(size_t ir, int n) {
+  return ir + ((unsigned)ir / (unsigned)n) * 2;   // rows of n + 2 values (n is even, at most 512)
+}
+
 __global__ void __launch_bounds__(DT_NT) k_delta_T(const float* __restrict__ xH, const float* __restrict__ deltax,
                                                    const float* __restrict__ TS, float* __restrict__ dT, int n,
                                                    float const_factor, double t_rad, int spin, int pec_vel_gt1,
                                                    float redshift, double* __restrict__ partials) {
-  const int padw = 2 * (n / 2 + 1);
-  const size_t rows = (size_t)n * n;
+  const size_t n3 = (size_t)n * n * n, step = (size_t)gridDim.x * DT_NT;
+  const double opz = 1. + (double)redshift;
   double acc = 0.0;
-  for (size_t row = blockIdx.x; row < rows; row += gridDim.x) {
-    for (int z = threadIdx.x; z < n; z += DT_NT) {
-      const size_t ir = row * n + z;
-      const double pixel_deltax = (double)deltax[row * padw + z];
-      const double pixel_x_HI = (double)xH[ir];
-      float v = (float)((double)const_factor * pixel_x_HI * (1.0 + pixel_deltax));
+  for (size_t i0 = (size_t)blockIdx.x * DT_NT + threadIdx.x; i0 < n3; i0 += DT_U * step) {
+    float x[DT_U], d[DT_U], t[DT_U];
+#pragma unroll
+    for (int k = 0; k < DT_U; ++k) {
+      const size_t i = i0 + k * step;
+      if (i >= n3) break;
+      x[k] = xH[i];
+      d[k] = deltax[dt_padded(i, n)];
+      t[k] = spin ? TS[i] : 1.f;
+    }
+#pragma unroll
+    for (int k = 0; k < DT_U; ++k) {
+      const size_t i = i0 + k * step;
+      if (i >= n3) break;
+      float v = (float)((double)const_factor * (double)x[k] * (1.0 + (double)d[k]));
       if (spin) {
         if (pec_vel_gt1) {
-          v = (float)((double)v * ((1. + (double)redshift) / (1000. * (double)TS[ir])));
+          v = (float)((double)v * (opz / (1000. * (double)t[k])));
         } else {
-          const double fac = 1 - t_rad / (double)TS[ir];
+          const double fac = 1 - t_rad / (double)t[k];
           v = (float)((double)v * fac);
         }
       }
-      dT[ir] = v;
+      dT[i] = v;
       acc += (double)v;
     }
   }
-  // block reduction in a fixed order
-  __shared__ double sh[DT_NT];
-  sh[threadIdx.x] = acc;
-  __syncthreads();
-  for (int w = DT_NT / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) partials[blockIdx.x] = sh[0];
+  dt_block_sum(acc, partials);
 }
 
 int delta_T_launch(rg_context* ctx, int n, const float* xH, const float* deltax, const float* TS, float* dT,
@@ -68,21 +92,29 @@ int delta_T_launch(rg_context* ctx, int n, const float* xH, const float* deltax,
 // optical-depth form with the uncapped gradient, 3 adds the line-of-sight re-binning of 50
 // sub-cells per cell (Greig & Mesinger 2018).  Every float/double step is the reference's.
 
-// velocity in the tree code's units -> comoving velocity (BrightnessTemperature.c:173-196);
-// the padding of each row is not touched (the r2c transform ignores it)
+// velocity in the tree code's units -> comoving velocity (BrightnessTemperature.c:173-196); the
+// padding of each row is not touched (the r2c transform ignores it).  f0 is the factor of the tree
+// code's units, f1 that of cm in Mpc, and the division by 1 / (1 + z) a product with 1 + z.
 __global__ void __launch_bounds__(DT_NT) k_vel_convert(const float* __restrict__ vel, float* __restrict__ vc, int n,
-                                                       int trees, float redshift) {
-  const int padw = 2 * (n / 2 + 1);
-  const size_t rows = (size_t)n * n;
-  for (size_t row = blockIdx.x; row < rows; row += gridDim.x) {
-    for (int z = threadIdx.x; z < n; z += DT_NT) {
-      const size_t ip = row * padw + z;
-      float v = vel[ip];
-      if (trees == 1) v = (float)(sqrt(1. / (1. + (double)redshift)) * (double)v / 1000.);
-      else if (trees == 0 || trees == 2) v = (float)((1. + (double)redshift) * (double)v);
-      v = (float)((double)v * (1000. * 100. / MPC));
-      v = (float)((double)v / (1. / (1. + (double)redshift)));
-      vc[ip] = v;
+                                                       int trees, double f0, double f1, double opz) {
+  const size_t n3 = (size_t)n * n * n, step = (size_t)gridDim.x * DT_NT;
+  for (size_t i0 = (size_t)blockIdx.x * DT_NT + threadIdx.x; i0 < n3; i0 += DT_U * step) {
+    float in[DT_U];
+#pragma unroll
+    for (int k = 0; k < DT_U; ++k) {
+      const size_t i = i0 + k * step;
+      if (i >= n3) break;
+      in[k] = vel[dt_padded(i, n)];
+    }
+#pragma unroll
+    for (int k = 0; k < DT_U; ++k) {
+      const size_t i = i0 + k * step;
+      if (i >= n3) break;
+      float v = in[k];
+      if (trees == 1) v = (float)(f0 * (double)v / 1000.);
+      else v = (float)(f0 * (double)v);
+      v = (float)((double)v * f1);
+      vc[dt_padded(i, n)] = (float)((double)v * opz);
     }
   }
 }
@@ -103,125 +135,173 @@ __global__ void __launch_bounds__(DT_NT) k_vel_grad_spec(cf* __restrict__ spec, 
   }
 }
 
-// the gradient correction of delta_T (BrightnessTemperature.c:215-305, spin temperature on)
+// the gradient correction of delta_T (BrightnessTemperature.c:215-305, spin temperature on), with the
+// FP64 sum of the result
 __global__ void __launch_bounds__(DT_NT) k_vel_correct(float* __restrict__ dT, const float* __restrict__ grad,
                                                        const float* __restrict__ TS, int n, int flag, float H_z,
-                                                       double t_rad, float redshift) {
-  const int padw = 2 * (n / 2 + 1);
-  const size_t rows = (size_t)n * n;
+                                                       double t_rad, float redshift, double* __restrict__ partials) {
+  const size_t n3 = (size_t)n * n * n, step = (size_t)gridDim.x * DT_NT;
   const double max_v_deriv = fabs((double)(MAX_DVDR * H_z));
-  for (size_t row = blockIdx.x; row < rows; row += gridDim.x) {
-    for (int z = threadIdx.x; z < n; z += DT_NT) {
-      const size_t ir = row * n + z;
-      const double g = (double)grad[row * padw + z];
-      float d = dT[ir];
+  const double inv_H = 1.0 / (double)H_z, f = 1000. / (1. + (double)redshift);
+  double acc = 0.0;
+  for (size_t i0 = (size_t)blockIdx.x * DT_NT + threadIdx.x; i0 < n3; i0 += DT_U * step) {
+    float d[DT_U], gr[DT_U], t[DT_U];
+#pragma unroll
+    for (int k = 0; k < DT_U; ++k) {
+      const size_t i = i0 + k * step;
+      if (i >= n3) break;
+      d[k] = dT[i];
+      gr[k] = grad[dt_padded(i, n)];
+      t[k] = flag == 1 ? 0.f : TS[i];
+    }
+#pragma unroll
+    for (int k = 0; k < DT_U; ++k) {
+      const size_t i = i0 + k * step;
+      if (i >= n3) break;
+      const double g = (double)gr[k];
+      float v;
       if (flag == 1) {
         double dvdx = g;
         if (fabs(dvdx) > max_v_deriv) dvdx = dvdx < 0 ? -max_v_deriv : max_v_deriv;
-        d = (float)((double)d / (dvdx / (double)H_z + 1.0));
+        v = (float)((double)d[k] / (dvdx * inv_H + 1.0));
       } else {
-        const double gc = fabs(g / (double)H_z + 1.0);
-        const double ts = (double)TS[ir];
-        if (gc < FRACT_FLOAT_ERR)
-          d = (float)(1000. * (ts - t_rad) / (1. + (double)redshift));
-        else
-          d = (float)((1. - exp(-(double)d / gc)) * 1000. * (ts - t_rad) / (1. + (double)redshift));
+        const double gc = fabs(g * inv_H + 1.0);
+        const double ts = ((double)t[k] - t_rad) * f;
+        v = gc < FRACT_FLOAT_ERR ? (float)ts : (float)((1. - exp(-(double)d[k] / gc)) * ts);
       }
-      dT[ir] = d;
+      dT[i] = v;
+      acc += (double)v;
     }
   }
+  dt_block_sum(acc, partials);
 }
 
 struct RsdConst {
   float x_pos[N_RSD_STEPS];          // sub-cell centres in cell widths
   float x_pos_offset[N_RSD_STEPS];   // ... in Mpc
-  double cell;                       // BoxSize / (float)ReionGridDim, Mpc
-  double sub_w;                      // sub-cell width, Mpc
+  double inv_cell;                   // 1 / cell width, Mpc^-1
+  double inv_w_sub, half;            // sub-cell width (inverse) and half width in cell widths
   float H_z;
+  int n_low;                         // sub-cells up to the cell's centre
 };
 
-// line-of-sight re-binning (BrightnessTemperature.c:307-509): one block per (x, y) line; every
-// contributing cell moves its 50 sub-cells by the interpolated displacement v / H(z) and adds
-// each (or its two parts) to the cells it lands in, periodically along z.  The line's sums live
-// in shared memory; the adds of different cells meet there in any order.
+// line-of-sight re-binning (BrightnessTemperature.c:307-509): every contributing cell moves its 50
+// sub-cells by the interpolated displacement v / H(z) and adds each (or its two parts) to the cells it
+// lands in, periodically along z.  A block takes whole (x, y) lines, whose sums live in shared memory;
+// the adds of different cells meet there in any order.
+//
+// The displacement is linear between cell centres, so on either side of a cell's centre the sub-cells
+// (length 1 in units of their width) start at L_s = U + s g, g = 1 + the change of the displacement
+// over a cell.  What of them lies left of a boundary B is
+//   F(B) = sum_s clamp(B - L_s, 0, 1) = n1 + sum over n1 <= s < n2 of (B - U - s g),
+// n1 sub-cells wholly left of B and n2 that reach it: a closed form in FP64, and a cell gets F(right
+// edge) - F(left edge).  Two or three cells a side instead of 50 sub-cells with one or two shared-memory
+// adds each (compare-and-swap loops, in divergent branches): 3.17 -> 0.51 ms at 256^3.  Where the
+// sub-cells cross or spread (g outside [1/50, 8]) or are far off, infinite or not numbers, they are
+// moved one by one as in the reference.
 __global__ void __launch_bounds__(DT_NT) k_rsd(float* __restrict__ dT, const float* __restrict__ xH,
-                                               const float* __restrict__ vc, int n, RsdConst c) {
+                                               const float* __restrict__ vc, int n, int lines, const RsdConst c,
+                                               double* __restrict__ partials) {
   extern __shared__ float acc[];
-  const int padw = 2 * (n / 2 + 1);
-  const size_t row = blockIdx.x;
-  for (int k = threadIdx.x; k < n; k += DT_NT) acc[k] = 0.f;
-  __syncthreads();
-  const float* v = vc + row * padw;
+  constexpr double NS = N_RSD_STEPS;
+  const int padw = n + 2;
+  const size_t nrows = (size_t)n * n;
   auto wrap = [n](int k) { return ((k % n) + n) % n; };   // the reference's periodic index
-  const double w_sub = c.sub_w / c.cell;
-  const double half = (c.sub_w / 2.) / c.cell;
-  // the reference divides by the cell and sub-cell widths in every sub-cell; multiplying by the
-  // reciprocals instead moves positions and shares by at most an ulp of double
-  const double inv_cell = 1.0 / c.cell, inv_w_sub = 1.0 / w_sub;
-  for (int kk = threadIdx.x; kk < n; kk += DT_NT) {
-    const float d = dT[row * n + kk];
-    if (!(fabs((double)d) >= FRACT_FLOAT_ERR && (double)xH[row * n + kk] >= FRACT_FLOAT_ERR)) continue;
-    const double d1_low = (double)(v[kk == 0 ? n - 1 : kk - 1] / c.H_z);
-    const double d2_low = (double)(v[kk] / c.H_z);
-    const double d1_high = (double)(v[kk] / c.H_z);
-    const double d2_high = (double)(v[kk == n - 1 ? 0 : kk + 1] / c.H_z);
-    const float val = d / (float)N_RSD_STEPS;
-    const double dd = (double)d / (double)N_RSD_STEPS;
-    auto put = [&](int k, double frac) { atomicAdd(acc + wrap(k), (float)(frac * dd)); };
-    for (int s = 0; s < N_RSD_STEPS; ++s) {
-      const double xp = (double)c.x_pos[s];
-      const double disp = xp <= 0.5 ? d1_low + ((xp + 0.5) - 0.) * (d2_low - d1_low) / (1. - 0.)
-                                    : d1_high + ((xp - 0.5) - 0.) * (d2_high - d1_high) / (1. - 0.);
-      const double pos = ((double)c.x_pos_offset[s] + disp) * inv_cell;
-      const double lo = pos - half, hi = pos + half;
-      if (lo >= 0.0 && hi < 1.0) {
-        atomicAdd(acc + kk, val);
-      } else if (lo < 0.0 && hi < 0.0) {
-        const double cd = ceil(fabs(lo)) - 1.;
-        const int ic = (int)cd;
-        if (fabs(hi) > cd) {
-          atomicAdd(acc + wrap(kk - (ic + 1)), val);
-        } else {
-          const double fo = (fabs(lo) - cd) * inv_w_sub, fw = 1. - fo;
-          put(kk - ic, fw);
-          put(kk - (ic + 1), fo);
+  double total = 0.0;
+  for (size_t row0 = (size_t)blockIdx.x * lines; row0 < nrows; row0 += (size_t)gridDim.x * lines) {
+    const int cells = (int)min((size_t)lines, nrows - row0) * n;
+    for (int i = threadIdx.x; i < cells; i += DT_NT) acc[i] = 0.f;
+    __syncthreads();
+    for (int i = threadIdx.x; i < cells; i += DT_NT) {
+      const int ln = i / n, kk = i - ln * n;
+      const size_t row = row0 + ln;
+      float* line = acc + ln * n;
+      const float* v = vc + row * padw;
+      const float d = dT[row * n + kk];
+      if (!(fabs((double)d) >= FRACT_FLOAT_ERR && (double)xH[row * n + kk] >= FRACT_FLOAT_ERR)) continue;
+      // displacements at the previous cell's, this and the next cell's centre, Mpc
+      const double d1 = (double)(v[kk == 0 ? n - 1 : kk - 1] / c.H_z);
+      const double d2 = (double)(v[kk] / c.H_z);
+      const double d3 = (double)(v[kk == n - 1 ? 0 : kk + 1] / c.H_z);
+      const double dd = (double)d / NS;
+      const double slope[2] = {(d2 - d1) * c.inv_cell, (d3 - d2) * c.inv_cell};
+      const double U[2] = {NS * d1 * c.inv_cell + 0.5 * NS * slope[0] + 0.5 * (1.0 + slope[0]) - 0.5,
+                           NS * d2 * c.inv_cell - 0.5 * NS * slope[1] + (c.n_low + 0.5) * (1.0 + slope[1]) - 0.5};
+      const double g0 = 1.0 + slope[0], g1 = 1.0 + slope[1];
+      if (g0 >= 0.02 && g0 <= 8.0 && g1 >= 0.02 && g1 <= 8.0 && fabs(U[0]) < 5e10 && fabs(U[1]) < 5e10) {
+        int cur = 0;   // the cell, relative to kk, whose share is kept
+        double share = 0.0;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int m = h ? N_RSD_STEPS - c.n_low : c.n_low;
+          const double g = h ? g1 : g0, inv_g = 1.0 / g;
+          const int k0 = (int)floor(U[h] * (1.0 / NS)), k1 = (int)floor((U[h] + (m - 1) * g + 1.0) * (1.0 / NS));
+          double left = 0.0;
+          for (int k = k0; k <= k1; ++k) {
+            double f = m;
+            if (k < k1) {
+              const double t = NS * (k + 1.0) - U[h];
+              const double n1 = fmin(fmax(floor((t - 1.0) * inv_g) + 1.0, 0.0), (double)m);
+              const double n2 = fmin(fmax(ceil(t * inv_g), n1), (double)m);
+              f = n1 + (n2 - n1) * t - 0.5 * g * (n2 * (n2 - 1.0) - n1 * (n1 - 1.0));
+            }
+            if (k != cur) {
+              if (share != 0.0) atomicAdd(line + wrap(kk + cur), (float)(share * dd));
+              cur = k;
+              share = 0.0;
+            }
+            share += f - left;
+            left = f;
+          }
         }
-      } else if (lo < 0.0 && (hi > 0.0 && hi < 1.0)) {
-        const double fw = hi * inv_w_sub, fo = 1. - fw;
-        put(kk - 1, fo);
-        put(kk, fw);
-      } else if ((lo >= 0.0 && lo < 1.0) && (hi >= 1.0)) {
-        const double fo = (hi - 1.) * inv_w_sub, fw = 1. - fo;
-        put(kk, fw);
-        put(kk + 1, fo);
-      } else {
-        const double cd = floor(fabs(hi));
-        const int ic = (int)cd;
-        if (lo >= cd) {
-          atomicAdd(acc + wrap(kk + ic), val);
+        if (share != 0.0) atomicAdd(line + wrap(kk + cur), (float)(share * dd));
+        continue;
+      }
+      const float val = d / (float)N_RSD_STEPS;
+      auto put = [&](int k, double frac) { atomicAdd(line + wrap(k), (float)(frac * dd)); };
+      for (int s = 0; s < N_RSD_STEPS; ++s) {
+        const double xp = (double)c.x_pos[s];
+        const double disp = s < c.n_low ? d1 + (xp + 0.5) * (d2 - d1) : d2 + (xp - 0.5) * (d3 - d2);
+        const double pos = ((double)c.x_pos_offset[s] + disp) * c.inv_cell;
+        const double lo = pos - c.half, hi = pos + c.half;
+        if (lo >= 0.0 && hi < 1.0) {
+          atomicAdd(line + kk, val);
+        } else if (lo < 0.0 && hi < 0.0) {
+          const double cd = ceil(fabs(lo)) - 1.;
+          const int ic = (int)cd;
+          if (fabs(hi) > cd) {
+            atomicAdd(line + wrap(kk - (ic + 1)), val);
+          } else {
+            const double fo = (fabs(lo) - cd) * c.inv_w_sub;
+            put(kk - ic, 1. - fo);
+            put(kk - (ic + 1), fo);
+          }
+        } else if (lo < 0.0 && (hi > 0.0 && hi < 1.0)) {
+          const double fw = hi * c.inv_w_sub;
+          put(kk - 1, 1. - fw);
+          put(kk, fw);
         } else {
-          const double fo = (hi - cd) * inv_w_sub, fw = 1. - fo;
-          put(kk + ic - 1, fw);
-          put(kk + ic, fo);
+          const double cd = floor(fabs(hi));
+          const int ic = (int)cd;
+          if (lo >= cd) {
+            atomicAdd(line + wrap(kk + ic), val);
+          } else {
+            const double fo = (hi - cd) * c.inv_w_sub;
+            put(kk + ic - 1, 1. - fo);
+            put(kk + ic, fo);
+          }
         }
       }
     }
-  }
-  __syncthreads();
-  for (int k = threadIdx.x; k < n; k += DT_NT) dT[row * n + k] = acc[k];
-}
-
-__global__ void __launch_bounds__(DT_NT) k_dT_sum(const float* __restrict__ dT, size_t n3, double* partials) {
-  double a = 0.0;
-  for (size_t i = (size_t)blockIdx.x * DT_NT + threadIdx.x; i < n3; i += (size_t)gridDim.x * DT_NT) a += dT[i];
-  __shared__ double sh[DT_NT];
-  sh[threadIdx.x] = a;
-  __syncthreads();
-  for (int w = DT_NT / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
     __syncthreads();
+    for (int i = threadIdx.x; i < cells; i += DT_NT) {
+      const float v = acc[i];
+      dT[row0 * n + i] = v;
+      total += (double)v;
+    }
+    __syncthreads();   // the lines are read before the next ones are zeroed
   }
-  if (threadIdx.x == 0) partials[blockIdx.x] = sh[0];
+  dt_block_sum(total, partials);
 }
 
 // the velocity stages after k_delta_T; leaves the FP64 sum of the final delta_T in partials
@@ -238,7 +318,9 @@ static int velocity_modes(rg_context* ctx, const rg_params* p, const rg_grids* g
   const Cosmo cm(p);
   const float H_z = (float)cm.hubble(redshift);
   prof_begin(ctx, "vel_convert", st);
-  k_vel_convert<<<nblocks, DT_NT, 0, st>>>(g->vel, vc, n, p->TreesID, redshift);
+  const double opz = 1. + (double)redshift;
+  k_vel_convert<<<nblocks, DT_NT, 0, st>>>(g->vel, vc, n, p->TreesID, p->TreesID == 1 ? std::sqrt(1. / opz) : opz,
+                                           1000. * 100. / MPC, opz);
   prof_end(ctx, 8.0 * n3, st);
   RG_CUDA_TRY(ctx, cudaGetLastError());
   const float* src = vc;
@@ -251,26 +333,33 @@ static int velocity_modes(rg_context* ctx, const rg_params* p, const rg_grids* g
   if ((rc = xy_ctrl_reset(ctx, (size_t)(n / 2 + 1), st))) return rc;
   if ((rc = spectrum_to_padded(ctx, grad, st))) return rc;
   prof_begin(ctx, "vel_correct", st);
-  k_vel_correct<<<nblocks, DT_NT, 0, st>>>(g->delta_T, grad, g->TS_box, n, flag, H_z, t_rad, redshift);
+  k_vel_correct<<<nblocks, DT_NT, 0, st>>>(g->delta_T, grad, g->TS_box, n, flag, H_z, t_rad, redshift,
+                                           ctx->partials);
   prof_end(ctx, 16.0 * n3, st);
   RG_CUDA_TRY(ctx, cudaGetLastError());
   if (flag == 3) {
     RsdConst c;
     const double box = p->BoxSize / p->Hubble_h;   // Mpc
-    c.sub_w = (box / ((double)n)) / (double)N_RSD_STEPS;
-    c.cell = box / (float)n;
-    for (int i = 0; i < N_RSD_STEPS; ++i) {
-      c.x_pos_offset[i] = (float)(c.sub_w * (float)i + c.sub_w / 2.);
-      c.x_pos[i] = (float)(c.x_pos_offset[i] / (box / (float)n));
-    }
+    const double sub_w = (box / ((double)n)) / (double)N_RSD_STEPS;
+    const double cell = box / (float)n;
+    c.inv_cell = 1.0 / cell;
+    c.inv_w_sub = cell / sub_w;
+    c.half = (sub_w / 2.) / cell;
     c.H_z = H_z;
+    c.n_low = 0;
+    for (int i = 0; i < N_RSD_STEPS; ++i) {
+      c.x_pos_offset[i] = (float)(sub_w * (float)i + sub_w / 2.);
+      c.x_pos[i] = (float)(c.x_pos_offset[i] / (box / (float)n));
+      // up to 0.5 between the previous cell's centre and this one's, beyond between this and the next
+      if ((double)c.x_pos[i] <= 0.5) c.n_low = i + 1;
+    }
+    // whole lines a block: 256 cells or one line
+    const int lines = std::max(1, DT_NT / n);
     prof_begin(ctx, "rsd_los", st);
-    k_rsd<<<(unsigned)((size_t)n * n), DT_NT, sizeof(float) * n, st>>>(g->delta_T, g->xH, vc, n, c);
+    k_rsd<<<nblocks, DT_NT, sizeof(float) * n * lines, st>>>(g->delta_T, g->xH, vc, n, lines, c, ctx->partials);
     prof_end(ctx, 16.0 * n3, st);
     RG_CUDA_TRY(ctx, cudaGetLastError());
   }
-  k_dT_sum<<<nblocks, DT_NT, 0, st>>>(g->delta_T, n3, ctx->partials);
-  RG_CUDA_TRY(ctx, cudaGetLastError());
   return RG_OK;
 }
 
