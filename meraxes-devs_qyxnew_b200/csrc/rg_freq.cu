@@ -4,12 +4,19 @@
 // Gauss-Kronrod rule (QUADPACK's QAGE) of the host engine in rg_xray.cpp, which serves the callers
 // without a device.
 //
-// What bounds it: one integral is a chain of rule applications, each 61 evaluations of about a
-// thousand dependent FP64 operations (cross sections, table interpolation), so a block of 64 threads
-// evaluates the 61 nodes of a rule side by side and the 1680 integrals of 40 shells (5040 with both
-// AGN bands) are 1680 blocks.  On 8 host threads the integrals took 9 to 10 ms a snapshot (19 ms with
-// both AGN bands), more than the rest of a 128^3 snapshot: ComputeTs went from 10.9 to 2.0 ms at
-// 128^3 and from 20.1 to 1.3 ms at 64^3 with both bands when they moved here.
+// What bounds them: an integral is a chain of rule applications, each 61 evaluations of about a
+// thousand dependent FP64 operations; where the interpolated tables jump (their index formula changes at
+// 1 keV) the rule halves its interval 20 times to get past it.  So a block takes one integral and
+// evaluates the 61 nodes of both halves side by side, each ion's part of the integrand in a group of
+// threads of its own, one step a halving.  The integrals of one shell and band share their frequencies:
+// the cross sections, spectrum and table positions at the nodes of the first four levels of halvings
+// are computed once (k_freq_nodes) for the 42 integrals that read them.
+//
+// On 8 host threads the integrals took 9 to 10 ms a snapshot (19 ms with both AGN bands), more than the
+// rest of a 128^3 snapshot: ComputeTs went from 10.9 to 2.0 ms at 128^3 and from 20.1 to 1.3 ms at 64^3
+// with both bands when they moved here, a rule at a time on 64 threads.  In steps of two halves and
+// three groups, nu_tau_one and the integrals went from 107 and 652 us (40 shells, on an
+// empty device) to 85 and 320, ComputeTs at 128^3 from 1.63 to 1.18 ms.
 #include <cfloat>
 #include <cstring>
 #include <vector>
@@ -20,7 +27,10 @@
 
 namespace rg {
 
-constexpr int FQ_NT = 64;          // threads of a block: one per rule node (61)
+constexpr int FQ_NT = 64;          // threads of a group: one per rule node (61)
+constexpr int FQ_BLOCK = 6 * FQ_NT;   // two intervals, three ions each
+constexpr int FQ_LEVELS = 4;       // halvings whose nodes are shared: intervals 0 .. 14 in heap order
+constexpr int FQ_SHARED = (1 << FQ_LEVELS) - 1;
 constexpr int FQ_LIMIT = 1000;     // intervals of one adaptive integral
 constexpr int FQ_BANDS = 3;        // galaxies, AGN soft, AGN hard
 
@@ -41,28 +51,21 @@ struct FreqConst {
 
 struct FqIv {
   double a, b, r, e;
+  int id;   // heap index: the halves of interval i are 2 i + 1 and 2 i + 2
 };
+__device__ __forceinline__ int fq_child(int id, int right) { return id < FQ_SHARED ? 2 * id + 1 + right : id; }
 
-// A block's integration workspace: partial sums of its two warps and the interval list.
+// A block's integration workspace: the parts of the integrand, the partial sums of each interval's first
+// two warps, and the interval list.
 struct FqShared {
-  double red[2][2][3];
+  double part[2][3][FQ_NT];
+  double red[2][2][2][3];   // [phase][interval][warp]
   FqIv iv[FQ_LIMIT];
 };
 
-// Sum of K values over the block; every thread gets the same bits.  `phase` alternates the buffer.
-template <int K>
-__device__ __forceinline__ void fq_sum(double (&v)[K], FqShared& sh, int phase) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-    for (int k = 0; k < K; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-  if ((threadIdx.x & 31) == 0)
-#pragma unroll
-    for (int k = 0; k < K; ++k) sh.red[phase][threadIdx.x >> 5][k] = v[k];
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < K; ++k) v[k] = sh.red[phase][0][k] + sh.red[phase][1][k];
-}
+struct FqRule {
+  double result, abserr, resabs, resasc;
+};
 
 __device__ __forceinline__ double fq_rescale(double err, double result_abs, double result_asc) {
   err = fabs(err);
@@ -77,47 +80,74 @@ __device__ __forceinline__ double fq_rescale(double err, double result_abs, doub
   return err;
 }
 
-// the 61-point rule over [a, b]: thread k < 30 of each warp takes node k on its side of the centre,
-// thread 30 of the first warp the centre
+// node k of a rule in thread order: lanes 0 .. 29 of the first warp take the nodes left of the centre,
+// lane 30 the centre, lanes 0 .. 29 of the second warp those right of it
+__device__ __forceinline__ bool fq_node_on(int thread) { return (thread & 31) < 30 || thread == 30; }
+__device__ __forceinline__ double fq_node_x(const FreqConst& c, double a, double b, int thread) {
+  const double center = 0.5 * (a + b), half = 0.5 * (b - a), d = half * c.X[thread & 31];
+  return thread < 32 ? center - d : center + d;
+}
+
+// the 61-point rule over n (1 or 2) intervals [iv[h].a, iv[h].b]; f(x, thread of the node, interval id,
+// ion) is one ion's part of the integrand.  Every thread of the block gets the same bits.
 template <class F>
-__device__ void fq_rule(const FreqConst& c, const F& f, double a, double b, FqShared& sh, double* result,
-                        double* abserr, double* resabs, double* resasc) {
-  const int k = threadIdx.x & 31, side = threadIdx.x >> 5;
-  const double center = 0.5 * (a + b), half = 0.5 * (b - a);
-  const bool on = k < 30 || (k == 30 && side == 0);
-  double fx = 0, wk = 0, wg = 0;
-  if (on) {
-    const double d = half * c.X[k];
-    fx = f(side ? center + d : center - d);
-    wk = c.WK[k];
-    wg = c.WG[k];
+__device__ void fq_rules(const FreqConst& c, const F& f, const FqIv (&iv)[2], int n, FqShared& sh, FqRule (&out)[2]) {
+  const int h = threadIdx.x / (3 * FQ_NT), ion = threadIdx.x / FQ_NT % 3, node = threadIdx.x % FQ_NT, k = node & 31;
+  const bool on = h < n && fq_node_on(node);
+  const double a = h ? iv[1].a : iv[0].a, b = h ? iv[1].b : iv[0].b;
+  sh.part[h][ion][node] = on ? f(fq_node_x(c, a, b, node), node, h ? iv[1].id : iv[0].id, ion) : 0.0;
+  __syncthreads();
+  const double wk = on ? c.WK[k] : 0.0, wg = on ? c.WG[k] : 0.0;
+  const bool adds = ion == 0 && h < n;   // whole warps
+  double fx = 0.0;
+  if (adds) {
+    fx = sh.part[h][0][node] + sh.part[h][1][node] + sh.part[h][2][node];
+    double s[3] = {wk * fx, wg * fx, wk * fabs(fx)};
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < 3; ++i) s[i] += __shfl_xor_sync(0xffffffffu, s[i], o);
+    if (k == 0)
+#pragma unroll
+      for (int i = 0; i < 3; ++i) sh.red[0][h][node >> 5][i] = s[i];
   }
-  double s[3] = {wk * fx, wg * fx, wk * fabs(fx)};
-  fq_sum<3>(s, sh, 0);
-  const double mean = 0.5 * s[0];
-  double asc[1] = {on ? wk * fabs(fx - mean) : 0.0};
-  fq_sum<1>(asc, sh, 1);
-  *result = s[0] * half;
-  *resabs = s[2] * fabs(half);
-  *resasc = asc[0] * fabs(half);
-  *abserr = fq_rescale((s[0] - s[1]) * half, *resabs, *resasc);
+  __syncthreads();
+  if (adds) {
+    const double mean = 0.5 * (sh.red[0][h][0][0] + sh.red[0][h][1][0]);
+    double d = on ? wk * fabs(fx - mean) : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+    if (k == 0) sh.red[1][h][node >> 5][0] = d;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    if (i >= n) break;
+    const double half = 0.5 * (iv[i].b - iv[i].a);
+    const double kronrod = sh.red[0][i][0][0] + sh.red[0][i][1][0], gauss = sh.red[0][i][0][1] + sh.red[0][i][1][1];
+    out[i].result = kronrod * half;
+    out[i].resabs = (sh.red[0][i][0][2] + sh.red[0][i][1][2]) * fabs(half);
+    out[i].resasc = (sh.red[1][i][0][0] + sh.red[1][i][1][0]) * fabs(half);
+    out[i].abserr = fq_rescale((kronrod - gauss) * half, out[i].resabs, out[i].resasc);
+  }
+  __syncthreads();   // the sums are read before the next rules write theirs
 }
 
 // QAGE; returns 0 on success.  Called by the whole block, the same scalars in every thread.
 template <class F>
 __device__ int fq_integrate(const FreqConst& c, const F& f, double a, double b, double epsrel, FqShared& sh,
                             double* result) {
-  double r0, e0, ra0, rc0;
-  fq_rule(c, f, a, b, sh, &r0, &e0, &ra0, &rc0);
-  double tolerance = epsrel * fabs(r0);
-  const double round_off = 50 * DBL_EPSILON * ra0;
-  *result = r0;
-  if (e0 <= round_off && e0 > tolerance) return 2;
-  if ((e0 <= tolerance && e0 != rc0) || e0 == 0.0) return 0;
-  __syncthreads();   // readers of an earlier integral's list are done
-  if (threadIdx.x == 0) sh.iv[0] = FqIv{a, b, r0, e0};
+  FqIv iv[2] = {FqIv{a, b, 0, 0, 0}, FqIv{a, b, 0, 0, 0}};
+  FqRule q[2];
+  fq_rules(c, f, iv, 1, sh, q);
+  double tolerance = epsrel * fabs(q[0].result);
+  const double round_off = 50 * DBL_EPSILON * q[0].resabs;
+  *result = q[0].result;
+  if (q[0].abserr <= round_off && q[0].abserr > tolerance) return 2;
+  if ((q[0].abserr <= tolerance && q[0].abserr != q[0].resasc) || q[0].abserr == 0.0) return 0;
+  if (threadIdx.x == 0) sh.iv[0] = FqIv{a, b, q[0].result, q[0].abserr, 0};
   __syncthreads();
-  double area = r0, errsum = e0;
+  double area = q[0].result, errsum = q[0].abserr;
   int n = 1, type1 = 0, type2 = 0, bad = 0;
   do {
     int im = 0;
@@ -125,13 +155,13 @@ __device__ int fq_integrate(const FreqConst& c, const F& f, double a, double b, 
       if (sh.iv[i].e > sh.iv[im].e) im = i;
     const FqIv cur = sh.iv[im];
     const double mid = 0.5 * (cur.a + cur.b);
-    double a1, e1, ab1, as1, a2, e2, ab2, as2;
-    fq_rule(c, f, cur.a, mid, sh, &a1, &e1, &ab1, &as1);
-    fq_rule(c, f, mid, cur.b, sh, &a2, &e2, &ab2, &as2);
-    const double area12 = a1 + a2, error12 = e1 + e2;
+    iv[0] = FqIv{cur.a, mid, 0, 0, fq_child(cur.id, 0)};
+    iv[1] = FqIv{mid, cur.b, 0, 0, fq_child(cur.id, 1)};
+    fq_rules(c, f, iv, 2, sh, q);   // ends with a barrier: cur is read everywhere
+    const double area12 = q[0].result + q[1].result, error12 = q[0].abserr + q[1].abserr;
     errsum += (error12 - cur.e);
     area += area12 - cur.r;
-    if (as1 != e1 && as2 != e2) {
+    if (q[0].resasc != q[0].abserr && q[1].resasc != q[1].abserr) {
       const double delta = cur.r - area12;
       if (fabs(delta) <= 1.0e-5 * fabs(area12) && error12 >= 0.99 * cur.e) type1++;
       if (n >= 10 && error12 > cur.e) type2++;
@@ -142,10 +172,9 @@ __device__ int fq_integrate(const FreqConst& c, const F& f, double a, double b, 
       const double tmp = (1 + 100 * DBL_EPSILON) * (fabs(mid) + 1000 * DBL_MIN);
       if (fabs(cur.a) <= tmp && fabs(cur.b) <= tmp) bad = 3;
     }
-    __syncthreads();
     if (threadIdx.x == 0) {
-      sh.iv[im] = FqIv{cur.a, mid, a1, e1};
-      sh.iv[n] = FqIv{mid, cur.b, a2, e2};
+      sh.iv[im] = FqIv{cur.a, mid, q[0].result, q[0].abserr, iv[0].id};
+      sh.iv[n] = FqIv{mid, cur.b, q[1].result, q[1].abserr, iv[1].id};
     }
     __syncthreads();
     ++n;
@@ -153,6 +182,7 @@ __device__ int fq_integrate(const FreqConst& c, const F& f, double a, double b, 
   double sum = 0;
   for (int i = 0; i < n; ++i) sum += sh.iv[i].r;
   *result = sum;
+  __syncthreads();   // the list is read before another integral starts
   if (errsum <= tolerance) return 0;
   return bad ? bad : 1;
 }
@@ -160,7 +190,7 @@ __device__ int fq_integrate(const FreqConst& c, const F& f, double a, double b, 
 // tauX(nu, x_e, zp, zpp); 1e10 where the integral fails, as the C does
 __device__ double fq_tau(const FreqConst& c, double nu, double zpp, FqShared& sh) {
   const double nu_0 = nu / (1 + c.zp);
-  auto f = [&](double z) {
+  auto f = [&](double z, int, int, int ion) {
     const double opz = (double)(1.0f + (float)z);   // dtdz takes a float redshift
     const double i1 = 1.0 / opz, i3 = i1 * i1 * i1;
     const double dt = c.dtdz_c * (i1 * i1 * sqrt(i1)) / sqrt(c.dtdz_s * i3 + 1);
@@ -170,8 +200,12 @@ __device__ double fq_tau(const FreqConst& c, double nu, double zpp, FqShared& sh
     if (fcoll < 0.0) fcoll = 0.0;
     double ff = fcoll < 1e-20 ? 1 : 1 - (c.ion_eff * fcoll) / (1.0 - c.x_e_ave);
     if (ff < 1e-4) ff = 1e-4;
-    const double sigma = c.f_H * (1 - c.x_e_ave) * HI_ion_crosssec(nu_h) +
-                         c.f_He * (1 - c.x_e_ave) * HeI_ion_crosssec(nu_h) + c.f_He * c.x_e_ave * HeII_ion_crosssec(nu_h);
+    double sigma;
+    if (ion == 1)
+      sigma = c.f_He * (1 - c.x_e_ave) * HeI_ion_crosssec(nu_h);
+    else   // the hydrogenic ions
+      sigma = (ion == 0 ? c.f_H * (1 - c.x_e_ave) : c.f_He * c.x_e_ave) *
+              hydrogenic_crosssec(nu_h, ion == 0 ? NUIONIZATION : HeII_NUIONIZATION, ion == 0 ? SIGMA_HI : 6.3e-18 / 4);
     return SPEED_OF_LIGHT * dt * (c.N_b0 * (o * o * o)) * ff * sigma;
   };
   double r;
@@ -180,7 +214,7 @@ __device__ double fq_tau(const FreqConst& c, double nu, double zpp, FqShared& sh
 
 // nu_tau_one: Brent's method on tauX - 1 between the HeI threshold and 1 MeV, to 2 per cent
 // (at most 100 iterations), one block per shell
-__global__ void __launch_bounds__(FQ_NT) k_freq_tau(const __grid_constant__ FreqConst c, const double* __restrict__ zpps,
+__global__ void __launch_bounds__(FQ_BLOCK) k_freq_tau(const __grid_constant__ FreqConst c, const double* __restrict__ zpps,
                                                     double* __restrict__ nu_one) {
   __shared__ FqShared sh;
   const double zpp = zpps[blockIdx.x];
@@ -273,18 +307,54 @@ __global__ void __launch_bounds__(FQ_NT) k_freq_tau(const __grid_constant__ Freq
   if (threadIdx.x == 0) nu_one[blockIdx.x] = root;
 }
 
+// limits of a band's integrals for shell r
+__device__ __forceinline__ void fq_limits(const FreqConst& c, int band, double zpp, double nu_one, double* lo,
+                                          double* hi) {
+  const double zf = c.redshifted[band] ? (1. + c.zp) / (1. + zpp) : 1.0;
+  *lo = fmax(nu_one, c.lo[band] * zf);
+  *hi = c.hi[band] * zf;
+}
+
+// the shared nodes of shell blockIdx.x and band blockIdx.y:
+// nodes[shell][band][interval][thread of a group][ion]
+__global__ void __launch_bounds__(256) k_freq_nodes(const __grid_constant__ FreqConst c,
+                                                    const double* __restrict__ zpps, const double* __restrict__ nu_one,
+                                                    XNode* __restrict__ nodes) {
+  double lo, hi;
+  fq_limits(c, blockIdx.y, zpps[blockIdx.x], nu_one[blockIdx.x], &lo, &hi);
+  if (!(lo < hi)) return;
+  XNode* out = nodes + ((size_t)blockIdx.x * c.nb + blockIdx.y) * FQ_SHARED * FQ_NT * 3;
+  const int j = blockIdx.z * 256 + threadIdx.x, ion = j / (FQ_SHARED * FQ_NT), i = j - ion * (FQ_SHARED * FQ_NT);
+  if (ion >= 3 || !fq_node_on(i % FQ_NT)) return;
+  // the interval's ends by the halvings that lead to it
+  double a = lo, b = hi;
+  const int id = i / FQ_NT + 1;
+  for (int l = 30 - __clz(id); l >= 0; --l) {
+    const double mid = 0.5 * (a + b);
+    if (id >> l & 1) a = mid;
+    else b = mid;
+  }
+  out[i * 3 + ion] =
+      xray_node(ion, c.t.E, c.f_H, c.f_He, c.alpha[blockIdx.y], c.nu_min, fq_node_x(c, a, b, i % FQ_NT));
+}
+
 // integrate_over_nu: block (shell, x_e node, 3 band + kind) into out[band][kind][node][shell]
-__global__ void __launch_bounds__(FQ_NT)
+__global__ void __launch_bounds__(FQ_BLOCK)
     k_freq_nu(const __grid_constant__ FreqConst c, const double* __restrict__ zpps, const double* __restrict__ nu_one,
-              double* __restrict__ out) {
+              const XNode* __restrict__ nodes, double* __restrict__ out) {
   __shared__ FqShared sh;
   const int r = blockIdx.x, m = blockIdx.y, band = blockIdx.z / 3, kind = blockIdx.z % 3;
-  const double zf = c.redshifted[band] ? (1. + c.zp) / (1. + zpps[r]) : 1.0;
-  const double lo = fmax(nu_one[r], c.lo[band] * zf), hi = c.hi[band] * zf;
+  double lo, hi;
+  fq_limits(c, band, zpps[r], nu_one[r], &lo, &hi);
   const double xe = (double)c.t.X[m];
+  const XNode* mine = nodes + ((size_t)r * c.nb + band) * FQ_SHARED * FQ_NT * 3;
   double v = 0.0;
   if (lo < hi) {
-    auto f = [&](double nu) { return xray_integrand(c.t, c.f_H, c.f_He, kind, xe, c.alpha[band], c.nu_min, nu); };
+    auto f = [&](double nu, int node, int id, int ion) {
+      const XNode x = id < FQ_SHARED ? mine[(id * FQ_NT + node) * 3 + ion]
+                                     : xray_node(ion, c.t.E, c.f_H, c.f_He, c.alpha[band], c.nu_min, nu);
+      return xray_part(c.t, kind, ion, xe, nu, x);
+    };
     if (fq_integrate(c, f, lo, hi, 0.01, sh, &v))
       v = 0.0;
     else if (kind == 2)
@@ -378,9 +448,13 @@ int ts_freq_start(rg_context* ctx, const rg_params* p, const TsShells& sh, doubl
   const int nS = sh.nS;
   c.nS = nS;
   c.nb = 1 + na;
-  // [zpp nS][nu_tau_one nS][tables c.nb 3 14 nS], the same layout on the device and in pinned memory
+  // [zpp nS][nu_tau_one nS][tables c.nb 3 14 nS], the same layout on the device and in pinned memory; on
+  // the device the shared nodes follow
   const size_t ntab = (size_t)c.nb * 3 * x_int_NXHII * nS, total = 2 * (size_t)nS + ntab;
-  if ((rc = ensure_device(ctx, &ctx->freq_d, &ctx->freq_d_elems, total))) return rc;
+  const size_t nnode = (size_t)nS * c.nb * FQ_SHARED * FQ_NT * 3;
+  static_assert(sizeof(XNode) % sizeof(double) == 0, "nodes behind doubles");
+  if ((rc = ensure_device(ctx, &ctx->freq_d, &ctx->freq_d_elems, total + nnode * sizeof(XNode) / sizeof(double))))
+    return rc;
   if (ctx->freq_h_elems < total) {
     if (ctx->freq_h) cudaFreeHost(ctx->freq_h);
     ctx->freq_h = nullptr;
@@ -394,9 +468,12 @@ int ts_freq_start(rg_context* ctx, const rg_params* p, const TsShells& sh, doubl
   cudaStream_t st = ctx->side_stream;
   double* d = ctx->freq_d;
   RG_CUDA_TRY(ctx, cudaMemcpyAsync(d, ctx->freq_h, sizeof(double) * nS, cudaMemcpyHostToDevice, st));
-  k_freq_tau<<<nS, FQ_NT, 0, st>>>(c, d, d + nS);
+  XNode* nodes = reinterpret_cast<XNode*>(d + total);
+  k_freq_tau<<<nS, FQ_BLOCK, 0, st>>>(c, d, d + nS);
   RG_CUDA_TRY(ctx, cudaGetLastError());
-  k_freq_nu<<<dim3(nS, x_int_NXHII, 3 * c.nb), FQ_NT, 0, st>>>(c, d, d + nS, d + 2 * nS);
+  k_freq_nodes<<<dim3(nS, c.nb, (3 * FQ_SHARED * FQ_NT + 255) / 256), 256, 0, st>>>(c, d, d + nS, nodes);
+  RG_CUDA_TRY(ctx, cudaGetLastError());
+  k_freq_nu<<<dim3(nS, x_int_NXHII, 3 * c.nb), FQ_BLOCK, 0, st>>>(c, d, d + nS, nodes, d + 2 * nS);
   RG_CUDA_TRY(ctx, cudaGetLastError());
   RG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->freq_h + nS, d + nS, sizeof(double) * (total - nS), cudaMemcpyDeviceToHost, st));
   return RG_OK;

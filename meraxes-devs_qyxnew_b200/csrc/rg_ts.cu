@@ -26,6 +26,7 @@
 #include <cstddef>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "rg_freq.h"
@@ -42,8 +43,11 @@ constexpr int TS_MAXSRC = 4;    // sources combined into one shell
 constexpr int TS_NSUM = 9;      // evolve sums (7, 8: the AGN heating of the two AGN units)
 constexpr int KSPL = 27;        // knots of the largest kappa table
 
+constexpr int KLUT = 64;
 struct KappaSpline {
   int n;
+  int lut[KLUT];           // last knot at or below the start of each of KLUT equal steps of the table
+  double x0, inv_step;
   double x[KSPL], y[KSPL], b[KSPL], c[KSPL], d[KSPL];
 };
 
@@ -62,20 +66,17 @@ struct TsZConst {
 
 struct TsDev {
   KappaSpline k10, kel, kpH;
+};
+// the scalars travel as a kernel parameter (operands of the constant bank)
+struct TsPar {
   TsZConst z;
   int max_iter;   // get_Ts fixed-point iterations before a cell counts as not converged
-  int pad_;
 };
 
 __device__ __forceinline__ double spline_eval(const KappaSpline& s, double x) {
-  int lo = 0, hi = s.n - 1;
-  while (hi > lo + 1) {
-    const int mid = (lo + hi) >> 1;
-    if (s.x[mid] > x)
-      hi = mid;
-    else
-      lo = mid;
-  }
+  // the last knot at or below x (x lies in the table), from the step's first candidate
+  int lo = s.lut[min(max((int)((x - s.x0) * s.inv_step), 0), KLUT - 1)];
+  while (lo < s.n - 2 && !(s.x[lo + 1] > x)) ++lo;
   const double dx = x - s.x[lo];
   return s.y[lo] + dx * (s.b[lo] + dx * (s.c[lo] + dx * s.d[lo]));
 }
@@ -100,11 +101,12 @@ __device__ __forceinline__ double log_kappa_table(const KappaSpline& s, double l
 // get_Ts with xcoll and the Wouthuysen-Field coupling (XRayHeatingFunctions.c:1639-1726,
 // 1973-2008).  The factors that do not change across the fixed-point iterations (xcoll, the
 // S_alpha terms in T_K only, xi) are evaluated once per cell.  The loop is capped at
-// C.max_iter iterations (10000 unless a test lowers it); a cell that reaches the cap counts in
+// P.max_iter iterations (10000 unless a test lowers it); a cell that reaches the cap counts in
 // *nonconv.
-__device__ float get_Ts(const TsDev& C, float delta, float TK, float xe, float Jalpha, float* curr_xalpha,
-                        int* nonconv) {
-  const TsZConst& Z = C.z;
+// The iteration runs on u = 1 / T_S, one division a step; |T_S - T_S,old| / T_S = |u_old - u| / u_old.
+__device__ __forceinline__ float get_Ts(const TsDev& C, const TsPar& P, float delta, float TK, float xe, float Jalpha,
+                                        float* curr_xalpha, int* nonconv) {
+  const TsZConst& Z = P.z;
   const double tk = (double)TK, d1 = 1.0 + (double)delta, x = (double)xe;
   const double lt = log(tk);
   const double xc = Z.xc_H * (1.0 - x) * d1 * exp(log_kappa_10(C.k10, lt)) +
@@ -120,20 +122,21 @@ __device__ float get_Ts(const TsDev& C, float delta, float TK, float xe, float J
     const double sb = (-0.401403 + 0.336463 * itk) * itk;                 // times 1 / T_S
     const double xaj = Z.xa0 * (double)Jalpha / den;
     const double ctc = 0.405535 * itk;
-    TS = Z.Trad;
-    double TSold = 0.0, xa_tilde = 0.0;
+    const double den_c = Z.inv_Trad + xc * itk, num_c = 1.0 + xc, tce_c = itk - ctc * itk;
+    double u = Z.inv_Trad, xa_tilde = 0.0;
     int it = 0;
-    while (fabs(TS - TSold) / TS > 1.0e-3) {
-      if (++it > C.max_iter) {
+    for (;;) {
+      if (++it > P.max_iter) {
         *nonconv += 1;
         break;
       }
-      TSold = TS;
-      const double u = 1.0 / TS;
+      const double uold = u;
       xa_tilde = xaj * (sa + sb * u);
-      const double tce_inv = itk + ctc * (u - itk);                        // 1 / Tc_eff
-      TS = (1.0 + xa_tilde + xc) / (Z.inv_Trad + xa_tilde * tce_inv + xc * itk);
+      // 1 / Tc_eff = 1 / T_K + ctc (1 / T_S - 1 / T_K)
+      u = (den_c + xa_tilde * (tce_c + ctc * u)) / (num_c + xa_tilde);
+      if (!(u > 0.0 && fabs(uold - u) > 1.0e-3 * uold)) break;
     }
+    TS = 1.0 / u;
     *curr_xalpha = (float)xa_tilde;
   } else {
     TS = (1.0 + xc) / (Z.inv_Trad + xc * itk);
@@ -197,23 +200,36 @@ __global__ void __launch_bounds__(256) k_ts_reduce0(const float* __restrict__ st
                                                     const float* __restrict__ xe, int n, double Mh2,
                                                     double fourthirds_pi_R3_over_pv, double* partials,
                                                     unsigned* __restrict__ xe_range) {
-  const int padw = 2 * (n / 2 + 1);
-  const size_t rows = (size_t)n * n;
+  constexpr int U = 4;   // cells of a thread whose loads are in flight together
+  const size_t n3 = (size_t)n * n * n, step = (size_t)gridDim.x * 256;
+  const double f = fourthirds_pi_R3_over_pv / Mh2;
   double acc[2] = {0.0, 0.0};
-  unsigned lo = ~0u, hi = 0u;   // range of x_e as ordered integers
-  for (size_t row = blockIdx.x; row < rows; row += gridDim.x)
-    for (int z = threadIdx.x; z < n; z += blockDim.x) {
-      const size_t ip = row * padw + z;
-      const double density_over_mean = 1.0 + (double)deltax[ip];
-      double c = (double)stars[ip] / (Mh2 * density_over_mean) * fourthirds_pi_R3_over_pv;
-      if (c > 1.0) c = 1.0;
-      acc[0] += c;
-      const float v = xe[ip];
-      acc[1] += (double)v;
-      const unsigned o = float_order(v);
-      lo = min(lo, o);
-      hi = max(hi, o);
+  float mn = INFINITY, mx = -INFINITY;
+  bool nan = false;
+  for (size_t i0 = (size_t)blockIdx.x * 256 + threadIdx.x; i0 < n3; i0 += U * step) {
+    float st[U], dx[U], v[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const size_t i = i0 + k * step;
+      if (i >= n3) break;
+      const size_t ip = i + ((unsigned)i / (unsigned)n) * 2;   // rows of n + 2 values
+      st[k] = stars[ip];
+      dx[k] = deltax[ip];
+      v[k] = xe[ip];
     }
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      if (i0 + k * step >= n3) break;
+      const double c = (double)st[k] * f / (1.0 + (double)dx[k]);
+      acc[0] += c > 1.0 ? 1.0 : c;
+      acc[1] += (double)v[k];
+      mn = fminf(mn, v[k]);
+      mx = fmaxf(mx, v[k]);
+      nan |= v[k] != v[k];
+    }
+  }
+  // the range of x_e as ordered integers; a NaN, which the minimum and maximum pass over, is its top
+  unsigned lo = float_order(mn), hi = nan ? ~0u : float_order(mx);
   block_sum_dyn<2>(acc, partials + (size_t)blockIdx.x * 2);
   __shared__ unsigned s_lo, s_hi;
   if (threadIdx.x == 0) {
@@ -355,9 +371,8 @@ __global__ void __launch_bounds__(YCfg<N>::NTH, RG_MINB(YCfg<N>::NTH))
 // are linear in the filtered grids xray_r and, between the table's x_e nodes X[m], linear in x_e:
 //   (1 - t) F_k[lo] + t F_k[lo + 1],  F_k[m] = sum_r f_rk(X[m]) xray_r,  t = (x_e - X[lo]) / (X[lo + 1] - X[lo])
 // so the sum over shells is taken in k-space, once per node that the box uses.  3 M transforms
-// instead of nS (M nodes: two where the whole box lies between neighbouring nodes).  At 512^3, 5
-// nodes and 40 shells, with the sharp-k pruning, ComputeTs went from 76.9 to 47.0 ms; at 256^3, 9
-// nodes, from 8.4 to 6.9 ms.
+// instead of nS (M nodes: two where the whole box lies between neighbouring nodes); ts_snapshot chooses
+// by cost.  At 128^3, 4 nodes and 40 sharp-k shells the X-ray part takes 0.53 ms by nodes, 0.61 by shells.
 
 struct TsNodeShell {
   int nk;                    // sources of the shell
@@ -422,10 +437,10 @@ struct TsEvolve {
 
 // One cell: sums[0..3] = the four evolveInt shell sums (heat, ion, lya, stellar lya) before
 // their snapshot prefactors; updates x_e and T_K, returns T_S and adds the cell to acc[0..6].
-__device__ __forceinline__ void evolve_cell(const TsDev& C, const TsEvolve& e, float delta, float xef, float tk0,
+__device__ __forceinline__ void evolve_cell(const TsDev& C, const TsPar& P, const TsEvolve& e, float delta, float xef, float tk0,
                                             const double (&sums)[4], float* xn_out, float* tk_out, float* ts_out,
                                             double (&acc)[TS_NSUM], int* nc) {
-  const TsZConst& Z = C.z;
+  const TsZConst& Z = P.z;
   const double x_e = (double)xef, T = (double)tk0;
   const double n_b = Z.nb0 * (double)(1.0f + delta);
   double dxheat_dt = 0, dxion_src = 0, dxlya = 0, dstarlya = 0;
@@ -459,7 +474,7 @@ __device__ __forceinline__ void evolve_cell(const TsDev& C, const TsEvolve& e, f
   if (tk < MAX_TK) tk = (float)((double)tk + d1 * e.dzp);
   if (tk < MIN_TK) tk = (float)(TCMB * (1 + e.zp));
   float xa;
-  const float ts = get_Ts(C, delta, tk, xn, (float)d2, &xa, nc);
+  const float ts = get_Ts(C, P, delta, tk, xn, (float)d2, &xa, nc);
   *xn_out = xn;
   *tk_out = tk;
   *ts_out = ts;
@@ -502,15 +517,19 @@ struct TsZev {
   double inv_scale[4];            // undo the FP32 scaling
 };
 
+// Plans: at 128 and 256 the default ones, one exchange at 16 values a thread (three blocks of 128
+// threads, up to 168 registers), elsewhere 8 values a thread (two blocks of 256).  At 256^3 the z pass of
+// 40 shells and 9 nodes took 1.86 ms with 8 values a thread and two exchanges, 1.64 with one.
 template <int N>
 struct TsZ {
-  using PL = Plan8<N>;
+  using PL = std::conditional_t<N == 128 || N == 256, Plan<N>, Plan8<N>>;
   static constexpr int T = PL::T;
-  static constexpr int V = N / T;            // 8
+  static constexpr int V = N / T;            // 8 or 16
   static constexpr int R0 = PL::R[0];
-  static constexpr int Q = pow2_div(N, cmax(256 / T, 4));   // rows per block
+  static constexpr int Q = pow2_div(N, cmax((V == 16 ? 128 : 256) / T, 4));   // rows per block
   static constexpr int NTH = T * Q;
-  static constexpr int MINB = NTH >= 512 ? 1 : 512 / NTH;   // 2 blocks of 256: at most 128 registers
+  static constexpr int MINB = V == 16 ? (NTH == 128 ? 3 : 1) : NTH >= 512 ? 1 : 512 / NTH;
+  using Nodes = std::conditional_t<V == 16, uint64_t, uint32_t>;   // four bits a cell
   static constexpr int NZ = N / 2 + 1;
   // A shell's rows come as up to NBOX tensor boxes of KZS + 1 kz rows, KZS apart (they overlap in one
   // row, so every box lands on a 128-byte boundary and none leaves the spectrum): as many as the
@@ -578,7 +597,8 @@ __global__ void __launch_bounds__(TsZ<N>::NTH, TsZ<N>::MINB)
   // this thread's cells: z = last_pos(t, s); x_e interpolation node and offset
   // (ComputeTs.c:1198-1209): by shells the offset itself, by nodes its share of the interval
   float dxe[V];
-  uint32_t lopack = 0;
+  typename Z::Nodes lopack = 0;
+  using Nodes = typename Z::Nodes;
 #pragma unroll
   for (int sl = 0; sl < V; ++sl) {
     double xc = (double)__ldg(xe_prev + row * PADW + last_pos<PL>(t, sl));
@@ -598,16 +618,16 @@ __global__ void __launch_bounds__(TsZ<N>::NTH, TsZ<N>::MINB)
         xm = zv.X[j];
         xn = zv.X[j + 1 < x_int_NXHII ? j + 1 : j];
       }
-    lopack |= (uint32_t)m << (4 * sl);
+    lopack |= (Nodes)m << (4 * sl);
     dxe[sl] = XS ? (float)(xc - (double)xm) : (float)((xc - (double)xm) / ((double)xn - (double)xm));
   }
   // every thread's cells each on one x_e node of their own (the common case early in
   // reionization): the coefficient reads leave the per-cell loops.  The choice is the block's, as
   // both paths run transforms with block barriers.
-  static_assert(V == 8, "eight x_e node indices in one 32-bit word");
-  const uint32_t lo0 = lopack & 15u;
+  static_assert(V == 8 || V == 16, "the cells' x_e node indices in one word");
+  const uint32_t lo0 = (uint32_t)lopack & 15u;
   bool uni = false;
-  if constexpr (XS) uni = __syncthreads_and(lopack == lo0 * 0x11111111u) != 0;
+  if constexpr (XS) uni = __syncthreads_and(lopack == (Nodes)(lo0 * 0x1111111111111111ull)) != 0;
   float a_heat[V], a_ion[V], a_lya[V], a_star[V];
   float a_agn0[NA > 0 ? V : 1], a_agn1[NA > 1 ? V : 1];
 #pragma unroll
@@ -782,59 +802,62 @@ __global__ void __launch_bounds__(TsZ<N>::NTH, TsZ<N>::MINB)
   }
 }
 
-// the per-cell update (ComputeTs.c:1171-1407) from the shell sums; sums == nullptr: no light
-__global__ void __launch_bounds__(256) k_ts_evolve(const TsDev* __restrict__ gC, TsEvolve e, double4 inv_scale, int n,
-                                                   const float4* __restrict__ sums,
-                                                   const float2* __restrict__ agn_heat,
-                                                   const float* __restrict__ deltax, float* __restrict__ xe_prev,
-                                                   float* __restrict__ xe_box, float* __restrict__ Tk,
-                                                   float* __restrict__ TS, double* __restrict__ partials,
-                                                   int* __restrict__ nonconv) {
+// the per-cell update (ComputeTs.c:1171-1407) from the shell sums; sums == nullptr: no light.  Cells
+// in memory order whatever the row length (a block per row left half of its threads idle at 128^3);
+// bound by its FP64 work, three exponentials, two logarithms, a cube root and the iteration a cell.
+// With the iteration on 1 / T_S, the scalars as parameters and the tables' index: 8.35 -> 7.25 ms at
+// 512^3, 0.25 -> 0.125 at 128^3.
+constexpr int EV_NT = 128;
+__global__ void __launch_bounds__(EV_NT, 5) k_ts_evolve(const TsDev* __restrict__ gC, const TsPar P, const TsEvolve e,
+                                                        double4 inv_scale, int n, const float4* __restrict__ sums,
+                                                        const float2* __restrict__ agn_heat,
+                                                        const float* __restrict__ deltax, float* __restrict__ xe_prev,
+                                                        float* __restrict__ xe_box, float* __restrict__ Tk,
+                                                        float* __restrict__ TS, double* __restrict__ partials,
+                                                        int* __restrict__ nonconv) {
   __shared__ TsDev C;
   {
     const int* src = reinterpret_cast<const int*>(gC);
     int* dst = reinterpret_cast<int*>(&C);
-    for (int i = threadIdx.x; i < (int)(sizeof(TsDev) / sizeof(int)); i += blockDim.x) dst[i] = src[i];
+    for (int i = threadIdx.x; i < (int)(sizeof(TsDev) / sizeof(int)); i += EV_NT) dst[i] = src[i];
   }
   __syncthreads();
-  const int padw = 2 * (n / 2 + 1);
-  const size_t rows = (size_t)n * n;
+  const size_t n3 = (size_t)n * n * n;
   double acc[TS_NSUM];
 #pragma unroll
   for (int i = 0; i < TS_NSUM; ++i) acc[i] = 0.0;
   int nc = 0;
-  for (size_t row = blockIdx.x; row < rows; row += gridDim.x)
-    for (int z = threadIdx.x; z < n; z += blockDim.x) {
-      const size_t ir = row * n + z, ip = row * padw + z;
-      double sm[4] = {0.0, 0.0, 0.0, 0.0};
-      if (sums) {
-        const float4 v = __ldg(sums + ir);
-        sm[0] = (double)v.x * inv_scale.x;
-        sm[1] = (double)v.y * inv_scale.y;
-        sm[2] = (double)v.z * inv_scale.z;
-        sm[3] = (double)v.w * inv_scale.w;
-      }
-      float xn, tk, ts;
-      const float xe0 = xe_prev[ip];
-      if (agn_heat) {
-        // the AGN heating terms of dT_K/dz (XRayHeatingFunctions.c:1519-1520) for their averages
-        const float2 a = __ldg(agn_heat + ir);
-        const double f = inv_scale.x * e.const_zp * e.heat_conv / (1.0 + (double)xe0);
-        acc[7] += (double)a.x * f;
-        acc[8] += (double)a.y * f;
-      }
-      evolve_cell(C, e, __ldg(deltax + ip), xe0, Tk[ir], sm, &xn, &tk, &ts, acc, &nc);
-      xe_prev[ip] = xn;
-      xe_box[ip] = xn;
-      Tk[ir] = tk;
-      TS[ir] = ts;
+  for (size_t ir = (size_t)blockIdx.x * EV_NT + threadIdx.x; ir < n3; ir += (size_t)gridDim.x * EV_NT) {
+    const size_t ip = ir + ((unsigned)ir / (unsigned)n) * 2;   // rows of n + 2 values
+    double sm[4] = {0.0, 0.0, 0.0, 0.0};
+    if (sums) {
+      const float4 v = __ldg(sums + ir);
+      sm[0] = (double)v.x * inv_scale.x;
+      sm[1] = (double)v.y * inv_scale.y;
+      sm[2] = (double)v.z * inv_scale.z;
+      sm[3] = (double)v.w * inv_scale.w;
     }
+    float xn, tk, ts;
+    const float xe0 = xe_prev[ip];
+    if (agn_heat) {
+      // the AGN heating terms of dT_K/dz (XRayHeatingFunctions.c:1519-1520) for their averages
+      const float2 a = __ldg(agn_heat + ir);
+      const double f = inv_scale.x * e.const_zp * e.heat_conv / (1.0 + (double)xe0);
+      acc[7] += (double)a.x * f;
+      acc[8] += (double)a.y * f;
+    }
+    evolve_cell(C, P, e, __ldg(deltax + ip), xe0, Tk[ir], sm, &xn, &tk, &ts, acc, &nc);
+    xe_prev[ip] = xn;
+    xe_box[ip] = xn;
+    Tk[ir] = tk;
+    TS[ir] = ts;
+  }
   if (nc) atomicAdd(nonconv, nc);
   block_sum_dyn<TS_NSUM>(acc, partials + (size_t)blockIdx.x * TS_NSUM);
 }
 
 // homogeneous branch (ComputeTs.c:252-278) and the closing averages (:1459-1494)
-__global__ void __launch_bounds__(256) k_ts_homog(const TsDev* __restrict__ gC, float xe0, float TK0,
+__global__ void __launch_bounds__(256) k_ts_homog(const TsDev* __restrict__ gC, const TsPar P, float xe0, float TK0,
                                                   float cT_ad, int n, const float* __restrict__ deltax,
                                                   float* __restrict__ xe_prev, float* __restrict__ xe_box,
                                                   float* __restrict__ Tk, float* __restrict__ TS,
@@ -858,7 +881,7 @@ __global__ void __launch_bounds__(256) k_ts_homog(const TsDev* __restrict__ gC, 
       const float delta = deltax[ip];
       const float tk = (float)((double)TK0 * (1.0 + (double)(cT_ad * delta)));
       float xa;
-      const float ts = get_Ts(C, delta, tk, xe0, 0.f, &xa, &nc);
+      const float ts = get_Ts(C, P, delta, tk, xe0, 0.f, &xa, &nc);
       xe_prev[ip] = xe0;
       xe_box[ip] = xe0;
       Tk[ir] = tk;
@@ -886,6 +909,14 @@ static void fill_spline(const CubicSpline& sp, const std::vector<double>& lx, co
       double a;
       sp.coeffs((size_t)i, &a, &k->b[i], &k->c[i], &k->d[i]);
     }
+  }
+  const double step = (lx.back() - lx[0]) / KLUT;
+  k->x0 = lx[0];
+  k->inv_step = 1.0 / step;
+  for (int s = 0, lo = 0; s < KLUT; ++s) {
+    // (a knot within rounding of the step's start is left to the device's search)
+    while (lo < k->n - 2 && lx[lo + 1] < lx[0] + (s - 1e-6) * step) ++lo;
+    k->lut[s] = lo;
   }
 }
 
@@ -1130,13 +1161,14 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
   fill_spline(ctx->tables.k10, ctx->tables.k10_lT, ctx->tables.k10_lk, &hc.k10);
   fill_spline(ctx->tables.kel, ctx->tables.kel_lT, ctx->tables.kel_lk, &hc.kel);
   fill_spline(ctx->tables.kpH, ctx->tables.kpH_lT, ctx->tables.kpH_lk, &hc.kpH);
-  hc.max_iter = ctx->ts_iter_limit;
+  TsPar par;
+  par.max_iter = ctx->ts_iter_limit;
   {
     // per-redshift factors of xcoll / taugp / xalpha_tilde / dT_comp / evolveInt; the C passes
     // the redshift to them as a float
     const float zf = (float)zp;
     const double z = (double)zf;
-    TsZConst& Z = hc.z;
+    TsZConst& Z = par.z;
     Z.Trad = TCMB * (1.0 + z);
     Z.inv_Trad = 1.0 / Z.Trad;
     const double opz3 = std::pow(1.0 + z, 3.0);
@@ -1226,7 +1258,7 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
     const float TK0 = (float)T_RECFAST(ctx->tables, (float)zp);
     prof_begin(ctx, "ts_homog", st);
     if ((rc = stage_wait(ctx, stg->closing, st))) return rc;   // Tk_box is overwritten
-    k_ts_homog<<<nblk, 256, 0, st>>>(d_hc, xe0, TK0, cT_approx((float)zp), N, g->deltax, g->x_e_box_prev,
+    k_ts_homog<<<nblk, 256, 0, st>>>(d_hc, par, xe0, TK0, cT_approx((float)zp), N, g->deltax, g->x_e_box_prev,
                                       g->x_e_box, g->Tk_box, g->TS_box, partials, d_nonconv);
     prof_end(ctx, 28.0 * n3, st);
     RG_CUDA_TRY(ctx, cudaGetLastError());
@@ -1269,9 +1301,20 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
       wide = wide || nk > TS_MAXSRC;
     }
     const int nused = std::max(1, (int)used.size());
-    // X-ray by nodes where 3 fields per node are fewer than the shells: the nodes m0 .. m0 + nm - 1
-    // around the box's x_e (clamped as each cell's is).  A shell with its combination in a spare
-    // slot, which later batches overwrite, and a NaN in x_e keep the shells.
+    // window cuts (filter() takes BoxSize in Mpc/h and R in Mpc, ComputeTs.c:532)
+    const int n2max = 3 * (N / 2) * (N / 2);
+    const bool sharp = p->TsHeatingFilterType == 1;
+    std::vector<int> cut(nS, TS_NOCUT);   // no filter on the first shell (ComputeTs.c:529)
+    if (sharp)
+      for (int r = 1; r < nS; ++r) cut[r] = sharpk_cut(2.0 * M_PI / p->BoxSize, sh.R[r], n2max);
+    // X-ray by nodes (m0 .. m0 + nm - 1, around the box's x_e clamped as each cell's is) or by shells,
+    // whichever costs less.  In units of a z unit (two spectra): a node takes three fields through
+    // k_ts_nodes and the x and y passes and 1.5 z units, 5.8 to 6.4 units measured at 128^3 to 512^3;
+    // a pair of shells a z unit with the table look-ups, 1.15 to 1.5, and a pass over what its window
+    // leaves, 0.42 a full one.  With 40 sharp-k shells the line lies between 4 and 6 nodes: 512^3 with 5
+    // nodes 24.8 ms by nodes and 21.8 by shells, 256^3 with 9 4.2 and 2.9, 128^3 with 4 0.53 and 0.61.
+    // A shell with its combination in a spare slot, which later batches overwrite, and a NaN in x_e
+    // keep the shells.
     auto node = [&](float v) {
       const float* X = ctx->tables.x_int_XHII.data();
       const double top = (double)X[x_int_NXHII - 1] * 0.999;
@@ -1281,7 +1324,12 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
     if (!wide && !std::isnan(xe_lo) && !std::isnan(xe_hi)) {
       zv.m0 = node(xe_lo);
       zv.nm = node(xe_hi) + 2 - zv.m0;
-      if (3 * zv.nm >= nS) zv.nm = 0;
+      double passes = 0;
+      for (int r = 0; r < nS; ++r) {
+        const double k = std::sqrt((double)cut[r]) / (N / 2);
+        passes += std::min(1.0, M_PI / 4 * k * k) + std::min(1.0, k);
+      }
+      if (6.0 * zv.nm >= 1.25 * (0.5 * nS) + 0.42 * passes) zv.nm = 0;
     }
     const int xs = zv.nm == 0;              // X-ray grids per shell
     const int Gs = 1 + xs + nagn;           // grids per shell
@@ -1306,13 +1354,8 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
       return src_host ? ctx->ts_stage + (j * G + which) * npad : src_grid(used[j], which);
     };
     // window rows for the shells (filter() takes BoxSize in Mpc/h and R in Mpc, ComputeTs.c:532)
-    const int n2max = 3 * (N / 2) * (N / 2);
-    // (the sharp-k rows are steps: their ends are all the passes need)
-    const bool sharp = p->TsHeatingFilterType == 1;
-    std::vector<int> cut(nS, TS_NOCUT);   // no filter on the first shell (ComputeTs.c:529)
-    if (sharp) {
-      for (int r = 1; r < nS; ++r) cut[r] = sharpk_cut(2.0 * M_PI / p->BoxSize, sh.R[r], n2max);
-    } else {
+    // (the sharp-k rows are steps: their cuts are all the passes need)
+    if (!sharp) {
       if ((rc = ensure_device(ctx, &ctx->d_radii, &ctx->d_radii_elems, (size_t)nS))) return rc;
       RG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->d_radii, sh.R.data(), sizeof(double) * nS, cudaMemcpyHostToDevice, st));
       if ((rc = ensure_device(ctx, &ctx->wtab, &ctx->wtab_elems, (size_t)nS * (n2max + 1)))) return rc;
@@ -1518,7 +1561,7 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
   const double4 inv = make_double4(zv.inv_scale[0], zv.inv_scale[1], zv.inv_scale[2], zv.inv_scale[3]);
   prof_begin(ctx, "ts_evolve", st);
   if ((rc = stage_wait(ctx, stg->closing, st))) return rc;
-  k_ts_evolve<<<nblk, 256, 0, st>>>(d_hc, e, inv, N, no_light ? nullptr : ctx->ts_sums,
+  k_ts_evolve<<<nblk, EV_NT, 0, st>>>(d_hc, par, e, inv, N, no_light ? nullptr : ctx->ts_sums,
                                      (no_light || !nagn) ? nullptr : ctx->ts_agn, g->deltax, g->x_e_box_prev,
                                      g->x_e_box, g->Tk_box, g->TS_box, partials, d_nonconv);
   prof_end(ctx, (double)n3 * (16 + 4 + 4 + 4 + 4 + 4 + 4 + 4), st);

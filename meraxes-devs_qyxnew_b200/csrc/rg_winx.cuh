@@ -14,7 +14,7 @@ struct WinX {
   static constexpr int V = N / T;
   static constexpr int B = Cfg<N>::BX;   // columns of a block
   static constexpr int NTH = T * B;
-  static constexpr int MINB = NTH >= 256 ? 3 : NTH >= 128 ? 5 : 8;
+  static constexpr int MINB = NTH >= 512 ? 1 : NTH >= 256 ? 3 : NTH >= 128 ? 5 : 8;
   static constexpr size_t smem() { return sizeof(cf) * (N + (size_t)line_buf_r0<N, PL::R[0], B>()); }
 };
 

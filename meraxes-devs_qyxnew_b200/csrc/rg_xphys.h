@@ -53,56 +53,67 @@ RG_HD inline int locate_xHII_index(const float* X, float x) {
   return m;
 }
 
-// bilinear interpolation of one table, float arithmetic in the order of the C
-RG_HD inline float interp_x_int(const XInt& t, const float* tab, float En, float xHII_call, float below) {
+RG_HD inline double xray_ion(int i) { return i == 0 ? NUIONIZATION : i == 1 ? HeI_NUIONIZATION : HeII_NUIONIZATION; }
+
+// What the integrands of one frequency share for an ion (0 HI, 1 HeI, 2 HeII), whatever the x_e and the
+// kind: the cross section times its number fraction and the spectrum (nu / nu0)^(-alpha - 1), the
+// electron energy within the tables and the energy interval it lies in (-1: below the tables).
+struct XNode {
+  double g;
+  float en;
+  int lo;
+};
+
+// nu0: the threshold frequency the spectrum is normalised at
+RG_HD inline XNode xray_node(int ion, const float* E, double f_H, double f_He, double alpha, double nu0, double nu) {
+  XNode x;
+  const double sigma = ion == 1 ? HeI_ion_crosssec(nu)
+                                : hydrogenic_crosssec(nu, ion == 0 ? NUIONIZATION : HeII_NUIONIZATION,
+                                                      ion == 0 ? SIGMA_HI : 6.3e-18 / 4);
+  x.g = (ion == 0 ? f_H : f_He) * sigma * pow(nu / nu0, -alpha - 1);
+  x.en = (float)((nu - xray_ion(ion)) / NU_over_EV);
+  if ((double)x.en > 0.999 * (double)E[x_int_NENERGY - 1]) x.en = (float)((double)E[x_int_NENERGY - 1] * 0.999);
+  x.lo = x.en < E[0] ? -1 : locate_energy_index(x.en);
+  return x;
+}
+
+// bilinear interpolation of one table at (energy en in interval n_low, x_e xf), float arithmetic in the
+// order of the C
+RG_HD inline float interp_x_int(const XInt& t, const float* tab, float en, int n_low, float xf, float below) {
   const float *E = t.E, *X = t.X;
-  if ((double)En > 0.999 * (double)E[x_int_NENERGY - 1]) {
-    En = (float)((double)E[x_int_NENERGY - 1] * 0.999);
-  } else if (En < E[0]) {
-    return below;
+  if (n_low < 0) return below;
+  if ((double)xf > (double)X[x_int_NXHII - 1] * 0.999) {
+    xf = (float)((double)X[x_int_NXHII - 1] * 0.999);
+  } else if (xf < X[0]) {
+    xf = (float)(1.001 * (double)X[0]);
   }
-  if ((double)xHII_call > (double)X[x_int_NXHII - 1] * 0.999) {
-    xHII_call = (float)((double)X[x_int_NXHII - 1] * 0.999);
-  } else if (xHII_call < X[0]) {
-    xHII_call = (float)(1.001 * (double)X[0]);
-  }
-  const int n_low = locate_energy_index(En), n_high = n_low + 1;
-  const int m_low = locate_xHII_index(X, xHII_call), m_high = m_low + 1;
+  const int n_high = n_low + 1;
+  const int m_low = locate_xHII_index(X, xf), m_high = m_low + 1;
   const float* lo = tab + m_low * x_int_NENERGY;
   const float* hi = tab + m_high * x_int_NENERGY;
   float elow = ((lo[n_high] - lo[n_low]) / (E[n_high] - E[n_low]));
-  elow *= (En - E[n_low]);
+  elow *= (en - E[n_low]);
   elow += lo[n_low];
   float ehigh = ((hi[n_high] - hi[n_low]) / (E[n_high] - E[n_low]));
-  ehigh *= (En - E[n_low]);
+  ehigh *= (en - E[n_low]);
   ehigh += hi[n_low];
   float r = (ehigh - elow) / (X[m_high] - X[m_low]);
-  r *= (xHII_call - X[m_low]);
+  r *= (xf - X[m_low]);
   r += elow;
   return r;
 }
 
-// integrand of integrate_over_nu: kind 0 heating, 1 ionisation, 2 Lyman-alpha; nu0 the threshold
-// frequency the spectrum nu^-alpha is normalised at
-RG_HD inline double xray_integrand(const XInt& t, double f_H, double f_He, int kind, double x_e, double alpha,
-                                   double nu0, double nu) {
+// an ion's part of the integrand of integrate_over_nu at frequency nu: kind 0 heating, 1 ionisation,
+// 2 Lyman-alpha
+RG_HD inline double xray_part(const XInt& t, int kind, int ion, double x_e, double nu, const XNode& x) {
   const float xf = (float)x_e;
-  const double ion[3] = {NUIONIZATION, HeI_NUIONIZATION, HeII_NUIONIZATION};
-  const double sig[3] = {f_H * (1 - x_e) * HI_ion_crosssec(nu), f_He * (1 - x_e) * HeI_ion_crosssec(nu),
-                         f_He * x_e * HeII_ion_crosssec(nu)};
-  double s = 0;
-  for (int i = 0; i < 3; ++i) {
-    const float en = (float)((nu - ion[i]) / NU_over_EV);
-    if (kind == 0)
-      s += interp_x_int(t, t.fheat, en, xf, 1.0f) * PLANCK * (nu - ion[i]) * sig[i];
-    else if (kind == 1)
-      s += (interp_x_int(t, t.nion_HI, en, xf, 0.0f) + interp_x_int(t, t.nion_HeI, en, xf, 0.0f) +
-            interp_x_int(t, t.nion_HeII, en, xf, 0.0f) + 1) *
-           sig[i];
-    else
-      s += interp_x_int(t, t.n_Lya, en, xf, 0.0f) * sig[i];
-  }
-  return s * pow(nu / nu0, -alpha - 1);
+  const double g = x.g * (ion < 2 ? 1 - x_e : x_e);
+  if (kind == 0) return interp_x_int(t, t.fheat, x.en, x.lo, xf, 1.0f) * PLANCK * (nu - xray_ion(ion)) * g;
+  if (kind == 1)
+    return (interp_x_int(t, t.nion_HI, x.en, x.lo, xf, 0.0f) + interp_x_int(t, t.nion_HeI, x.en, x.lo, xf, 0.0f) +
+            interp_x_int(t, t.nion_HeII, x.en, x.lo, xf, 0.0f) + 1) *
+           g;
+  return interp_x_int(t, t.n_Lya, x.en, x.lo, xf, 0.0f) * g;
 }
 
 }  // namespace rg

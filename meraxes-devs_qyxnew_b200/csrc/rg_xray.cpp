@@ -480,7 +480,11 @@ int ts_tables(const rg_params* p, const Tables& t, const TsShells& sh, double zp
   auto integrate_over_nu = [&](double local_x_e, double lo, double hi, int FLAG, double alpha) {
     if (lo >= hi) return 0.0;
     auto f = [&](double nu) {
-      return xray_integrand(xi, cm.f_H, cm.f_He, FLAG, local_x_e, alpha, thresh * NU_over_EV, nu);
+      double s = 0;
+      for (int ion = 0; ion < 3; ++ion)
+        s += xray_part(xi, FLAG, ion, local_x_e, nu,
+                       xray_node(ion, xi.E, cm.f_H, cm.f_He, alpha, thresh * NU_over_EV, nu));
+      return s;
     };
     double result, error;
     const int status = qag61(f, lo, hi, 0, 0.01, 1000, &result, &error);
