@@ -404,8 +404,9 @@ int rg_delta_T(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const 
   if (vel_modes && (rc = velocity_modes(ctx, p, g, redshift, t_rad, nblocks, st))) return rc;
   if ((rc = reduce_partials(ctx, ctx->partials, nblocks, 1, ctx->d_sums, st))) return rc;
   RG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_sums, ctx->d_sums, sizeof(double), cudaMemcpyDeviceToHost, st));
+  if (vel_modes && (rc = xy_ctrl_fetch(ctx, st))) return rc;
   RG_CUDA_TRY(ctx, cudaStreamSynchronize(st));
-  if (vel_modes && (rc = xy_ctrl_check(ctx, st))) return rc;
+  if (vel_modes && (rc = xy_ctrl_result(ctx))) return rc;
   // the reference divides by N^3 before its Allreduce (BrightnessTemperature.c:528); on one rank
   // that is the same division
   *volume_ave_Tb = ctx->h_sums[0] / std::pow((double)n, 3);

@@ -154,9 +154,16 @@ __device__ __forceinline__ void block_sum(double (&acc)[K], double* out) {
 // cell's temperature, ComputePartiallyIoinizedTemperature of the neutral gas's T at residual xH 1,
 // is that T: Tk_box with the spin temperature, else the adiabatic T; the floor is the same T.
 constexpr int CLOSE_NT = 256;
+struct HiiCloseUnits {   // snapshots of a launch (blockIdx.y)
+  HiiConst c[HII_ZU];
+  HiiState s[HII_ZU];
+};
 
 template <int N>
-__global__ void __launch_bounds__(CLOSE_NT) k_hii_close(HiiConst c, HiiState s, double* __restrict__ partials) {
+__global__ void __launch_bounds__(CLOSE_NT) k_hii_close(const __grid_constant__ HiiCloseUnits us,
+                                                        double* __restrict__ partials) {
+  const HiiConst& c = us.c[blockIdx.y];
+  const HiiState& s = us.s[blockIdx.y];
   constexpr int PADW = 2 * (N / 2 + 1);
   const size_t n3 = (size_t)N * N * N;
   double acc[HII_NSUM];
@@ -185,16 +192,17 @@ __global__ void __launch_bounds__(CLOSE_NT) k_hii_close(HiiConst c, HiiState s, 
     acc[7] += (double)temp * domu;
     acc[8] += domu;
   }
-  block_sum<CLOSE_NT, HII_NSUM>(acc, partials + (size_t)blockIdx.x * HII_NSUM);
+  block_sum<CLOSE_NT, HII_NSUM>(acc, partials + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * HII_NSUM);
 }
 
 template <int N>
-int launch_hii_close(rg_context* ctx, const HiiConst& c, const HiiState& s, double* partials, int nblocks,
+int launch_hii_close(rg_context* ctx, const HiiCloseUnits& us, int nu, double* partials, int nblocks,
                      cudaStream_t st) {
   prof_begin(ctx, "hii_close", st);
-  k_hii_close<N><<<nblocks, CLOSE_NT, 0, st>>>(c, s, partials);
+  k_hii_close<N><<<dim3(nblocks, nu), CLOSE_NT, 0, st>>>(us, partials);
   // xH, deltax, z_at_ionization, temperature, weighted_sfr (and Tk_box, ...) read, xH and temperature written
-  prof_end(ctx, 4.0 * N * N * N * (7 + c.spin + (s.bhar != nullptr) + (s.wsfrIII != nullptr)), st);
+  prof_end(ctx, nu * 4.0 * N * N * N * (7 + us.c[0].spin + (us.s[0].bhar != nullptr) + (us.s[0].wsfrIII != nullptr)),
+           st);
   RG_CUDA_TRY(ctx, cudaGetLastError());
   return RG_OK;
 }
@@ -655,9 +663,20 @@ static int hii_z(rg_context* ctx, int n, const cf* work, size_t stride, int ng, 
 // snapshots one z launch takes at this size
 static int hii_z_units(int n) { return n <= 128 ? HII_ZU : 1; }
 
-static int hii_close(rg_context* ctx, int n, const HiiConst& c, const HiiState& s, double* partials, int nblocks,
-                     cudaStream_t st) {
-  RG_DISPATCH_N(n, launch_hii_close<NN>(ctx, c, s, partials, nblocks, st));
+// the closing passes of nu snapshots; snapshot u's partial sums at partials + u nblocks HII_NSUM
+static int hii_close(rg_context* ctx, int n, const HiiConst* c, const HiiState* s, int nu, double* partials,
+                     int nblocks, cudaStream_t st) {
+  for (int u0 = 0; u0 < nu; u0 += HII_ZU) {
+    const int cu = std::min(HII_ZU, nu - u0);
+    HiiCloseUnits us;
+    std::copy(c + u0, c + u0 + cu, us.c);
+    std::copy(s + u0, s + u0 + cu, us.s);
+    double* p = partials + (size_t)u0 * nblocks * HII_NSUM;
+    auto go = [&]() -> int { RG_DISPATCH_N(n, launch_hii_close<NN>(ctx, us, cu, p, nblocks, st)); };
+    const int rc = go();
+    if (rc) return rc;
+  }
+  return RG_OK;
 }
 
 static int hii_recomb(rg_context* ctx, int n, const RecTables& tab, const RecConst& c, const RecState& s,
@@ -702,15 +721,27 @@ int xy_ctrl_reset(rg_context* ctx, size_t max_jobs, cudaStream_t st) {
   return RG_OK;
 }
 
-int xy_ctrl_check(rg_context* ctx, cudaStream_t st) {
-  if (!ctx->xy_ctrl) return RG_OK;
-  uint32_t err = 0;
-  RG_CUDA_TRY(ctx, cudaMemcpyAsync(&err, ctx->xy_ctrl, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-  RG_CUDA_TRY(ctx, cudaStreamSynchronize(st));
+int xy_ctrl_fetch(rg_context* ctx, cudaStream_t st) {
+  std::memset(ctx->h_sums + 63, 0, sizeof(double));
+  if (ctx->xy_ctrl)
+    RG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_sums + 63, ctx->xy_ctrl, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+  return RG_OK;
+}
+
+int xy_ctrl_result(rg_context* ctx) {
+  uint32_t err;
+  std::memcpy(&err, ctx->h_sums + 63, sizeof(err));
   if (err)
     return set_error(ctx, RG_ETIMEDOUT,
                      "a bounded device wait ran out (the fused x/y pass's wait for a plane, or a tensor tile's)");
   return RG_OK;
+}
+
+int xy_ctrl_check(rg_context* ctx, cudaStream_t st) {
+  int rc = xy_ctrl_fetch(ctx, st);
+  if (rc) return rc;
+  RG_CUDA_TRY(ctx, cudaStreamSynchronize(st));
+  return xy_ctrl_result(ctx);
 }
 
 // ---------------------------------------------------------------------------
@@ -963,7 +994,7 @@ int hii_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, cons
     if ((rc = hii_z(ctx, N, ctx->work, nc, ntest, 1, us, b3, st))) return rc;
   }
   if ((rc = stage_wait(ctx, stg->closing, st))) return rc;
-  if ((rc = hii_close(ctx, N, c, hs, partials, cb, st))) return rc;
+  if ((rc = hii_close(ctx, N, &c, &hs, 1, partials, cb, st))) return rc;
   if ((rc = reduce_partials(ctx, partials, cb, HII_NSUM, ctx->d_sums, st))) return rc;
   if (rec) {
     RecTables tab;
@@ -998,9 +1029,10 @@ int hii_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, cons
     if ((rc = reduce_partials(ctx, partials, rb, REC_NSUM, ctx->d_sums + 16, st))) return rc;
   }
   RG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_sums, ctx->d_sums, sizeof(double) * 32, cudaMemcpyDeviceToHost, st));
+  if ((rc = xy_ctrl_fetch(ctx, st))) return rc;
   RG_CUDA_TRY(ctx, cudaStreamSynchronize(st));
   prof_resolve(ctx);
-  if ((rc = xy_ctrl_check(ctx, st))) return rc;
+  if ((rc = xy_ctrl_result(ctx))) return rc;
   hii_outputs(p, nr, ctx->h_sums, out);
   return RG_OK;
 }
@@ -1094,14 +1126,14 @@ int hii_batch(rg_context* ctx, int nu, const rg_params* p, const rg_snapshot* s,
         return rc;
     }
   }
-  for (int u = 0; u < nu; ++u)
-    if ((rc = hii_close(ctx, N, cs[u], hs[u], partials + (size_t)u * cb * HII_NSUM, cb, st))) return rc;
+  if ((rc = hii_close(ctx, N, cs.data(), hs.data(), nu, partials, cb, st))) return rc;
   if ((rc = reduce_partials(ctx, partials, cb, HII_NSUM, ctx->batch_sums, st, nu, (size_t)cb * HII_NSUM, 32))) return rc;
   RG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_batch_sums, ctx->batch_sums, sizeof(double) * 32 * nu,
                                    cudaMemcpyDeviceToHost, st));
+  if ((rc = xy_ctrl_fetch(ctx, st))) return rc;
   RG_CUDA_TRY(ctx, cudaStreamSynchronize(st));
   prof_resolve(ctx);
-  if ((rc = xy_ctrl_check(ctx, st))) return rc;
+  if ((rc = xy_ctrl_result(ctx))) return rc;
   for (int u = 0; u < nu; ++u) hii_outputs(&p[u], nr, ctx->h_batch_sums + 32 * u, &out[u]);
   return RG_OK;
 }

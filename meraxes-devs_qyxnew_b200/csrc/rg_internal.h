@@ -179,6 +179,10 @@ int twiddles_for(rg_context* ctx, int n, const cf** out);
 // the host after a stream sync and returns RG_ETIMEDOUT when a wait ran out.
 int xy_ctrl_reset(rg_context* ctx, size_t max_jobs, cudaStream_t st);
 int xy_ctrl_check(rg_context* ctx, cudaStream_t st);
+// the same without a synchronisation of its own: queue the copy of the error word into pinned memory,
+// and read it after the stream has been synchronised
+int xy_ctrl_fetch(rg_context* ctx, cudaStream_t st);
+int xy_ctrl_result(rg_context* ctx);
 
 // Per-kernel event timing (active when ctx->prof_on).  prof_begin records a start event on
 // the stream; prof_end records the stop event and the launch's algorithmic bytes.
@@ -233,7 +237,8 @@ struct rg_context {
   double* partials = nullptr;
   size_t partials_elems = 0;
   double* d_sums = nullptr;      // reduced sums
-  double* h_sums = nullptr;      // pinned host copy
+  double* h_sums = nullptr;      // pinned host copy [64]; [63] the error word of the device waits
+  std::vector<char> ts_host;     // ComputeTs: coefficients on their way to the device
   double* batch_sums = nullptr;  // rg_find_HII_bubbles_batch: reduced sums per snapshot [unit][32]
   size_t batch_sums_elems = 0;
   double* h_batch_sums = nullptr;   // their pinned host copy (h_batch_sums_elems snapshots)

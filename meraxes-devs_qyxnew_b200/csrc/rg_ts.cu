@@ -814,7 +814,8 @@ __global__ void __launch_bounds__(EV_NT, 5) k_ts_evolve(const TsDev* __restrict_
                                                         const float* __restrict__ deltax, float* __restrict__ xe_prev,
                                                         float* __restrict__ xe_box, float* __restrict__ Tk,
                                                         float* __restrict__ TS, double* __restrict__ partials,
-                                                        int* __restrict__ nonconv) {
+                                                        int* __restrict__ nonconv, const uint32_t* __restrict__ err) {
+  if (err && *err) return;   // a tile's wait ran out: the sums are not to be used, the state stays
   __shared__ TsDev C;
   {
     const int* src = reinterpret_cast<const int*>(gC);
@@ -1207,14 +1208,18 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
   const double Mh2 = rtom(p, R0) * p->Hubble_h * p->Hubble_h;
   const double ftpr3 = (4.0 / 3.0) * M_PI * std::pow(R0, 3.0) / pixel_volume;
 
+  bool waits = false;   // kernels with device waits were launched
   auto finish = [&](bool homog, int nblocks) -> int {
     if ((rc = kick())) return rc;
     if ((rc = reduce_partials(ctx, partials, nblocks, TS_NSUM, ctx->d_sums, st))) return rc;
     RG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_sums, ctx->d_sums, sizeof(double) * TS_NSUM, cudaMemcpyDeviceToHost, st));
-    int nonconv = 0;
-    RG_CUDA_TRY(ctx, cudaMemcpyAsync(&nonconv, d_nonconv, sizeof(int), cudaMemcpyDeviceToHost, st));
+    RG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_sums + 62, d_nonconv, sizeof(int), cudaMemcpyDeviceToHost, st));
+    if (waits && (rc = xy_ctrl_fetch(ctx, st))) return rc;
     RG_CUDA_TRY(ctx, cudaStreamSynchronize(st));
     prof_resolve(ctx);
+    if (waits && (rc = xy_ctrl_result(ctx))) return rc;
+    int nonconv;
+    std::memcpy(&nonconv, ctx->h_sums + 62, sizeof(nonconv));
     const double* S = ctx->h_sums;
     const double nn = (double)n3;
     if (!homog) {
@@ -1527,10 +1532,15 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
             hco[r].QA[j][kind][m] = (float)(QAd[o] * scale[kind]);
           }
     }
-    RG_CUDA_TRY(ctx, cudaMemcpyAsync(d_co, hco.data(), sizeof(TsShellCoef) * (nS + 1), cudaMemcpyHostToDevice, st));
+    // the copies' source lives in the context: nothing here waits for them
+    const size_t co_bytes = sizeof(TsShellCoef) * (nS + 1), node_bytes = zv.nm ? sizeof(TsNodeShell) * nS : 0;
+    ctx->ts_host.resize(co_bytes + node_bytes);
+    std::memcpy(ctx->ts_host.data(), hco.data(), co_bytes);
+    if (node_bytes) std::memcpy(ctx->ts_host.data() + co_bytes, nodes.data(), node_bytes);
+    RG_CUDA_TRY(ctx, cudaMemcpyAsync(d_co, ctx->ts_host.data(), co_bytes, cudaMemcpyHostToDevice, st));
     zv.nS = nS;
     if (zv.nm) {
-      RG_CUDA_TRY(ctx, cudaMemcpyAsync(d_node, nodes.data(), sizeof(TsNodeShell) * nS, cudaMemcpyHostToDevice, st));
+      RG_CUDA_TRY(ctx, cudaMemcpyAsync(d_node, ctx->ts_host.data() + co_bytes, node_bytes, cudaMemcpyHostToDevice, st));
       if ((rc = ts_nodes(ctx, N, ctx->spec, ctx->work + (size_t)nS * Gs * nc, nc, G, d_node, nS, zv.nm, ctx->wtab,
                          n2max + 1, st)))
         return rc;
@@ -1543,8 +1553,7 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
     if ((rc = ts_zsum(ctx, N, ctx->work, nc, nagn, d_co, zv, g->x_e_box_prev, ctx->ts_sums,
                       nagn ? ctx->ts_agn : nullptr, planes, st)))
       return rc;
-    RG_CUDA_TRY(ctx, cudaStreamSynchronize(st));  // hco outlives the copy
-    if ((rc = xy_ctrl_check(ctx, st))) return rc;
+    waits = true;
   }
 
   TsEvolve e;
@@ -1563,7 +1572,8 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
   if ((rc = stage_wait(ctx, stg->closing, st))) return rc;
   k_ts_evolve<<<nblk, EV_NT, 0, st>>>(d_hc, par, e, inv, N, no_light ? nullptr : ctx->ts_sums,
                                      (no_light || !nagn) ? nullptr : ctx->ts_agn, g->deltax, g->x_e_box_prev,
-                                     g->x_e_box, g->Tk_box, g->TS_box, partials, d_nonconv);
+                                     g->x_e_box, g->Tk_box, g->TS_box, partials, d_nonconv,
+                                     no_light ? nullptr : ctx->xy_ctrl);
   prof_end(ctx, (double)n3 * (16 + 4 + 4 + 4 + 4 + 4 + 4 + 4), st);
   RG_CUDA_TRY(ctx, cudaGetLastError());
   return finish(false, nblk);
