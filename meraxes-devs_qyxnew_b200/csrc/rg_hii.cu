@@ -947,8 +947,9 @@ int hii_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, cons
   // one state byte per cell between radius batches (in words of four)
   if ((rc = ensure_device(ctx, &ctx->bits, &ctx->bits_elems, ((size_t)N * N * N + 3) / 4))) return rc;
   if ((rc = stage_wait(ctx, stg->inputs, st))) return rc;
-  for (int g0 = 0; g0 < ng; g0 += MAXG)   // at most MAXG grids per forward launch
-    if ((rc = fft_forward(ctx, N, srcs + g0, std::min(MAXG, ng - g0), ctx->spec + nc * g0, nc,
+  const int fg = fft_forward_group(N);   // grids per forward launch
+  for (int g0 = 0; g0 < ng; g0 += fg)
+    if ((rc = fft_forward(ctx, N, srcs + g0, std::min(fg, ng - g0), ctx->spec + nc * g0, nc,
                           1.0 / std::pow((double)N, 3), st)))
       return rc;
 
@@ -1079,8 +1080,9 @@ int hii_batch(rg_context* ctx, int nu, const rg_params* p, const rg_snapshot* s,
       return set_error(ctx, RG_ENOMEM, "pinned batch sums");
     ctx->h_batch_sums_elems = (size_t)nu;
   }
-  for (int g0 = 0; g0 < ng; g0 += MAXG)
-    if ((rc = fft_forward(ctx, N, srcs.data() + g0, std::min(MAXG, ng - g0), ctx->spec + nc * g0, nc,
+  const int fg = fft_forward_group(N);
+  for (int g0 = 0; g0 < ng; g0 += fg)
+    if ((rc = fft_forward(ctx, N, srcs.data() + g0, std::min(fg, ng - g0), ctx->spec + nc * g0, nc,
                           1.0 / std::pow((double)N, 3), st)))
       return rc;
   if ((rc = hii_windows(ctx, &p[0], sched, st))) return rc;

@@ -114,6 +114,7 @@ constexpr int HII_NSUM = 10;  // closing-pass sums
 constexpr int KB_MAX = 16;    // radii per batch
 
 // Forward r2c of ng padded real grids into spectra spec_base + g * stride, scaled.
+int fft_forward_group(int n);   // grids a call of fft_forward takes
 int fft_forward(rg_context* ctx, int n, const float* const* d_real, int ng, cf* spec_base, size_t stride,
                 double scale, cudaStream_t st);
 // Windowed inverse x and y passes of nr radii of the ng spectra at spec (ngu per snapshot) into

@@ -144,7 +144,7 @@ cudaError_t na_roundtrip(unsigned char* base, const float* in, float* out, doubl
   cf* tw = reinterpret_cast<cf*>(base + NA_TW_OFF);
   const size_t nc = (size_t)C::NZ * N * N;
   k_na_twiddles<<<1, N, 0, st>>>(tw, N);
-  GridPtrs srcs{};
+  FwdSrcs srcs{};
   srcs.p[0] = in;
   k_fwd_z<N><<<dim3(N / (2 * ZFCfg<N>::QF), N, 1), ZFCfg<N>::NTH, na_smem_fz<N>(), st>>>(srcs, spec, nc, tw);
   k_pass_y<N, false><<<dim3(N / YCfg<N>::BY, C::NZ, 1), YCfg<N>::NTH, na_smem_y<N>(), st>>>(spec, nc, tw);

@@ -38,7 +38,8 @@
 
 namespace rg {
 
-constexpr int TS_KB = 8;        // shells per batch
+constexpr int TS_KB = 8;        // spare slots for combinations, and the least shells per batch
+constexpr int TS_MAXB = 40;     // most shells per batch
 constexpr int TS_MAXSRC = 4;    // sources combined into one shell
 constexpr int TS_NSUM = 9;      // evolve sums (7, 8: the AGN heating of the two AGN units)
 constexpr int KSPL = 27;        // knots of the largest kappa table
@@ -255,12 +256,13 @@ __global__ void __launch_bounds__(256) k_ts_reduce0(const float* __restrict__ st
 
 struct TsBatch {
   int nr;
-  int nk[TS_KB];
-  int ks[TS_KB][TS_MAXSRC];
-  float cs[TS_KB][TS_MAXSRC];
-  int filtered[TS_KB];
-  int wrow[TS_KB];
-  int cut[TS_KB];     // last n2 that the shell's window keeps (TS_NOCUT: all)
+  int chunk;          // shells a block of the x pass takes
+  int nk[TS_MAXB];
+  int ks[TS_MAXB][TS_MAXSRC];
+  float cs[TS_MAXB][TS_MAXSRC];
+  int filtered[TS_MAXB];
+  int wrow[TS_MAXB];
+  int cut[TS_MAXB];     // last n2 that the shell's window keeps (TS_NOCUT: all)
   int gs;             // grids per source: sfr, X-ray, then 0 to 2 AGN bands
   int ng;             // grids per shell: the same, without X-ray where that goes by nodes
   int skip;           // 1: X-ray goes by nodes
@@ -271,7 +273,7 @@ constexpr int TS_NOCUT = 0x7fffffff;
 // At 512^3 with 40 sharp-k shells the shells' volumes add up to 4 grids of 40 and their columns to 6.
 template <int N>
 __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::BX, (x_pass_minb<N>()))
-    k_ts_x(const cf* __restrict__ spec, size_t stride, cf* __restrict__ work, TsBatch bt,
+    k_ts_x(const cf* __restrict__ spec, size_t stride, cf* __restrict__ work, const __grid_constant__ TsBatch bt,
            const float* __restrict__ wtab, int wpitch, const cf* __restrict__ g_tw) {
   constexpr int T = Cfg<N>::T, B = Cfg<N>::BX, V = Cfg<N>::V;
   extern __shared__ cf smem[];
@@ -295,7 +297,8 @@ __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::BX, (x_pass_minb<N>()))
     n2[sl] = nx * nx + ny * ny + kz * kz;
   }
   __syncthreads();
-  for (int r = 0; r < bt.nr; ++r) {
+  const int r_end = min(bt.nr, ((int)blockIdx.z + 1) * bt.chunk);
+  for (int r = blockIdx.z * bt.chunk; r < r_end; ++r) {
     const int cut = bt.cut[r];
     if (n2min > cut) continue;
     float wv[V];
@@ -342,7 +345,7 @@ __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::BX, (x_pass_minb<N>()))
 // batch's planes.  blockIdx.z: shell r, grid g at work + (r ng + g) stride.
 template <int N>
 __global__ void __launch_bounds__(YCfg<N>::NTH, RG_MINB(YCfg<N>::NTH))
-    k_ts_y(cf* __restrict__ work, size_t stride, TsBatch bt, const cf* __restrict__ g_tw) {
+    k_ts_y(cf* __restrict__ work, size_t stride, const __grid_constant__ TsBatch bt, const cf* __restrict__ g_tw) {
   using Y = YCfg<N>;
   using PL = typename Y::PL;
   constexpr int T = Y::T, B = Y::BY;
@@ -978,7 +981,7 @@ static int ts_combine(rg_context* ctx, int n, cf* spec, size_t stride, int G, co
 // fused x/y kernel of find_HII_bubbles, run on these batches, measured slower at 512^3: 48.8 ms
 // against 43.5 ms for the two passes; the x pass here reads its history spectra mostly from L2.)
 template <int N>
-static int launch_ts_xy(rg_context* ctx, const cf* spec, cf* work_base, size_t stride, const TsBatch& bt,
+static int launch_ts_xy(rg_context* ctx, const cf* spec, cf* work_base, size_t stride, TsBatch& bt,
                         const float* wtab, int wpitch, cudaStream_t st) {
   using C = Cfg<N>;
   const cf* tw;
@@ -999,7 +1002,12 @@ static int launch_ts_xy(rg_context* ctx, const cf* spec, cf* work_base, size_t s
   const size_t smx = sizeof(cf) * (N + (size_t)line_buf<N, C::BX>());
   RG_CUDA_TRY(ctx, cudaFuncSetAttribute(k_ts_x<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smx));
   prof_begin(ctx, "ts_x_c2c_combine_window", st);
-  k_ts_x<N><<<dim3(N / C::BX, kzmax + 1), C::T * C::BX, smx, st>>>(spec, stride, work_base, bt, wtab, wpitch, tw);
+  // A block takes up to 8 shells, which mostly combine the same sources; fewer where that leaves under 8
+  // blocks an SM.  40 shells of 3 grids at 64^3, x and y passes with the frequency integrals running
+  // beside: 216 us in one launch each of 2 shells a block, 321 in five launches of 8.
+  const int per_shell = (N / C::BX) * (kzmax + 1);
+  bt.chunk = std::min(TS_KB, std::max(1, bt.nr * per_shell / (8 * ctx->num_sms)));
+  k_ts_x<N><<<dim3(N / C::BX, kzmax + 1, (bt.nr + bt.chunk - 1) / bt.chunk), C::T * C::BX, smx, st>>>(spec, stride, work_base, bt, wtab, wpitch, tw);
   prof_end(ctx, bt.ng * 8.0 * (src_reads + cols), st);
   RG_CUDA_TRY(ctx, cudaGetLastError());
   using Y = YCfg<N>;
@@ -1094,7 +1102,7 @@ static int launch_ts_zsum(rg_context* ctx, const cf* work, size_t stride, int na
     default: return set_error(ctx, RG_EUNSUPPORTED, "ComputeTs needs a power-of-two ReionGridDim"); \
   }
 
-static int ts_xy(rg_context* ctx, int n, const cf* spec, cf* work_base, size_t stride, const TsBatch& bt,
+static int ts_xy(rg_context* ctx, int n, const cf* spec, cf* work_base, size_t stride, TsBatch& bt,
                  const float* wtab, int wpitch, cudaStream_t st) {
   RG_TS_DISPATCH(n, launch_ts_xy<NN>(ctx, spec, work_base, stride, bt, wtab, wpitch, st));
 }
@@ -1371,19 +1379,24 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
     std::vector<TsNodeShell> nodes(nS);
     std::memset(nodes.data(), 0, sizeof(TsNodeShell) * nodes.size());
 
-    // Batches of TS_KB shells: the forward transforms of the sources a batch uses first (`used`
+    // Batches of shells, as many as 128 MB of spectra hold (the windows leave a part of each) but at least
+    // TS_KB, and TS_KB where combinations pass through the spare slots: the forward transforms of the sources a batch uses first (`used`
     // is in order of first use), then its x and y passes into work[r][g].  From host arrays,
     // each group of sources is copied on the copy stream and its transform waits for the copy,
     // so the copies of later sources overlap the passes of earlier batches.
     size_t next_slot = 0;   // used[0, next_slot) are transformed into spec[slot * G + g]
-    for (int r0 = 0; r0 < nS; r0 += TS_KB) {
-      const int cnt = std::min(TS_KB, nS - r0);
+    const int kb = wide ? TS_KB
+                        : std::min(TS_MAXB, std::max(TS_KB, (int)(128.0 * 1024 * 1024 / (8.0 * nc * Gs))));
+    // sources per forward launch: host arrays come in small groups, whose copies overlap the passes
+    const size_t group = (src_host ? MAXG : fft_forward_group(N)) / G;
+    for (int r0 = 0; r0 < nS; r0 += kb) {
+      const int cnt = std::min(kb, nS - r0);
       size_t need = next_slot;
       for (int r = r0; r < r0 + cnt; ++r)
         for (int k = 0; k < sh.nsrc; ++k)
           if (sh.coef[(size_t)r * sh.nsrc + k] != 0.f) need = std::max(need, (size_t)slot_of[k] + 1);
       while (next_slot < need) {
-        const size_t end = std::min(need, next_slot + (size_t)(MAXG / G));
+        const size_t end = std::min(need, next_slot + group);
         if (src_host) {
           for (size_t j = next_slot; j < end; ++j)
             for (int which = 0; which < G; ++which)
@@ -1393,7 +1406,7 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
           if ((rc = stage_record(ctx, 4 + next_slot, ctx->copy_stream, &e))) return rc;
           if ((rc = stage_wait(ctx, e, st))) return rc;
         }
-        const float* srcs[MAXG];
+        const float* srcs[FWD_MAXG];
         int ng = 0;
         for (size_t j = next_slot; j < end; ++j)
           for (int which = 0; which < G; ++which) srcs[ng++] = dev_grid(j, which);
