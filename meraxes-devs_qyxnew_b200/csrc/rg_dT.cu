@@ -196,9 +196,10 @@ struct RsdConst {
 //   F(B) = sum_s clamp(B - L_s, 0, 1) = n1 + sum over n1 <= s < n2 of (B - U - s g),
 // n1 sub-cells wholly left of B and n2 that reach it: a closed form in FP64, and a cell gets F(right
 // edge) - F(left edge).  Two or three cells a side instead of 50 sub-cells with one or two shared-memory
-// adds each (compare-and-swap loops, in divergent branches): 3.17 -> 0.51 ms at 256^3.  Where the
-// sub-cells cross or spread (g outside [1/50, 8]) or are far off, infinite or not numbers, they are
-// moved one by one as in the reference.
+// adds each (compare-and-swap loops, in divergent branches): 3.17 -> 0.51 ms at 256^3; on velocities that
+// cross and spread the sub-cells everywhere (white noise, 512^3) 43.0 -> 6.4 ms, and 51.2 with those cells one
+// by one.  Where they spread over more than 16 cells a side (|g| beyond 32) or are far off, infinite or not
+// numbers, they are moved one by one as in the reference.
 __global__ void __launch_bounds__(DT_NT) k_rsd(float* __restrict__ dT, const float* __restrict__ xH,
                                                const float* __restrict__ vc, int n, int lines, const RsdConst c,
                                                double* __restrict__ partials) {
@@ -228,19 +229,21 @@ __global__ void __launch_bounds__(DT_NT) k_rsd(float* __restrict__ dT, const flo
       const double U[2] = {NS * d1 * c.inv_cell + 0.5 * NS * slope[0] + 0.5 * (1.0 + slope[0]) - 0.5,
                            NS * d2 * c.inv_cell - 0.5 * NS * slope[1] + (c.n_low + 0.5) * (1.0 + slope[1]) - 0.5};
       const double g0 = 1.0 + slope[0], g1 = 1.0 + slope[1];
-      if (g0 >= 0.02 && g0 <= 8.0 && g1 >= 0.02 && g1 <= 8.0 && fabs(U[0]) < 5e10 && fabs(U[1]) < 5e10) {
+      if (fabs(g0) <= 32.0 && fabs(g1) <= 32.0 && fabs(U[0]) < 5e10 && fabs(U[1]) < 5e10) {
         int cur = 0;   // the cell, relative to kk, whose share is kept
         double share = 0.0;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int m = h ? N_RSD_STEPS - c.n_low : c.n_low;
-          const double g = h ? g1 : g0, inv_g = 1.0 / g;
-          const int k0 = (int)floor(U[h] * (1.0 / NS)), k1 = (int)floor((U[h] + (m - 1) * g + 1.0) * (1.0 / NS));
+          // crossed sub-cells (g < 0) counted from their other end; g = 0: the infinities and NaN of
+          // inv_g end at the bounds of n1 and n2
+          const double gs = h ? g1 : g0, g = fabs(gs), inv_g = 1.0 / g, L0 = gs < 0.0 ? U[h] + (m - 1) * gs : U[h];
+          const int k0 = (int)floor(L0 * (1.0 / NS)), k1 = (int)floor((L0 + (m - 1) * g + 1.0) * (1.0 / NS));
           double left = 0.0;
           for (int k = k0; k <= k1; ++k) {
             double f = m;
             if (k < k1) {
-              const double t = NS * (k + 1.0) - U[h];
+              const double t = NS * (k + 1.0) - L0;
               const double n1 = fmin(fmax(floor((t - 1.0) * inv_g) + 1.0, 0.0), (double)m);
               const double n2 = fmin(fmax(ceil(t * inv_g), n1), (double)m);
               f = n1 + (n2 - n1) * t - 0.5 * g * (n2 * (n2 - 1.0) - n1 * (n1 - 1.0));
