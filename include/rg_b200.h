@@ -384,6 +384,12 @@ int rg_debug_ts_agn_tables(const rg_params* p, const rg_snapshot* s, int n_hist,
 int rg_debug_ts_device_tables(rg_context* ctx, const rg_params* p, const rg_snapshot* s, int n_hist, double x_e_ave,
                               double collapse_fraction, int max_shells, double* freq);
 
+/* How rg_compute_Ts forms the X-ray sums of a box whose x_e lies in [xe_lo, xe_hi] (host only):
+     out[0], out[1] first x_e node and number of nodes; no nodes: shell by shell
+     out[2]         launches side by side that form the nodes' fields
+     out[3], out[4] coefficients they read of a shell, and how many a shell holds. */
+int rg_debug_ts_nodes(const rg_params* p, const rg_snapshot* s, int n_hist, float xe_lo, float xe_hi, int* out);
+
 /* ---- allocation-free round trip (no counterpart in the reference) ----
    rg_debug_filter_roundtrip without a context and without any device allocation, for
    callers that cannot allocate: one that has given the device's memory to its own pool,

@@ -867,6 +867,18 @@ int rg_debug_ts_device_tables(rg_context* ctx, const rg_params* p, const rg_snap
   return RG_OK;
 }
 
+int rg_debug_ts_nodes(const rg_params* p, const rg_snapshot* s, int n_hist, float xe_lo, float xe_hi, int* out) {
+  if (!p || !s || !s->ZZ || !out || n_hist < 0 || p->ReionGridDim < 8) return RG_EINVAL;
+  if (s->snapshot < 0 || s->snapshot >= s->n_snapshots || p->TsNumFilterSteps < 1) return RG_EINVAL;
+  TsShells sh = ts_shells(p, s->ZZ, s->n_snapshots, s->snapshot, n_hist);
+  if (sh.error) return RG_EINVAL;
+  Tables t;
+  if (!p->TablesForXHeatingDir) return RG_ETABLE;
+  if (!load_tables(p->TablesForXHeatingDir, p->ReionNionPhotPerBary, &t).empty()) return RG_ETABLE;
+  ts_debug_nodes(p, sh, t.x_int_XHII.data(), xe_lo, xe_hi, out);
+  return RG_OK;
+}
+
 int rg_debug_ts_agn_tables(const rg_params* p, const rg_snapshot* s, int n_hist, double x_e_ave,
                            double collapse_fraction, int max_shells, double* agn, double* const_zp) {
   if (!p || !s || !s->ZZ || !agn || !const_zp || n_hist < 0) return RG_EINVAL;

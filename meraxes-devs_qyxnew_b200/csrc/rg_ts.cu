@@ -377,12 +377,26 @@ __global__ void __launch_bounds__(YCfg<N>::NTH, RG_MINB(YCfg<N>::NTH))
 // instead of nS (M nodes: two where the whole box lies between neighbouring nodes); ts_snapshot chooses
 // by cost.  At 128^3, 4 nodes and 40 sharp-k shells the X-ray part takes 0.53 ms by nodes, 0.61 by shells.
 
+// Nodes that one chunk of k_ts_nodes (a blockIdx.y) takes: all of them up to 4, else as even as 3 or 4
+// nodes a chunk go.
+constexpr int ts_node_chunk(int nm) {
+  return nm <= 2 ? 2 : (nm == 3 || nm == 5 || nm == 6 || nm == 9) ? 3 : 4;
+}
+constexpr int ts_node_chunks(int nm) { return (nm + ts_node_chunk(nm) - 1) / ts_node_chunk(nm); }
+// Coefficients a launch reads of each shell: those of whole chunks, so up to 2 nodes beyond nm (zeros)
+constexpr int ts_node_reads(int nm) { return 3 * ts_node_chunk(nm) * ts_node_chunks(nm); }
+constexpr int ts_node_most_reads() {
+  int most = 0;
+  for (int nm = 1; nm <= x_int_NXHII; ++nm) most = ts_node_reads(nm) > most ? ts_node_reads(nm) : most;
+  return most;
+}
+
 struct TsNodeShell {
   int nk;                    // sources of the shell
   int filtered, cut;         // as in TsBatch
   int ks[TS_MAXSRC];
   float cs[TS_MAXSRC];
-  float f[3 * x_int_NXHII];  // coefficient of field 3 j + kind, node m0 + j
+  float f[ts_node_most_reads()];   // coefficient of field 3 j + kind, node m0 + j; zero beyond the last node
 };
 
 // fields [f0, f0 + NF) of nf (f0 = blockIdx.y NF): work[f] = sum_r f_r W_r sum_i c_i spec[k_i][1].
@@ -1028,9 +1042,8 @@ static int launch_ts_nodes(rg_context* ctx, const cf* spec, cf* fields, size_t s
   int rc = twiddles_for(ctx, N, &tw);
   if (rc) return rc;
   const int nf = 3 * nm, log2n = __builtin_ctz(N);
-  // fields a thread accumulates: one chunk up to 4 nodes, else as even as 3 or 4 nodes a chunk go
-  const int per = nm <= 2 ? 2 : (nm == 3 || nm == 5 || nm == 6 || nm == 9) ? 3 : 4;
-  const dim3 grid((unsigned)std::min((stride + 255) / 256, (size_t)ctx->num_sms * 64), (nm + per - 1) / per);
+  const int per = ts_node_chunk(nm);
+  const dim3 grid((unsigned)std::min((stride + 255) / 256, (size_t)ctx->num_sms * 64), ts_node_chunks(nm));
   prof_begin(ctx, "ts_xray_nodes", st);
   if (per == 2)
     k_ts_nodes<6><<<grid, 256, 0, st>>>(spec, stride, gs, fields, d_sh, nS, nf, wtab, wpitch, log2n);
@@ -1130,6 +1143,60 @@ static int sharpk_cut(double delta_k, double R, int n2max) {
       lo = mid;
   }
   return lo;
+}
+
+// the cuts of the shells' windows: sharp-k, without the first shell, which is not filtered (ComputeTs.c:529)
+static std::vector<int> ts_cuts(const rg_params* p, const TsShells& sh, int n2max) {
+  std::vector<int> cut(sh.nS, TS_NOCUT);
+  if (p->TsHeatingFilterType == 1)
+    for (int r = 1; r < sh.nS; ++r) cut[r] = sharpk_cut(2.0 * M_PI / p->BoxSize, sh.R[r], n2max);
+  return cut;
+}
+
+// a shell combines more than TS_MAXSRC history snapshots
+static bool ts_wide(const TsShells& sh) {
+  for (int r = 0; r < sh.nS; ++r) {
+    int nk = 0;
+    for (int k = 0; k < sh.nsrc; ++k) nk += sh.coef[(size_t)r * sh.nsrc + k] != 0.f;
+    if (nk > TS_MAXSRC) return true;
+  }
+  return false;
+}
+
+// X-ray by nodes (m0 .. m0 + nm - 1, around the box's x_e, xe_lo to xe_hi, clamped as each cell's is) or
+// by shells (nm 0), whichever costs less.  In units of a z unit (two spectra): a node takes three fields
+// through k_ts_nodes and the x and y passes and 1.5 z units, 5.8 to 6.4 units measured at 128^3 to 512^3;
+// a pair of shells a z unit with the table look-ups, 1.15 to 1.5, and a pass over what its window
+// leaves, 0.42 a full one.  With 40 sharp-k shells the line lies between 4 and 6 nodes: 512^3 with 5
+// nodes 24.8 ms by nodes and 21.8 by shells, 256^3 with 9 4.2 and 2.9, 128^3 with 4 0.53 and 0.61.
+// A shell with its combination in a spare slot, which later batches overwrite, and a NaN in x_e
+// keep the shells.
+static void ts_choose_nodes(const float* X, int N, const std::vector<int>& cut, bool wide, float xe_lo, float xe_hi,
+                            int* m0, int* nm) {
+  *m0 = *nm = 0;
+  if (wide || std::isnan(xe_lo) || std::isnan(xe_hi)) return;
+  auto node = [&](float v) {
+    const double top = (double)X[x_int_NXHII - 1] * 0.999;
+    const double xc = (double)v > top ? top : (double)v < (double)X[0] ? 1.001 * (double)X[0] : (double)v;
+    return locate_xHII_index(X, (float)xc);
+  };
+  const int first = node(xe_lo), count = node(xe_hi) + 2 - first;
+  double passes = 0;
+  for (int c : cut) {
+    const double k = std::sqrt((double)c) / (N / 2);
+    passes += std::min(1.0, M_PI / 4 * k * k) + std::min(1.0, k);
+  }
+  if (6.0 * count >= 1.25 * (0.5 * cut.size()) + 0.42 * passes) return;
+  *m0 = first;
+  *nm = count;
+}
+
+void ts_debug_nodes(const rg_params* p, const TsShells& sh, const float* X, float xe_lo, float xe_hi, int* out) {
+  const int N = p->ReionGridDim;
+  ts_choose_nodes(X, N, ts_cuts(p, sh, 3 * (N / 2) * (N / 2)), ts_wide(sh), xe_lo, xe_hi, &out[0], &out[1]);
+  out[2] = out[1] ? ts_node_chunks(out[1]) : 0;
+  out[3] = out[1] ? ts_node_reads(out[1]) : 0;
+  out[4] = (int)(sizeof(TsNodeShell::f) / sizeof(float));
 }
 
 static double pow2_scale(double maxabs) {
@@ -1307,43 +1374,13 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
         }
     // a shell that combines more than TS_MAXSRC history snapshots gets its combination formed
     // beforehand (k_ts_combine) into one of TS_KB spare slots after the used sources
-    bool wide = false;
-    for (int r = 0; r < nS; ++r) {
-      int nk = 0;
-      for (int k = 0; k < sh.nsrc; ++k) nk += sh.coef[(size_t)r * sh.nsrc + k] != 0.f;
-      wide = wide || nk > TS_MAXSRC;
-    }
+    const bool wide = ts_wide(sh);
     const int nused = std::max(1, (int)used.size());
     // window cuts (filter() takes BoxSize in Mpc/h and R in Mpc, ComputeTs.c:532)
     const int n2max = 3 * (N / 2) * (N / 2);
     const bool sharp = p->TsHeatingFilterType == 1;
-    std::vector<int> cut(nS, TS_NOCUT);   // no filter on the first shell (ComputeTs.c:529)
-    if (sharp)
-      for (int r = 1; r < nS; ++r) cut[r] = sharpk_cut(2.0 * M_PI / p->BoxSize, sh.R[r], n2max);
-    // X-ray by nodes (m0 .. m0 + nm - 1, around the box's x_e clamped as each cell's is) or by shells,
-    // whichever costs less.  In units of a z unit (two spectra): a node takes three fields through
-    // k_ts_nodes and the x and y passes and 1.5 z units, 5.8 to 6.4 units measured at 128^3 to 512^3;
-    // a pair of shells a z unit with the table look-ups, 1.15 to 1.5, and a pass over what its window
-    // leaves, 0.42 a full one.  With 40 sharp-k shells the line lies between 4 and 6 nodes: 512^3 with 5
-    // nodes 24.8 ms by nodes and 21.8 by shells, 256^3 with 9 4.2 and 2.9, 128^3 with 4 0.53 and 0.61.
-    // A shell with its combination in a spare slot, which later batches overwrite, and a NaN in x_e
-    // keep the shells.
-    auto node = [&](float v) {
-      const float* X = ctx->tables.x_int_XHII.data();
-      const double top = (double)X[x_int_NXHII - 1] * 0.999;
-      const double xc = (double)v > top ? top : (double)v < (double)X[0] ? 1.001 * (double)X[0] : (double)v;
-      return locate_xHII_index(X, (float)xc);
-    };
-    if (!wide && !std::isnan(xe_lo) && !std::isnan(xe_hi)) {
-      zv.m0 = node(xe_lo);
-      zv.nm = node(xe_hi) + 2 - zv.m0;
-      double passes = 0;
-      for (int r = 0; r < nS; ++r) {
-        const double k = std::sqrt((double)cut[r]) / (N / 2);
-        passes += std::min(1.0, M_PI / 4 * k * k) + std::min(1.0, k);
-      }
-      if (6.0 * zv.nm >= 1.25 * (0.5 * nS) + 0.42 * passes) zv.nm = 0;
-    }
+    const std::vector<int> cut = ts_cuts(p, sh, n2max);
+    ts_choose_nodes(ctx->tables.x_int_XHII.data(), N, cut, wide, xe_lo, xe_hi, &zv.m0, &zv.nm);
     const int xs = zv.nm == 0;              // X-ray grids per shell
     const int Gs = 1 + xs + nagn;           // grids per shell
     const size_t slots = (size_t)nused + (wide ? TS_KB : 0);

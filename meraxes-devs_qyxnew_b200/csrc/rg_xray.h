@@ -74,6 +74,10 @@ int ts_tables(const rg_params* p, const Tables& t, const TsShells& sh, double zp
 // The Lyman-n sums of the shells with the kink correction (ComputeTs.c:900-1011).
 void ts_sum_lyn(const Tables& t, const rg_params* p, const TsShells& sh, double zp, std::vector<double>* sum_lyn);
 
+// How rg_compute_Ts takes the X-ray sums (rg_ts.cu): first node and nodes (0: by shells), chunks of
+// k_ts_nodes, coefficients it reads of a shell, coefficients a shell holds.
+void ts_debug_nodes(const rg_params* p, const TsShells& sh, const float* X, float xe_lo, float xe_hi, int* out);
+
 // Per-snapshot prefactors (ComputeTs.c:1014-1109)
 struct TsPrefactors {
   double growth_factor_zp, dgrowth_factor_dzp, dt_dzp, const_zp_prefactor_GAL, Luminosity_conversion_factor_GAL;

@@ -152,6 +152,7 @@ _SIGS = {
                                          C.c_void_p, C.c_void_p]),
     "rg_debug_ts_device_tables": (C.c_int, [C.c_void_p, _P(rg_params), _P(rg_snapshot), C.c_int, C.c_double,
                                             C.c_double, C.c_int, C.c_void_p]),
+    "rg_debug_ts_nodes": (C.c_int, [_P(rg_params), _P(rg_snapshot), C.c_int, C.c_float, C.c_float, _P(C.c_int)]),
     "rg_filter_roundtrip_noalloc": (C.c_int, [_P(rg_params), C.c_void_p, C.c_void_p, C.c_double, C.c_int,
                                               C.c_void_p, C.c_char_p, C.c_size_t]),
 }
@@ -243,6 +244,15 @@ def ts_agn_tables(p: rg_params, zz, snap: int, n_hist: int, x_e_ave: float, coll
     check(None, load().rg_debug_ts_agn_tables(C.byref(p), C.byref(s), n_hist, x_e_ave, collapse_fraction, ns,
                                               agn.ctypes.data, cz.ctypes.data))
     return agn, cz
+
+
+def ts_nodes(p: rg_params, zz, snap: int, n_hist: int, xe_lo: float, xe_hi: float):
+    """(first node, nodes, chunks, coefficients read, coefficients held) of ComputeTs' X-ray sums for a box
+    with x_e in [xe_lo, xe_hi]; no nodes: shell by shell (no device work)."""
+    out = (C.c_int * 5)()
+    s = snapshot(zz, snap)
+    check(None, load().rg_debug_ts_nodes(C.byref(p), C.byref(s), n_hist, xe_lo, xe_hi, out))
+    return tuple(out)
 
 
 def snapshot(zz, snap: int, stored_fcoll=None):
