@@ -86,6 +86,12 @@ std::vector<std::pair<double, bool>> radius_schedule(const rg_params* p, double 
   return out;
 }
 
+int upload(rg_context* ctx, void* dst, const void* src, size_t bytes, cudaStream_t st) {
+  RG_CUDA_TRY(ctx, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
+  RG_CUDA_TRY(ctx, cudaStreamSynchronize(st));
+  return RG_OK;
+}
+
 int twiddles_for(rg_context* ctx, int n, const cf** out) {
   for (auto& e : ctx->twiddles)
     if (e.first == n) {

@@ -365,6 +365,7 @@ __global__ void __launch_bounds__(FQ_BLOCK)
 
 // the electron tables on the device, uploaded once per table directory
 static int freq_tables_on_device(rg_context* ctx, XInt* t) {
+  int rc;
   const Tables& h = ctx->tables;
   const size_t per = (size_t)x_int_NXHII * x_int_NENERGY, total = x_int_NENERGY + x_int_NXHII + 5 * per;
   if (!ctx->freq_xint || ctx->freq_dir != h.dir) {
@@ -378,7 +379,8 @@ static int freq_tables_on_device(rg_context* ctx, XInt* t) {
          {&h.x_int_Energy, &h.x_int_XHII, &h.fheat, &h.n_Lya, &h.nion_HI, &h.nion_HeI, &h.nion_HeII})
       v.insert(v.end(), a->begin(), a->end());
     ctx->freq_dir.clear();
-    RG_CUDA_TRY(ctx, cudaMemcpy(ctx->freq_xint, v.data(), sizeof(float) * total, cudaMemcpyHostToDevice));
+    // on the stream of the kernels that read them, and there before v goes
+    if ((rc = upload(ctx, ctx->freq_xint, v.data(), sizeof(float) * total, ctx->side_stream))) return rc;
     ctx->freq_dir = h.dir;
   }
   const float* b = ctx->freq_xint;

@@ -79,6 +79,11 @@ int set_error(rg_context* ctx, int status, const std::string& msg);
       return ::rg::set_error((ctx), RG_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
+// Copy pageable host data to the device, ordered on `st`, and wait for it.  (A plain cudaMemcpy runs on the
+// legacy stream, which the context's non-blocking streams do not wait for, and may return while the copy from
+// its staging buffer is still under way.)
+int upload(rg_context* ctx, void* dst, const void* src, size_t bytes, cudaStream_t st);
+
 // A context buffer of at least `need` elements: kept when large enough, else freed and allocated
 // again (the old contents are not kept).
 template <typename T>
