@@ -105,7 +105,11 @@ int twiddles_for(rg_context* ctx, int n, const cf** out) {
   }
   cf* d = nullptr;
   RG_CUDA_TRY(ctx, cudaMalloc((void**)&d, sizeof(cf) * n));
-  RG_CUDA_TRY(ctx, cudaMemcpy(d, h.data(), sizeof(cf) * n, cudaMemcpyHostToDevice));
+  const int rc = upload(ctx, d, h.data(), sizeof(cf) * n, ctx->stream);
+  if (rc) {
+    cudaFree(d);
+    return rc;
+  }
   ctx->twiddles.emplace_back(n, d);
   *out = d;
   return RG_OK;
@@ -610,17 +614,17 @@ int rg_set_recombination_tables(rg_context* ctx, const double* lnGamma, int n_z,
     ctx->rec_knots = ctx->rec_y = ctx->rec_c = nullptr;
     return set_error(ctx, RG_ENOMEM, "cudaMalloc of the recombination tables failed");
   }
-  cudaError_t e = cudaMemcpy(ctx->rec_knots, lnGamma, sizeof(double) * n_gamma, cudaMemcpyHostToDevice);
-  for (int k = 0; k < 3 && e == cudaSuccess; ++k)
-    e = cudaMemcpy(ctx->rec_y + (size_t)k * per, tabs[k], sizeof(double) * per, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(ctx->rec_c, c.data(), sizeof(double) * 3 * per, cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) {
+  int rc = upload(ctx, ctx->rec_knots, lnGamma, sizeof(double) * n_gamma, ctx->stream);
+  for (int k = 0; k < 3 && !rc; ++k)
+    rc = upload(ctx, ctx->rec_y + (size_t)k * per, tabs[k], sizeof(double) * per, ctx->stream);
+  if (!rc) rc = upload(ctx, ctx->rec_c, c.data(), sizeof(double) * 3 * per, ctx->stream);
+  if (rc) {
     // no half-filled tables stay behind: find_HII_bubbles then asks for the tables again
     cudaFree(ctx->rec_knots);
     cudaFree(ctx->rec_y);
     cudaFree(ctx->rec_c);
     ctx->rec_knots = ctx->rec_y = ctx->rec_c = nullptr;
-    return set_error(ctx, RG_ECUDA, std::string("copying the recombination tables: ") + cudaGetErrorString(e));
+    return rc;
   }
   ctx->rec_nz = n_z;
   ctx->rec_nt = n_t;

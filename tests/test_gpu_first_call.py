@@ -31,3 +31,24 @@ def test_first_frequency_tables_equal_later_ones(x_e):
         ctx.close()
         assert np.any(first[0] > 0)
         assert np.array_equal(first, again)
+
+
+def roundtrip(ctx, n, d_in, d_out):
+    p = rg.make_params(n, float(n))
+    ctx.call("rg_debug_filter_roundtrip", C.byref(p), d_in.data_ptr(), d_out.data_ptr(), 3.0, 0)
+    return d_out.clone()
+
+
+@pytest.mark.parametrize("n", [8, 96, 128])
+def test_first_transform_equals_later_ones(n):
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    d_in = torch.randn(n * n * (n + 2), generator=gen, device="cuda")
+    d_out = torch.zeros_like(d_in)
+    torch.cuda.synchronize()
+    for _ in range(8):
+        ctx = rg.Context(n)
+        first = roundtrip(ctx, n, d_in, d_out)
+        again = roundtrip(ctx, n, d_in, d_out)
+        ctx.close()
+        assert torch.equal(first, again)
