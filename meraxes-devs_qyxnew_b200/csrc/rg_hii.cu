@@ -232,7 +232,13 @@ struct HiiZ {
 // Grids in rt: 0 deltax, 1 stars, then x_e (spin temperature), then effective_bhm (BH), then
 // starsIII (Pop III), then with recombinations N_rec, weighted_sfr, effective_bhar (BH) and
 // weighted_sfrIII (Pop III); bt.ng of them.
-template <int N>
+//
+// NG: the number of grids (2 to 4) without recombinations or Pop III, so that the loop over them and the
+// test compile without the other grids' branches; 0: any count, from bt.  FINAL: the batch ends with the
+// snapshot's last radius (as in k_hii_zr).  With both known only at run time the pass of a small box took
+// about twice as long: 24^3, 34 radii of 2 grids, 483 us against 209; 48^3, 41 radii, 770 against 375;
+// 128^3 with Pop III sources 1.90 ms a call against 1.84.
+template <int N, int NG, bool FINAL>
 __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::QZ, (HiiZ<N>::MINB))
     k_hii_z(const cf* __restrict__ work, size_t stride, const cf* __restrict__ g_tw, HiiBatch bt, HiiBatchIII b3,
             HiiConst c, HiiState s) {
@@ -249,7 +255,8 @@ __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::QZ, (HiiZ<N>::MINB))
   // ZB shared tiles (with two, grid u + 1 is copied while grid u is transformed); the tile of
   // unit u is the exchange buffer of its transform
   // (after the row buffers of the grids there are)
-  cf* tiles = reinterpret_cast<cf*>(rt + round_up(bt.ng * ROWS * RP, 4));
+  const int ng = NG ? NG : bt.ng;
+  cf* tiles = reinterpret_cast<cf*>(rt + round_up(ng * ROWS * RP, 4));
   const int x = blockIdx.y, y0 = blockIdx.x * ROWS;
   load_twiddles<N>(s_tw, g_tw);
 
@@ -276,8 +283,7 @@ __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::QZ, (HiiZ<N>::MINB))
     A[w] = a;
     I[w] = iv;
   }
-  const int ng = bt.ng;
-  const bool rec = c.rec, mini = c.mini;
+  const bool rec = NG == 0 && c.rec, mini = NG == 0 && c.mini;
   int gi = 2;
   const int gx = c.spin ? gi++ : -1;
   const int gb = c.bh ? gi++ : -1;
@@ -319,7 +325,7 @@ __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::QZ, (HiiZ<N>::MINB))
         cp_async_commit();
       }
     }
-    const bool last = bt.last && r == bt.nr - 1;
+    const bool last = FINAL && r == bt.nr - 1;
     const double pref = bt.fcoll_pref[r];
 #pragma unroll
     for (int w = 0; w < W; ++w) {
@@ -419,7 +425,7 @@ __global__ void __launch_bounds__(Cfg<N>::T* Cfg<N>::QZ, (HiiZ<N>::MINB))
     }
   }
 
-  if (!bt.last) {
+  if constexpr (!FINAL) {
 #pragma unroll
     for (int w = 0; w < W; ++w) {
       const int nb = IT - 32 * w < 32 ? IT - 32 * w : 32;
@@ -595,7 +601,7 @@ constexpr int hii_ngx() {
   return ng;
 }
 
-template <int N>
+template <int N, int NG>
 int launch_hii_zrow(rg_context* ctx, const cf* work, size_t stride, const HiiZUnit& u, const HiiBatchIII& b3,
                     cudaStream_t st) {
   const cf* tw;
@@ -603,20 +609,22 @@ int launch_hii_zrow(rg_context* ctx, const cf* work, size_t stride, const HiiZUn
   if (rc) return rc;
   using C = Cfg<N>;
   const HiiBatch& bt = u.bt;
-  if (bt.ng > hii_ngx<N>())
+  constexpr int NGX = NG ? NG : hii_ngx<N>();
+  if (bt.ng > NGX)
     return set_error(ctx, RG_EUNSUPPORTED,
                      "this combination of grids (recombinations, Pop III, BH feedback, spin temperature) needs "
                      "more row buffers than one z pass holds at this ReionGridDim");
-  static_assert(HiiZ<N>::smem(hii_ngx<N>()) <= 227 * 1024, "z pass shared memory above the per-block limit");
+  static_assert(HiiZ<N>::smem(NGX) <= 227 * 1024, "z pass shared memory above the per-block limit");
   // the shared memory of the grids there are, not of the maximum
   const size_t sm = HiiZ<N>::smem(bt.ng);
-  RG_CUDA_TRY(ctx, prep(k_hii_z<N>, HiiZ<N>::smem(hii_ngx<N>())));
+  auto kern = bt.last ? k_hii_z<N, NG, true> : k_hii_z<N, NG, false>;
+  RG_CUDA_TRY(ctx, prep(kern, HiiZ<N>::smem(NGX)));
   const dim3 grid(N / (2 * C::QZ), N);
   // algorithmic bytes: the Hermitian halves of the grids per radius, z_at_ionization on the
   // first batch, xH at the end
   const double n3 = (double)N * N * N, nzc = (double)C::NZ * N * N;
   prof_begin(ctx, bt.last ? "inv_z_c2r_test_final" : "inv_z_c2r_test", st);
-  k_hii_z<N><<<grid, C::T * C::QZ, sm, st>>>(work, stride, tw, bt, b3, u.c, u.s);
+  kern<<<grid, C::T * C::QZ, sm, st>>>(work, stride, tw, bt, b3, u.c, u.s);
   prof_end(ctx, bt.nr * bt.ng * 8.0 * nzc + (bt.first || bt.last ? 4.0 * n3 : 2.0 * n3), st);
   RG_CUDA_TRY(ctx, cudaGetLastError());
   return RG_OK;
@@ -627,12 +635,24 @@ int launch_hii_zrow(rg_context* ctx, const cf* work, size_t stride, const HiiZUn
 template <int N>
 int launch_hii_z(rg_context* ctx, const cf* work, size_t stride, int ng, int nu, const HiiZUnits& us,
                  const HiiBatchIII& b3, cudaStream_t st) {
+  const HiiConst& c = us.u[0].c;
+  auto row = [&](auto ngc, int k) {
+    return launch_hii_zrow<N, decltype(ngc)::value>(ctx, work + (size_t)k * us.u[k].bt.nr * ng * stride, stride,
+                                                    us.u[k], b3, st);
+  };
   if constexpr (HiiZR<N>::USED) {
-    if (!us.u[0].c.mini) return launch_hii_zr<N>(ctx, work, nu, us, st);
+    if (!c.mini) return launch_hii_zr<N>(ctx, work, nu, us, st);
   }
   for (int k = 0; k < nu; ++k) {
-    const int rc =
-        launch_hii_zrow<N>(ctx, work + (size_t)k * us.u[k].bt.nr * ng * stride, stride, us.u[k], b3, st);
+    int rc;
+    if constexpr (HiiZR<N>::USED) {
+      rc = row(std::integral_constant<int, 0>{}, k);
+    } else {
+      rc = c.mini || c.rec ? row(std::integral_constant<int, 0>{}, k)
+           : ng == 2       ? row(std::integral_constant<int, 2>{}, k)
+           : ng == 3       ? row(std::integral_constant<int, 3>{}, k)
+                           : row(std::integral_constant<int, 4>{}, k);
+    }
     if (rc) return rc;
   }
   return RG_OK;
