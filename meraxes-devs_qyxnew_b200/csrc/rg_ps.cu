@@ -98,13 +98,22 @@ __device__ __forceinline__ float ps_kmag(int nx, int ny, int nz, int n, float dk
 }
 
 // per-block sums [3][nb]: k^3 |d|^2 norm, k, count over the Hermitian modes S[kz][x][y].  A thread
-// walks x at its own (kz, y), a block taking PS_XC values of x and PS_NT columns (kz, y) at a time: its
+// walks x at its own (kz, y), a block taking xc values of x and PS_NT columns (kz, y) at a time: its
 // bin changes a few times in a walk, so it sums in registers and adds to the block's shared sums when
 // the bin changes (an FP64 add in shared memory is a compare-and-swap loop; one per mode or warp took
 // 0.34 ms at 256^3, now 0.09).
-constexpr int PS_XC = 64;
+constexpr int PS_XC = 64;   // the longest walk
 
-__global__ void __launch_bounds__(PS_NT) k_ps_bins(const cf* __restrict__ spec, int n, const PsBins b,
+// The longest walk that still gives two blocks an SM.  us with walks of 64 and by this rule: 16^3 38, 16;
+// 64^3 85, 28; 96^3 89, 31; 128^3 80, 35; 192^3 81, 56 (walks of 2 at 256^3: 352 against 87).
+static int ps_walk(int n, int num_sms) {
+  const int groups = ((n / 2 + 1) * n + PS_NT - 1) / PS_NT;
+  int xc = PS_XC;
+  while (xc > 2 && groups * ((n + xc - 1) / xc) < 2 * num_sms) xc /= 2;
+  return xc;
+}
+
+__global__ void __launch_bounds__(PS_NT) k_ps_bins(const cf* __restrict__ spec, int n, int xc, const PsBins b,
                                                    double* __restrict__ partials) {
   __shared__ double sums[3][PS_MAXBINS];
   __shared__ float ceil_s[PS_MAXBINS];
@@ -115,12 +124,12 @@ __global__ void __launch_bounds__(PS_NT) k_ps_bins(const cf* __restrict__ spec, 
   __syncthreads();
   const int nb = max(b.nb, 1);
   const size_t cols = (size_t)(n / 2 + 1) * n;   // (kz, y), y fastest
-  const size_t groups = (cols + PS_NT - 1) / PS_NT, chunks = (n + PS_XC - 1) / PS_XC;
+  const size_t groups = (cols + PS_NT - 1) / PS_NT, chunks = (n + xc - 1) / xc;
   for (size_t w = blockIdx.x; w < groups * chunks; w += gridDim.x) {
     const size_t col = w / chunks * PS_NT + threadIdx.x;
     if (col >= cols) continue;
     const int y = (int)(col % n), kz = (int)(col / n);
-    const int x0 = (int)(w % chunks) * PS_XC, x1 = min(n, x0 + PS_XC);
+    const int x0 = (int)(w % chunks) * xc, x1 = min(n, x0 + xc);
     int bin = -1;
     double pw = 0.0, kk = 0.0;
     int cnt = 0;
@@ -195,7 +204,7 @@ static int power_spectrum(rg_context* ctx, const rg_params* p, const float* d_dT
   const float* src = ctx->ps_pad;
   if ((rc = fft_forward(ctx, N, &src, 1, ctx->spec, nc, 1.0, st))) return rc;
   prof_begin(ctx, "ps_bins", st);
-  k_ps_bins<<<nblk, PS_NT, 0, st>>>(ctx->spec, N, b, partials);
+  k_ps_bins<<<nblk, PS_NT, 0, st>>>(ctx->spec, N, ps_walk(N, ctx->num_sms), b, partials);
   prof_end(ctx, 8.0 * nc, st);
   RG_CUDA_TRY(ctx, cudaGetLastError());
   std::vector<double> h((size_t)nblk * 3 * PS_MAXBINS);
