@@ -242,7 +242,7 @@ struct rg_context {
   int rec_nz = 0, rec_nt = 0, rec_ng = 0;
   double* partials = nullptr;
   size_t partials_elems = 0;
-  double* d_sums = nullptr;      // reduced sums
+  double* d_sums = nullptr;      // reduced sums [64]; ComputeTs' status words at [48]
   double* h_sums = nullptr;      // pinned host copy [64]; [63] the error word of the device waits
   std::vector<char> ts_host;     // ComputeTs: coefficients on their way to the device
   double* batch_sums = nullptr;  // rg_find_HII_bubbles_batch: reduced sums per snapshot [unit][32]

@@ -196,11 +196,23 @@ static float float_of_order(unsigned o) {
   return v;
 }
 
+// What a snapshot's kernels report next to their sums, all zero before the first of them: one memset and no
+// copy of its own (it lies behind the sums, d_sums[TS_STATUS]).  As three words set and fetched each by
+// itself a homogeneous call took 119 us at 64^3; so it takes 110.
+struct TsStatus {
+  unsigned xe_top;       // the largest x_e in float_order
+  unsigned xe_bottom;    // the smallest, complemented
+  int nonconv;           // cells whose get_Ts ran out of iterations
+  int pad;
+};
+constexpr int TS_STATUS = 48;
+static_assert(sizeof(TsStatus) == 2 * sizeof(double), "two slots of the sums");
+
 // collapse fraction, <x_e> and the range of x_e over the box (ComputeTs.c:585-677)
 __global__ void __launch_bounds__(256) k_ts_reduce0(const float* __restrict__ stars, const float* __restrict__ deltax,
                                                     const float* __restrict__ xe, int n, double Mh2,
                                                     double fourthirds_pi_R3_over_pv, double* partials,
-                                                    unsigned* __restrict__ xe_range) {
+                                                    TsStatus* __restrict__ status) {
   constexpr int U = 4;   // cells of a thread whose loads are in flight together
   const size_t n3 = (size_t)n * n * n, step = (size_t)gridDim.x * 256;
   const double f = fourthirds_pi_R3_over_pv / Mh2;
@@ -230,24 +242,21 @@ __global__ void __launch_bounds__(256) k_ts_reduce0(const float* __restrict__ st
     }
   }
   // the range of x_e as ordered integers; a NaN, which the minimum and maximum pass over, is its top
-  unsigned lo = float_order(mn), hi = nan ? ~0u : float_order(mx);
+  unsigned bottom = ~float_order(mn), top = nan ? ~0u : float_order(mx);
   block_sum_dyn<2>(acc, partials + (size_t)blockIdx.x * 2);
-  __shared__ unsigned s_lo, s_hi;
-  if (threadIdx.x == 0) {
-    s_lo = ~0u;
-    s_hi = 0u;
-  }
+  __shared__ unsigned s_bottom, s_top;
+  if (threadIdx.x == 0) s_bottom = s_top = 0u;
   __syncthreads();
-  lo = __reduce_min_sync(0xffffffffu, lo);
-  hi = __reduce_max_sync(0xffffffffu, hi);
+  bottom = __reduce_max_sync(0xffffffffu, bottom);
+  top = __reduce_max_sync(0xffffffffu, top);
   if ((threadIdx.x & 31) == 0) {
-    atomicMin(&s_lo, lo);
-    atomicMax(&s_hi, hi);
+    atomicMax(&s_bottom, bottom);
+    atomicMax(&s_top, top);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    atomicMin(xe_range, s_lo);
-    atomicMax(xe_range + 1, s_hi);
+    atomicMax(&status->xe_bottom, s_bottom);
+    atomicMax(&status->xe_top, s_top);
   }
 }
 
@@ -1259,22 +1268,26 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
     Z.f_H = cm.f_H;
     Z.f_He = cm.f_He;
   }
-  // device constants, the non-convergence counter, the range of x_e and the per-shell coefficients
-  // live in one context buffer: [TsDev][int, x_e range][TsShellCoef x shells][TsNodeShell x shells]
+  // device constants and the per-shell coefficients live in one context buffer:
+  // [TsDev][TsShellCoef x shells][TsNodeShell x shells]
   const int nS_all = p->TsNumFilterSteps;
-  const size_t off_co = (sizeof(TsDev) + 16 + 255) / 256 * 256;
+  const size_t off_co = (sizeof(TsDev) + 255) / 256 * 256;
   if ((rc = ensure_device(ctx, &ctx->ts_const, &ctx->ts_const_elems,
                           off_co + (sizeof(TsShellCoef) + sizeof(TsNodeShell)) * (nS_all + 1))))
     return rc;
   TsDev* d_hc = reinterpret_cast<TsDev*>(ctx->ts_const);
-  int* d_nonconv = reinterpret_cast<int*>(ctx->ts_const + sizeof(TsDev));
+  TsStatus* d_status = reinterpret_cast<TsStatus*>(ctx->d_sums + TS_STATUS);
   TsShellCoef* d_co = reinterpret_cast<TsShellCoef*>(ctx->ts_const + off_co);
   RG_CUDA_TRY(ctx, cudaMemcpyAsync(d_hc, &hc, sizeof(TsDev), cudaMemcpyHostToDevice, st));
   TsNodeShell* d_node = reinterpret_cast<TsNodeShell*>(d_co + nS_all + 1);
-  unsigned* d_range = reinterpret_cast<unsigned*>(d_nonconv + 1);
-  RG_CUDA_TRY(ctx, cudaMemsetAsync(d_nonconv, 0, sizeof(int), st));
-  RG_CUDA_TRY(ctx, cudaMemsetAsync(d_range, 0xff, sizeof(unsigned), st));
-  RG_CUDA_TRY(ctx, cudaMemsetAsync(d_range + 1, 0, sizeof(unsigned), st));
+  RG_CUDA_TRY(ctx, cudaMemsetAsync(d_status, 0, sizeof(TsStatus), st));
+  // the sums and the status behind them, in one copy
+  TsStatus status;
+  auto fetch = [&]() -> int {
+    RG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_sums, ctx->d_sums, sizeof(double) * TS_STATUS + sizeof(TsStatus),
+                                     cudaMemcpyDeviceToHost, st));
+    return RG_OK;
+  };
   const int nblk = 148 * 8;
   double* partials = ensure_partials(ctx, (size_t)nblk * TS_NSUM);
   if (!partials) return set_error(ctx, RG_ENOMEM, "partials");
@@ -1287,14 +1300,12 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
   auto finish = [&](bool homog, int nblocks) -> int {
     if ((rc = kick())) return rc;
     if ((rc = reduce_partials(ctx, partials, nblocks, TS_NSUM, ctx->d_sums, st))) return rc;
-    RG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_sums, ctx->d_sums, sizeof(double) * TS_NSUM, cudaMemcpyDeviceToHost, st));
-    RG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_sums + 62, d_nonconv, sizeof(int), cudaMemcpyDeviceToHost, st));
+    if ((rc = fetch())) return rc;
     if (waits && (rc = xy_ctrl_fetch(ctx, st))) return rc;
     RG_CUDA_TRY(ctx, cudaStreamSynchronize(st));
     prof_resolve(ctx);
     if (waits && (rc = xy_ctrl_result(ctx))) return rc;
-    int nonconv;
-    std::memcpy(&nonconv, ctx->h_sums + 62, sizeof(nonconv));
+    std::memcpy(&status, ctx->h_sums + TS_STATUS, sizeof(status));
     const double* S = ctx->h_sums;
     const double nn = (double)n3;
     if (!homog) {
@@ -1309,7 +1320,7 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
     out->volume_ave_TK = S[5] / nn;
     out->volume_ave_xe = S[6] / nn;
     out->homogeneous = homog;
-    if (nonconv)
+    if (status.nonconv)
       return set_error(ctx, RG_ETIMEDOUT, "get_Ts did not converge in " + std::to_string(ctx->ts_iter_limit) +
                                               " iterations for some cells");
     return RG_OK;
@@ -1318,18 +1329,16 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
   // collapse fraction and <x_e> (both branches compute the collapse fraction)
   prof_begin(ctx, "ts_reduce0", st);
   if ((rc = stage_wait(ctx, stg->inputs, st))) return rc;
-  k_ts_reduce0<<<nblk, 256, 0, st>>>(g->stars, g->deltax, g->x_e_box_prev, N, Mh2, ftpr3, partials, d_range);
+  k_ts_reduce0<<<nblk, 256, 0, st>>>(g->stars, g->deltax, g->x_e_box_prev, N, Mh2, ftpr3, partials, d_status);
   prof_end(ctx, 12.0 * n3, st);
   RG_CUDA_TRY(ctx, cudaGetLastError());
   if ((rc = reduce_partials(ctx, partials, nblk, 2, ctx->d_sums, st))) return rc;
-  RG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_sums, ctx->d_sums, sizeof(double) * 2, cudaMemcpyDeviceToHost, st));
-  RG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_sums + 2, d_range, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+  if ((rc = fetch())) return rc;
   RG_CUDA_TRY(ctx, cudaStreamSynchronize(st));
   const double collapse_fraction = ctx->h_sums[0] / (double)n3;
   const double x_e_ave = ctx->h_sums[1] / (double)n3;
-  unsigned range[2];
-  std::memcpy(range, ctx->h_sums + 2, sizeof(range));
-  const float xe_lo = float_of_order(range[0]), xe_hi = float_of_order(range[1]);
+  std::memcpy(&status, ctx->h_sums + TS_STATUS, sizeof(status));
+  const float xe_lo = float_of_order(~status.xe_bottom), xe_hi = float_of_order(status.xe_top);
   out->collapse_fraction = collapse_fraction;
   out->x_e_ave = x_e_ave;
 
@@ -1339,7 +1348,7 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
     prof_begin(ctx, "ts_homog", st);
     if ((rc = stage_wait(ctx, stg->closing, st))) return rc;   // Tk_box is overwritten
     k_ts_homog<<<nblk, 256, 0, st>>>(d_hc, par, xe0, TK0, cT_approx((float)zp), N, g->deltax, g->x_e_box_prev,
-                                      g->x_e_box, g->Tk_box, g->TS_box, partials, d_nonconv);
+                                      g->x_e_box, g->Tk_box, g->TS_box, partials, &d_status->nonconv);
     prof_end(ctx, 28.0 * n3, st);
     RG_CUDA_TRY(ctx, cudaGetLastError());
     return finish(true, nblk);
@@ -1622,7 +1631,7 @@ int ts_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const
   if ((rc = stage_wait(ctx, stg->closing, st))) return rc;
   k_ts_evolve<<<nblk, EV_NT, 0, st>>>(d_hc, par, e, inv, N, no_light ? nullptr : ctx->ts_sums,
                                      (no_light || !nagn) ? nullptr : ctx->ts_agn, g->deltax, g->x_e_box_prev,
-                                     g->x_e_box, g->Tk_box, g->TS_box, partials, d_nonconv,
+                                     g->x_e_box, g->Tk_box, g->TS_box, partials, &d_status->nonconv,
                                      no_light ? nullptr : ctx->xy_ctrl);
   prof_end(ctx, (double)n3 * (16 + 4 + 4 + 4 + 4 + 4 + 4 + 4), st);
   RG_CUDA_TRY(ctx, cudaGetLastError());
