@@ -297,7 +297,8 @@ int rg_smooth_grid(rg_context* ctx, double box_size, int reion_grid_dim, const f
    adds d_values[p * n_gal + g] to grid p at the cell pos_to_ngp (src/core/misc_tools.c:207-217)
    gives; each grid is then clamped at zero, divided by divisors[p] (a host array, or null for
    none; the sfr grid's SFR timescale) and left in the padded layout.  The grids are overwritten
-   (device pointers, n_prop <= 8).  Which galaxy property goes to which grid, the black-hole mass
+   (device pointers, n_prop <= 8); one given for several properties collects all of them and is
+   clamped and divided once for each, in their order.  Which galaxy property goes to which grid, the black-hole mass
    limit and the history shift stay with the caller.  A position below the box returns RG_EINVAL
    (the reference asserts). */
 int rg_deposit_ngp(rg_context* ctx, double box_size, int n_gal, const float* d_pos, int n_prop,

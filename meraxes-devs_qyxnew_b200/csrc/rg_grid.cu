@@ -77,13 +77,13 @@ struct NgpDiv {
   double d[MAXG];
 };
 
-// clamp at zero and divide the cells of grid blockIdx.y (the padding holds zeros).  A grid whose values
+// clamp at zero and divide the cells of grid p0 + blockIdx.y (the padding holds zeros).  A grid whose values
 // were all at least zero and whose divisor is 1 is final as it is: with the pass over it left out, and
 // the others' in runs of 4, four grids of a 128^3 box and 10^6 galaxies took 82 us
 // a call (145 before).
-__global__ void __launch_bounds__(NGP_NT) k_ngp_finish(GridPtrsW grids, size_t npad, NgpDiv div,
+__global__ void __launch_bounds__(NGP_NT) k_ngp_finish(GridPtrsW grids, int p0, size_t npad, NgpDiv div,
                                                        const int* __restrict__ ctrl) {
-  const int p = blockIdx.y;
+  const int p = p0 + blockIdx.y;
   double dv = div.d[0];
 #pragma unroll
   for (int i = 1; i < MAXG; ++i)
@@ -147,10 +147,17 @@ int rg_deposit_ngp(rg_context* ctx, double box_size, int n_gal, const float* d_p
     prof_end(ctx, (double)n_gal * (12.0 + 8.0 * n_prop), st);
     RG_CUDA_TRY(ctx, cudaGetLastError());
   }
+  // properties that share a grid finish it one after the other, in their order
+  bool shared = false;
+  for (int p = 0; p < n_prop; ++p)
+    for (int q = 0; q < p; ++q) shared = shared || gp.p[p] == gp.p[q];
+  const int per = shared ? 1 : n_prop;
   prof_begin(ctx, "ngp_finish", st);
-  k_ngp_finish<<<dim3(nblk, n_prop), NGP_NT, 0, st>>>(gp, npad, dv, ctx->ngp_bad);
+  for (int p = 0; p < n_prop; p += per) {
+    k_ngp_finish<<<dim3(nblk, per), NGP_NT, 0, st>>>(gp, p, npad, dv, ctx->ngp_bad);
+    RG_CUDA_TRY(ctx, cudaGetLastError());
+  }
   prof_end(ctx, 8.0 * n_prop * (double)n * n * n, st);
-  RG_CUDA_TRY(ctx, cudaGetLastError());
   int bad = 0;
   RG_CUDA_TRY(ctx, cudaMemcpyAsync(&bad, ctx->ngp_bad, sizeof(int), cudaMemcpyDeviceToHost, st));
   RG_CUDA_TRY(ctx, cudaStreamSynchronize(st));
