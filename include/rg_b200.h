@@ -194,7 +194,9 @@ int rg_destroy(rg_context* ctx);
 int rg_set_mode(rg_context* ctx, int mode);
 /* Radii per batch of the fused mode's x/y and z passes: 0 = the default, 16 where the windowed
    spectra of a batch take at most 6 GB, else 8; larger values are cut to 16 (the tuner in
-   autotune.py picks one per workload shape). */
+   autotune.py picks one per workload shape).  Where the device has no room for a batch's buffers the
+   radii go in smaller ones, with the same results; the size that fitted is kept until the next
+   rg_set_radius_batch. */
 int rg_set_radius_batch(rg_context* ctx, int radii_per_batch);
 /* cudaStream_t to launch on (NULL = the context's own stream). */
 int rg_set_stream(rg_context* ctx, void* stream);

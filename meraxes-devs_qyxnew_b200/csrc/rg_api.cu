@@ -186,7 +186,10 @@ double* ensure_partials(rg_context* ctx, size_t n) {
   if (ctx->partials) cudaFree(ctx->partials);
   ctx->partials = nullptr;
   ctx->partials_elems = 0;
-  if (cudaMalloc((void**)&ctx->partials, sizeof(double) * n) != cudaSuccess) return nullptr;
+  if (cudaMalloc((void**)&ctx->partials, sizeof(double) * n) != cudaSuccess) {
+    cudaGetLastError();   // reported by the caller: the next launch's check is not to find it
+    return ctx->partials = nullptr;
+  }
   ctx->partials_elems = n;
   return ctx->partials;
 }
@@ -395,6 +398,7 @@ int rg_set_mode(rg_context* ctx, int mode) {
 int rg_set_radius_batch(rg_context* ctx, int k) {
   if (!ctx || k < 0 || k > 64) return RG_EINVAL;
   ctx->radius_batch = k;
+  ctx->hii_fit = ~(size_t)0;
   return RG_OK;
 }
 

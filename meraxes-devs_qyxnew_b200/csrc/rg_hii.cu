@@ -917,21 +917,10 @@ static int hii_close_blocks(const rg_context* ctx, int n) {
 
 // radii per batch of the fused mode: the caller's, or 16 where their windowed spectra take at most 6 GB
 // and 8 above (fewer launches and less state between batches: 0.34 -> 0.31 ms at 64^3, 4.74 -> 4.53 at
-// 192^3, no gain at 512^3)
+// 192^3, no gain at 512^3), and no more than the device has had room for (hii_buffers)
 static int radius_batch(const rg_context* ctx, size_t nc, int ng, int nr) {
-  int kb = ctx->radius_batch > 0 ? ctx->radius_batch : nc * ng * 16 * sizeof(cf) <= ((size_t)6 << 30) ? 16 : 8;
-  return std::max(1, std::min({kb, KB_MAX, nr}));
-}
-
-// the work buffer of kb radii; *kb is halved down to 8 where the device has no room for the default 16
-static int ensure_work(rg_context* ctx, size_t nc, int ng, int* kb) {
-  int rc = ensure_device(ctx, &ctx->work, &ctx->work_elems, nc * ng * *kb);
-  if (rc == RG_ENOMEM && ctx->radius_batch == 0 && *kb > 8) {
-    cudaGetLastError();   // the failed allocation is dealt with
-    *kb = 8;
-    rc = ensure_device(ctx, &ctx->work, &ctx->work_elems, nc * ng * *kb);
-  }
-  return rc;
+  const int kb = ctx->radius_batch > 0 ? ctx->radius_batch : nc * ng * 16 * sizeof(cf) <= ((size_t)6 << 30) ? 16 : 8;
+  return std::max(1, std::min({kb, KB_MAX, nr, (int)std::min(ctx->hii_fit / (nc * ng), (size_t)KB_MAX)}));
 }
 
 // radii whose window planes are formed at a time: whole batches, at most 256 MB where that is more
@@ -939,6 +928,51 @@ static int ensure_work(rg_context* ctx, size_t nc, int ng, int* kb) {
 static int plane_radii(int n, int kb, int nr) {
   const int fit = (int)((256u << 20) / (sizeof(float) * wplane_size(n))) / kb * kb;
   return std::min(nr, std::max(kb, fit));
+}
+
+// Every buffer of the radius loop over nr radii of nu snapshots (ng grids in all), before the first launch:
+// *kb radii a batch, *npl window planes at a time (none for sharp-k).  A batch's spectra and planes grow with
+// the batch, so where the device has no room for all of it the two are given back and half the radii are tried:
+// the default batch and its planes then need no more than 8 radii without planes did.  A batch that the
+// caller set and whose spectra alone do not fit is RG_ENOMEM.  The context remembers what fitted, so that
+// later calls do not allocate and free again.
+static int hii_buffers(rg_context* ctx, size_t nc, int ng, int nr, int nu, bool planes, size_t npart, int* kb,
+                       int* npl) {
+  const int N = ctx->N, n2max = 3 * (N / 2) * (N / 2);
+  const size_t n3 = (size_t)N * N * N;
+  auto all = [&]() -> int {
+    int rc = ensure_device(ctx, &ctx->work, &ctx->work_elems, nc * ng * *kb);
+    if (!rc) rc = ensure_device(ctx, &ctx->wplanes, &ctx->wplanes_elems, planes ? *npl * wplane_size(N) : 1);
+    if (!rc) rc = ensure_device(ctx, &ctx->spec, &ctx->spec_elems, nc * ng);
+    // one state byte per cell between radius batches (in words of four)
+    if (!rc) rc = ensure_device(ctx, &ctx->bits, &ctx->bits_elems, (n3 * nu + 3) / 4);
+    if (!rc) rc = ensure_device(ctx, &ctx->d_radii, &ctx->d_radii_elems, (size_t)nr);
+    if (!rc) rc = ensure_device(ctx, &ctx->wtab, &ctx->wtab_elems, (size_t)nr * (n2max + 1));
+    if (!rc) rc = ensure_device(ctx, &ctx->wcut, &ctx->wcut_elems, (size_t)nr);
+    if (!rc) rc = ensure_device(ctx, &ctx->xy_ctrl, &ctx->xy_ctrl_elems, (size_t)(N / 2 + 1) * *kb + 2);
+    if (!rc && !ensure_partials(ctx, npart)) rc = set_error(ctx, RG_ENOMEM, "partials");
+    return rc;
+  };
+  auto release = [](auto** ptr, size_t* elems) {
+    if (*ptr) cudaFree(*ptr);
+    *ptr = nullptr;
+    *elems = 0;
+  };
+  int rc;
+  if (ctx->radius_batch > 0 && (rc = ensure_device(ctx, &ctx->work, &ctx->work_elems, nc * ng * *kb))) return rc;
+  for (;;) {
+    *npl = plane_radii(N, *kb, nr);
+    rc = all();
+    if (rc == RG_ENOMEM && planes && *npl > *kb) {
+      *npl = *kb;
+      rc = all();
+    }
+    if (rc != RG_ENOMEM || *kb == 1) return rc;
+    release(&ctx->work, &ctx->work_elems);
+    release(&ctx->wplanes, &ctx->wplanes_elems);
+    *kb /= 2;
+    ctx->hii_fit = nc * ng * *kb;
+  }
 }
 
 int hii_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, const rg_grids* g, rg_hii_scalars* out,
@@ -962,10 +996,12 @@ int hii_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, cons
   auto sched = radius_schedule(p, redshift);
   const int nr = (int)sched.size();
   int kb = plain ? 1 : radius_batch(ctx, nc, ng, nr);
-  if ((rc = ensure_device(ctx, &ctx->spec, &ctx->spec_elems, nc * ng))) return rc;
-  if ((rc = ensure_work(ctx, nc, ng, &kb))) return rc;
-  // one state byte per cell between radius batches (in words of four)
-  if ((rc = ensure_device(ctx, &ctx->bits, &ctx->bits_elems, ((size_t)N * N * N + 3) / 4))) return rc;
+  const int cb = hii_close_blocks(ctx, N);
+  int npl = 0;
+  if ((rc = hii_buffers(ctx, nc, ng, nr, 1, p->ReionFilterType != 1,
+                        std::max((size_t)cb * HII_NSUM, (size_t)4 * ctx->num_sms * REC_NSUM), &kb, &npl)))
+    return rc;
+  double* partials = ctx->partials;
   if ((rc = stage_wait(ctx, stg->inputs, st))) return rc;
   const int fg = fft_forward_group(N);   // grids per forward launch
   for (int g0 = 0; g0 < ng; g0 += fg)
@@ -976,8 +1012,6 @@ int hii_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, cons
   if ((rc = hii_windows(ctx, p, sched, st))) return rc;
   const int n2max = 3 * (N / 2) * (N / 2);
   const int* wcut = p->ReionFilterType == 1 ? ctx->wcut : nullptr;
-  const int npl = plane_radii(N, kb, nr);
-  if ((rc = ensure_device(ctx, &ctx->wplanes, &ctx->wplanes_elems, wcut ? 1 : npl * wplane_size(N)))) return rc;
 
   // r_bubble is only written on the recombination branch: zero it once
   RG_CUDA_TRY(ctx, cudaMemsetAsync(g->r_bubble, 0, sizeof(float) * (size_t)N * N * N, st));
@@ -989,9 +1023,6 @@ int hii_snapshot(rg_context* ctx, const rg_params* p, const rg_snapshot* s, cons
     RG_CUDA_TRY(ctx, cudaMemcpyAsync(stg->host_r_bubble, g->r_bubble, sizeof(float) * (size_t)N * N * N,
                                      cudaMemcpyDeviceToHost, ctx->copy_stream));
   }
-  const int cb = hii_close_blocks(ctx, N);
-  double* partials = ensure_partials(ctx, std::max((size_t)cb * HII_NSUM, (size_t)4 * ctx->num_sms * REC_NSUM));
-  if (!partials) return set_error(ctx, RG_ENOMEM, "partials");
   const HiiState hs = hii_state(p, g, reinterpret_cast<uint8_t*>(ctx->bits));
 
   if ((rc = xy_ctrl_reset(ctx, (size_t)(N / 2 + 1) * kb, st))) return rc;
@@ -1087,10 +1118,11 @@ int hii_batch(rg_context* ctx, int nu, const rg_params* p, const rg_snapshot* s,
   const size_t nc = (size_t)(N / 2 + 1) * N * N, n3 = (size_t)N * N * N;
   const int nr = (int)sched.size();
   int kb = radius_batch(ctx, nc, ng, nr);
-  if ((rc = ensure_device(ctx, &ctx->spec, &ctx->spec_elems, nc * ng))) return rc;
-  if ((rc = ensure_work(ctx, nc, ng, &kb))) return rc;
-  // one state byte per cell of every unit
-  if ((rc = ensure_device(ctx, &ctx->bits, &ctx->bits_elems, (n3 * nu + 3) / 4))) return rc;
+  const int cb = hii_close_blocks(ctx, N);
+  int npl = 0;
+  if ((rc = hii_buffers(ctx, nc, ng, nr, nu, p[0].ReionFilterType != 1, (size_t)nu * cb * HII_NSUM, &kb, &npl)))
+    return rc;
+  double* partials = ctx->partials;
   if ((rc = ensure_device(ctx, &ctx->batch_sums, &ctx->batch_sums_elems, (size_t)32 * nu))) return rc;
   if ((size_t)nu > ctx->h_batch_sums_elems) {
     if (ctx->h_batch_sums) cudaFreeHost(ctx->h_batch_sums);
@@ -1108,13 +1140,8 @@ int hii_batch(rg_context* ctx, int nu, const rg_params* p, const rg_snapshot* s,
   if ((rc = hii_windows(ctx, &p[0], sched, st))) return rc;
   const int n2max = 3 * (N / 2) * (N / 2);
   const int* wcut = p[0].ReionFilterType == 1 ? ctx->wcut : nullptr;
-  const int npl = plane_radii(N, kb, nr);
-  if ((rc = ensure_device(ctx, &ctx->wplanes, &ctx->wplanes_elems, wcut ? 1 : npl * wplane_size(N)))) return rc;
   for (int u = 0; u < nu; ++u)
     RG_CUDA_TRY(ctx, cudaMemsetAsync(g[u].r_bubble, 0, sizeof(float) * n3, st));
-  const int cb = hii_close_blocks(ctx, N);
-  double* partials = ensure_partials(ctx, (size_t)nu * cb * HII_NSUM);
-  if (!partials) return set_error(ctx, RG_ENOMEM, "partials");
   std::vector<HiiState> hs(nu);
   for (int u = 0; u < nu; ++u)
     hs[u] = hii_state(&p[u], &g[u], reinterpret_cast<uint8_t*>(ctx->bits) + n3 * u);

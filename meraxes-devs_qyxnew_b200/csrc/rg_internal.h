@@ -93,7 +93,11 @@ int ensure_device(rg_context* ctx, T** ptr, size_t* have, size_t need) {
   *ptr = nullptr;
   *have = 0;
   const cudaError_t e = cudaMalloc((void**)ptr, sizeof(T) * (need ? need : 1));
-  if (e != cudaSuccess) return set_error(ctx, RG_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) {
+    *ptr = nullptr;
+    cudaGetLastError();   // reported here: the next launch's check is not to find it
+    return set_error(ctx, RG_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+  }
   *have = need;
   return RG_OK;
 }
@@ -204,6 +208,7 @@ struct rg_context {
   int N = 0;
   int mode = RG_MODE_FUSED;
   int radius_batch = 0;
+  size_t hii_fit = ~(size_t)0;   // elements of work that find_HII's buffers have found room for
   cudaStream_t own_stream = nullptr;
   cudaStream_t stream = nullptr;
   std::string last_error;

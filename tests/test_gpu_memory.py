@@ -1,0 +1,105 @@
+"""find_HII_bubbles on a device with little room: the radii go in smaller batches, with the same results;
+where not even one radius fits the call returns RG_ENOMEM and the context stays usable.
+
+The memory is taken by the test before the call (plain allocations that fail are errors of the API, not
+faults).  At 128^3 with two grids 16 radii take 273 MB, their windows 19 MB, the spectra 17 MB."""
+
+import numpy as np
+import pytest
+
+import rg_b200 as rg
+import test_gpu_hii_paths as tp
+import workloads as wl
+
+pytestmark = pytest.mark.gpu
+
+N, MB = 128, 1 << 20
+
+
+class Taken:
+    """All but `left` bytes of the device."""
+
+    def __init__(self, left):
+        import torch
+        self.torch = torch
+        self.parts = []
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        step = 1 << 36
+        while step >= 2 * MB:
+            if torch.cuda.mem_get_info()[0] - step < left:
+                step //= 2
+                continue
+            self.parts.append(torch.empty(step, dtype=torch.uint8, device="cuda"))
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        self.parts.clear()
+        self.torch.cuda.empty_cache()
+
+
+def call(ctx, dg, p):
+    import ctypes as C
+    zz, snap = wl.snapshot_redshifts(8.0)
+    s = rg.snapshot(zz, snap)
+    out = rg.rg_hii_scalars()
+    ctx.call("rg_find_HII_bubbles", C.byref(p), C.byref(s), C.byref(dg.g), C.byref(out))
+    return out
+
+
+def fresh(seed):
+    return tp.case(N, seed, False, False, False, 0)
+
+
+@pytest.mark.parametrize("left", [320 * MB, 294 * MB, 200 * MB, 64 * MB])
+def test_smaller_batches_give_the_same(left):
+    want, p = fresh(5)
+    ref = rg.Context(N)
+    o = call(ref, want, p)           # loads the kernels too
+    ref.close()
+    a, _ = fresh(5)
+    b, _ = fresh(5)
+    ctx = rg.Context(N)
+    with Taken(left):
+        got = [call(ctx, a, p), call(ctx, b, p)]     # the second with the size that fitted
+    ctx.close()
+    for dg, g in zip((a, b), got):
+        assert g.as_dict() == o.as_dict()
+        for k in tp.OUT:
+            assert np.array_equal(dg.get(k), want.get(k)), k
+
+
+def test_no_room_is_enomem_and_the_context_stays_usable():
+    want, p = fresh(6)
+    ref = rg.Context(N)
+    o = call(ref, want, p)
+    ref.close()
+    a, _ = fresh(6)
+    ctx = rg.Context(N)
+    with Taken(12 * MB):
+        with pytest.raises(rg.RGError) as e:
+            call(ctx, a, p)
+        assert e.value.status == rg.RG_ENOMEM
+    assert call(ctx, a, p).as_dict() == o.as_dict()
+    ctx.close()
+    for k in tp.OUT:
+        assert np.array_equal(a.get(k), want.get(k)), k
+
+
+def test_a_set_batch_that_does_not_fit_is_enomem():
+    want, p = fresh(7)
+    ref = rg.Context(N)
+    o = call(ref, want, p)
+    ref.close()
+    a, _ = fresh(7)
+    ctx = rg.Context(N)
+    ctx.call("rg_set_radius_batch", 16)
+    with Taken(200 * MB):
+        with pytest.raises(rg.RGError) as e:
+            call(ctx, a, p)
+        assert e.value.status == rg.RG_ENOMEM
+        ctx.call("rg_set_radius_batch", 4)
+        assert call(ctx, a, p).as_dict() == o.as_dict()
+    ctx.close()
