@@ -17,6 +17,8 @@
 namespace rg {
 
 int set_error(rg_context* ctx, int status, const std::string& msg) {
+  // a failed allocation is reported by this status: the next launch's check is not to find it again
+  if (status == RG_ENOMEM) cudaGetLastError();
   if (ctx) ctx->last_error = msg;
   return status;
 }
@@ -186,10 +188,7 @@ double* ensure_partials(rg_context* ctx, size_t n) {
   if (ctx->partials) cudaFree(ctx->partials);
   ctx->partials = nullptr;
   ctx->partials_elems = 0;
-  if (cudaMalloc((void**)&ctx->partials, sizeof(double) * n) != cudaSuccess) {
-    cudaGetLastError();   // reported by the caller: the next launch's check is not to find it
-    return ctx->partials = nullptr;
-  }
+  if (cudaMalloc((void**)&ctx->partials, sizeof(double) * n) != cudaSuccess) return ctx->partials = nullptr;
   ctx->partials_elems = n;
   return ctx->partials;
 }

@@ -95,7 +95,6 @@ int ensure_device(rg_context* ctx, T** ptr, size_t* have, size_t need) {
   const cudaError_t e = cudaMalloc((void**)ptr, sizeof(T) * (need ? need : 1));
   if (e != cudaSuccess) {
     *ptr = nullptr;
-    cudaGetLastError();   // reported here: the next launch's check is not to find it
     return set_error(ctx, RG_ENOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
   }
   *have = need;

@@ -103,3 +103,22 @@ def test_a_set_batch_that_does_not_fit_is_enomem():
         ctx.call("rg_set_radius_batch", 4)
         assert call(ctx, a, p).as_dict() == o.as_dict()
     ctx.close()
+
+
+def test_a_failed_allocation_does_not_reach_later_calls():
+    import ctypes as C
+
+    import torch
+    n = 32
+    p = rg.make_params(n, float(n), Flag_IncludeSpinTemp=1)
+    ctx = rg.Context(n)
+    g = rg.rg_grids()
+    with pytest.raises(rg.RGError) as e:
+        ctx.call("rg_alloc_grids", C.byref(p), 2_000_000, C.byref(g))    # 278 GB a history grid
+    assert e.value.status == rg.RG_ENOMEM
+    x = torch.ones(n * n * (n + 2), device="cuda")
+    y = torch.zeros_like(x)
+    torch.cuda.synchronize()
+    ctx.call("rg_debug_filter_roundtrip", C.byref(p), x.data_ptr(), y.data_ptr(), 3.0, -1)
+    ctx.close()
+    assert torch.allclose(y.view(n, n, n + 2)[:, :, :n], torch.ones(n, n, n, device="cuda"), atol=1e-5)
