@@ -17,27 +17,26 @@ N, MB = 128, 1 << 20
 
 
 class Taken:
-    """All but `left` bytes of the device."""
+    """All but `left` to `left` + 10 MB of the device."""
 
     def __init__(self, left):
-        import torch
-        self.torch = torch
-        self.parts = []
-        torch.cuda.synchronize()
-        torch.cuda.empty_cache()
-        step = 1 << 36
-        while step >= 2 * MB:
-            if torch.cuda.mem_get_info()[0] - step < left:
-                step //= 2
-                continue
-            self.parts.append(torch.empty(step, dtype=torch.uint8, device="cuda"))
+        self.left, self.parts = left, []
 
     def __enter__(self):
-        return self
+        import torch
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        while True:
+            # from 10 MB on a tensor is an allocation of its own, of its size in steps of 2 MB
+            size = min(1 << 36, (torch.cuda.mem_get_info()[0] - self.left) // (2 * MB) * (2 * MB))
+            if size < 10 * MB:
+                return self
+            self.parts.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
 
     def __exit__(self, *exc):
+        import torch
         self.parts.clear()
-        self.torch.cuda.empty_cache()
+        torch.cuda.empty_cache()
 
 
 def call(ctx, dg, p):
