@@ -46,11 +46,31 @@ int launch_inverse_xy(rg_context* ctx, const cf* spec, int ng, int ngu, cf* work
   if (ctx->mode == RG_MODE_FUSED) {
     if (stride != (size_t)C::NZ * N * N) return set_error(ctx, RG_EINVAL, "fused x/y pass: spectra must be contiguous");
     const double bytes = ng * 8.0 * nzc * (1 + nr);
-    // 96^3: the plan over 16 threads a line from 6 grids an item (several snapshots) on, 1.5 against 2.1
-    // ms for 12 grids; its smaller items cost more with the 2 or 3 grids of one (0.40 against 0.29 ms)
-    if constexpr (N == 96)
-      if (ng >= 6) return launch_xy_fused<N, PlanZ<N>>(ctx, op, spec, ng, nr, "inv_xy_c2c_window", bytes, st);
-    return launch_xy_fused<N, PlanW<N>>(ctx, op, spec, ng, nr, "inv_xy_c2c_window", bytes, st);
+#define RG_XY(PLAN, BL) launch_xy_fused<N, PLAN<N>, BL>(ctx, op, spec, ng, nr, "inv_xy_c2c_window", bytes, st)
+    // Where 3 divides N, the plan over more threads a line (PlanZ: 12 values a thread at most; PlanW: 24): always
+    // while its lines take up to 8 threads; with up to 32 (a warp) from 4 grids an item on, at three blocks
+    // an SM, which PlanW's registers do not allow (they spill); with 64, blocks of 512, never.  us for
+    // 2, 3, 4, 6, 12 grids an item, PlanW then PlanZ:
+    //   24^3    44 52 61 78 130        40 44 47 60 81
+    //   48^3    101 129 168 246 459    74 87 104 134 246
+    //   96^3    288 410 545 901 1909   330 425 524 720 1481   (at two blocks 405 509 616 827 1494)
+    //   192^3   1.84 2.72 4.78 7.92 16.4   2.61 3.44 4.30 6.09 12.4 (ms; 6 snapshots take the 12)
+    //   384^3   14.1 21.4 33.6 51.4 -      29.3 39.0 48.8 69.0 -   (ms)
+    if constexpr (N % 3 == 0 && PlanZ<N>::T <= 32) {
+      if constexpr (PlanZ<N>::T <= 8) return RG_XY(PlanZ, 2);
+      if (ng >= 4) return RG_XY(PlanZ, 3);
+    }
+    // Powers of two: three blocks an SM for 2 grids an item, two for more, whose planes in flight do not stay in
+    // L2 with the third.  us for 2, 3, 4, 6 grids, two blocks then three:
+    //   64^3    90 115 138 186         87 112 136 198
+    //   128^3   470 650 831 1304       474 653 832 1308
+    //   256^3   3.04 4.20 5.37 9.00    2.89 4.42 7.24 12.6 (ms)
+    //   512^3   31.6 44.7 - -          33.5 47.3 - -       (ms; its registers spill at three)
+    // (Smaller boxes have no blocks of 256 threads.)
+    if constexpr (N % 3 != 0 && PlanW<N>::T <= 16 && XYF<N, PlanW<N>, 2>::NTH == 256)
+      if (ng <= 2) return RG_XY(PlanW, 3);
+    return RG_XY(PlanW, 2);
+#undef RG_XY
   }
   if (ngu != ng) return set_error(ctx, RG_EINVAL, "several snapshots in one pass need the fused mode");
   return launch_win_xy<N>(ctx, op, spec, stride, ng, nr, st);

@@ -87,15 +87,14 @@ __device__ __forceinline__ void xy_wait(const XYSched& s, int job) {
 // The fused pass's plans (PlanW): at 512, 8 x 16 x 4 over 32 threads a line measured faster than
 // 8 x 8 x 8 over 64 (77.2 against 81.3 ms for the 61 radii of a 512^3 snapshot; 16 x 16 x 2 took
 // 78.5 ms, and 16 columns an item instead of 8 took 85-87 ms), and its Y lines are warp-local.
-template <int N, class Plan_>
+// BL: resident blocks of 256 threads an SM that the registers are to allow.
+template <int N, class Plan_, int BL>
 struct XYF {
   using PL = Plan_;
   static constexpr int T = PL::T;
   static constexpr int V = stage_rounds<PL, 0>() * PL::R[0];   // inputs of a thread
   static constexpr int B = pow2_div(N, cmax(256 / T, 8));      // columns per X item, lines per Y item
-  // three blocks an SM at 256 (2.95 against 3.17 ms for the 42 radii of a 256^3 snapshot), two where
-  // a block's registers or the planes in flight do not leave room for the third (512^3: 65.6, 67.9)
-  static constexpr int MINB = T * B >= 512 ? 1 : N == 256 ? 3 : RG_MINB(T * B);
+  static constexpr int MINB = T * B >= 512 ? 1 : BL * 256 / (T * B);
   static constexpr int NTH = T * B;
   static constexpr int M = N / B;
   static constexpr int XROWS = N <= 256 ? N : N / 2;   // x rows per tensor box (box dimensions <= 256)
@@ -127,10 +126,10 @@ __device__ __forceinline__ void xy_signal(uint32_t* p) {
 //   cf* out(int r, int g) const               output grid (plane kz at kz N^2)
 // The X input of grid g is W(k) * spectrum_g(k); the spectra are the tensor `smap` (floats, y
 // innermost, then x, then kz of grid g at g (N/2 + 1) + kz).
-template <int N, class PL_, class Op>
-__global__ void __launch_bounds__(XYF<N, PL_>::NTH, XYF<N, PL_>::MINB)
+template <int N, class PL_, int BL, class Op>
+__global__ void __launch_bounds__(XYF<N, PL_, BL>::NTH, XYF<N, PL_, BL>::MINB)
     k_xy_fused(XYSched sch, Op op, const __grid_constant__ CUtensorMap smap, const cf* __restrict__ g_tw) {
-  using F = XYF<N, PL_>;
+  using F = XYF<N, PL_, BL>;
   using PL = PL_;
   constexpr int T = F::T, B = F::B, V = F::V, TB = F::TB, NZ = N / 2 + 1, R0 = PL::R[0];
   extern __shared__ unsigned char smem_raw[];
@@ -269,10 +268,10 @@ __global__ void __launch_bounds__(XYF<N, PL_>::NTH, XYF<N, PL_>::MINB)
 
 // Launch the fused pass of one batch of nr radii (or shells); the control words must have been
 // sized by xy_ctrl_reset for at least (N/2 + 1) nr jobs.
-template <int N, class PL, class Op>
+template <int N, class PL, int BL, class Op>
 int launch_xy_fused(rg_context* ctx, const Op& op, const cf* spec, int nspec, int nr, const char* name,
                     double alg_bytes, cudaStream_t st) {
-  using F = XYF<N, PL>;
+  using F = XYF<N, PL, BL>;
   const cf* tw;
   int rc = twiddles_for(ctx, N, &tw);
   if (rc) return rc;
@@ -285,7 +284,7 @@ int launch_xy_fused(rg_context* ctx, const Op& op, const cf* spec, int nspec, in
   if (mrc != 0) return set_error(ctx, RG_ECUDA, "cuTensorMapEncodeTiled failed (" + std::to_string(mrc) + ")");
   const int J = Cfg<N>::NZ * nr;
   if (nr < 1 || (size_t)J + 2 > ctx->xy_ctrl_elems) return set_error(ctx, RG_EINVAL, "fused x/y pass: batch too large");
-  auto kern = k_xy_fused<N, PL, Op>;
+  auto kern = k_xy_fused<N, PL, BL, Op>;
   RG_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F::smem()));
   int per_sm = 0;
   RG_CUDA_TRY(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, F::NTH, F::smem()));
