@@ -543,12 +543,17 @@ struct TsZev {
   double inv_scale[4];            // undo the FP32 scaling
 };
 
-// Plans: at 128 and 256 the default ones, one exchange at 16 values a thread (three blocks of 128
-// threads, up to 168 registers), elsewhere 8 values a thread (two blocks of 256).  At 256^3 the z pass of
-// 40 shells and 9 nodes took 1.86 ms with 8 values a thread and two exchanges, 1.64 with one.
-template <int N>
+// LOOK: a pass with look-ups and sums per cell and shell (X-ray by shells, or AGN units).  It takes 8 values a
+// thread (two blocks of 256 threads); without (X-ray by nodes, no AGN) the default plan where that has one
+// exchange at 16 values a thread (128, 256; three blocks of 128 threads, up to 168 registers).  The passes over 40
+// shells, sharp-k or top-hat, us at 8 values a thread and in the one-exchange plan:
+//   by nodes            128^3, 4 nodes 195 190; 9 nodes 293 271     256^3, 2 nodes 1260 1140; 9 nodes 2129 1831
+//   by shells           128^3 303 315                               256^3 2358 2360; top-hat 2917 2848
+//   AGN, by nodes       128^3, 4 nodes 568 675                      256^3, 2 nodes 4277 4858; 9 nodes 5692 6040
+//   AGN, by shells      128^3 659 783                               256^3 5330 6011
+template <int N, bool LOOK>
 struct TsZ {
-  using PL = std::conditional_t<N == 128 || N == 256, Plan<N>, Plan8<N>>;
+  using PL = std::conditional_t<!LOOK && Plan<N>::S == 2 && N / Plan<N>::T == 16, Plan<N>, Plan8<N>>;
   static constexpr int T = PL::T;
   static constexpr int V = N / T;            // 8 or 16
   static constexpr int R0 = PL::R[0];
@@ -578,9 +583,8 @@ constexpr int TS_TMA_WAIT_LIMIT = 1 << 22;   // polls of an mbarrier before a wa
 
 // complex line of row q of the two spectra in a tile (a real part, b imaginary part), whose planes
 // beyond ka and kb are zero; the tile holds tile[s][k][j] = (s ? b : a)[k][x][y0 + j], b at TS
-template <int N, int Q>
+template <int N, int Q, int TS>
 __device__ __forceinline__ cf ts_tile_input(const cf* tile, int q, int p, int ka, int kb) {
-  constexpr int TS = TsZ<N>::TS;
   const int k = p <= N / 2 ? p : N - p;
   const cf A = k <= ka ? tile[k * Q + q] : cf{0.f, 0.f}, B = k <= kb ? tile[TS + k * Q + q] : cf{0.f, 0.f};
   if (p == 0 || p == N / 2) return cf{A.x, B.x};
@@ -595,11 +599,11 @@ __device__ __forceinline__ cf ts_tile_input(const cf* tile, int q, int p, int ka
 // innermost, then x, then kz of spectrum s at s (N/2 + 1) + kz), STAGES tiles in flight, one
 // mbarrier each; a spectrum's planes beyond its cut are not loaded.
 template <int N, bool XS, int NA>
-__global__ void __launch_bounds__(TsZ<N>::NTH, TsZ<N>::MINB)
+__global__ void __launch_bounds__((TsZ<N, XS || NA != 0>::NTH), (TsZ<N, XS || NA != 0>::MINB))
     k_ts_zsum(const __grid_constant__ CUtensorMap tmap, const cf* __restrict__ g_tw,
               const TsShellCoef* __restrict__ gco, TsZev zv, const float* __restrict__ xe_prev,
               float4* __restrict__ sums, float2* __restrict__ agn_heat, uint32_t* err) {
-  using Z = TsZ<N>;
+  using Z = TsZ<N, XS || NA != 0>;
   using PL = typename Z::PL;
   constexpr int Q = Z::Q, V = Z::V, NZ = Z::NZ;
   constexpr int G = 1 + XS + NA;
@@ -708,7 +712,7 @@ __global__ void __launch_bounds__(TsZ<N>::NTH, TsZ<N>::MINB)
   // the unit in work
   const cf* tile = tiles;
   int sp[2] = {0, 0}, kl[2] = {0, 0};
-  auto input = [&](int p, int) { return ts_tile_input<N, Q>(tile, q, p, kl[0], kl[1]); };
+  auto input = [&](int p, int) { return ts_tile_input<N, Q, Z::TS>(tile, q, p, kl[0], kl[1]); };
   // an AGN unit j: clamped at 0 (ComputeTs.c:615-630), its own band tables
   auto agn_unit = [&](int j, float (&ah)[NA > 0 ? V : 1]) {
     line_fft_p<PL, true>(
@@ -1081,7 +1085,7 @@ static int launch_ts_zsum_g(rg_context* ctx, const cf* work, size_t stride, cons
   const cf* tw;
   int rc = twiddles_for(ctx, N, &tw);
   if (rc) return rc;
-  using Z = TsZ<N>;
+  using Z = TsZ<N, XS || NA != 0>;
   const double n3 = (double)N * N * N;
   if (stride != (size_t)Z::NZ * N * N) return set_error(ctx, RG_EINVAL, "Ts z pass: shell spectra must be contiguous");
   // every spectrum (S[kz][x][y], one after another) as a 3-D float tensor
