@@ -36,6 +36,19 @@ __device__ __forceinline__ bool sharpk_zero(double delta_k, int n2, double R) {
   return kR * 0.413566994 > 1.0;
 }
 
+__device__ __forceinline__ float window_value(double delta_k, int n2, double R, int ftype) {
+  if (ftype == 1) return sharpk_zero(delta_k, n2, R) ? 0.f : 1.f;
+  const double kR = delta_k * sqrt((double)n2) * R;
+  double w = 1.0;
+  if (ftype == 0) {
+    if (kR > 1e-4) w = 3.0 * (sin(kR) / (kR * kR * kR) - cos(kR) / (kR * kR));
+  } else {
+    const double g = kR * 0.643;
+    w = exp(-g * g / 2.0);
+  }
+  return (float)w;
+}
+
 // For the sharp-k filter (ftype 1) the row is a step in n2 (kR grows with n2); wcut[r], when
 // given, receives the last n2 of the step (written by that entry alone), so
 // W[r][n2] == (n2 <= wcut[r]).
@@ -45,18 +58,9 @@ __global__ void k_window_table(float* wtab, int n2max, const double* __restrict_
   if (r >= nr) return;
   const double R = radii[r];
   for (int n2 = blockIdx.x * blockDim.x + threadIdx.x; n2 <= n2max; n2 += gridDim.x * blockDim.x) {
-    const double kR = delta_k * sqrt((double)n2) * R;
-    double w = 1.0;
-    if (ftype == 0) {
-      if (kR > 1e-4) w = 3.0 * (sin(kR) / (kR * kR * kR) - cos(kR) / (kR * kR));
-    } else if (ftype == 1) {
-      if (sharpk_zero(delta_k, n2, R)) w = 0.0;
-    } else {
-      const double g = kR * 0.643;
-      w = exp(-g * g / 2.0);
-    }
-    wtab[(size_t)r * (n2max + 1) + n2] = (float)w;
-    if (ftype == 1 && wcut && w == 1.0 && (n2 == n2max || sharpk_zero(delta_k, n2 + 1, R))) wcut[r] = n2;
+    const float w = window_value(delta_k, n2, R, ftype);
+    wtab[(size_t)r * (n2max + 1) + n2] = w;
+    if (ftype == 1 && wcut && w == 1.f && (n2 == n2max || sharpk_zero(delta_k, n2 + 1, R))) wcut[r] = n2;
   }
 }
 
@@ -77,6 +81,20 @@ __global__ void __launch_bounds__(256) k_window_planes(const float* __restrict__
       out[((size_t)kz * h + nx) * wp + ny] = w;
       out[((size_t)nx * h + kz) * wp + ny] = w;
     }
+}
+
+// The plane of one radius by itself (rg_smooth_grid), each value evaluated where it goes: the table and its
+// gather are a launch more, about 6 us of a 64^3 call's 60.  smooth_grid, us with window rows gathered in the x/y
+// pass, and so: 64^3 60, 55; 128^3 75, 70; 256^3 223, 214; 512^3 1722, 1635.
+__global__ void __launch_bounds__(64) k_window_plane(double delta_k, double R, int ftype, int n,
+                                                     float* __restrict__ plane) {
+  const int h = n / 2 + 1, wp = wplane_pitch(n), kz = blockIdx.x, nx = blockIdx.y;
+  if (nx < kz) return;
+  for (int ny = threadIdx.x; ny < h; ny += 64) {
+    const float w = window_value(delta_k, kz * kz + nx * nx + ny * ny, R, ftype);
+    plane[((size_t)kz * h + nx) * wp + ny] = w;
+    plane[((size_t)nx * h + kz) * wp + ny] = w;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1209,13 +1227,11 @@ int debug_roundtrip(rg_context* ctx, const rg_params* p, const float* d_in, floa
   if ((rc = fft_forward(ctx, N, srcs, 1, ctx->spec, nc, 1.0 / std::pow((double)N, 3), st))) return rc;
   const float* wplane = nullptr;
   if (ftype >= 0) {
-    const int n2max = 3 * (N / 2) * (N / 2);
-    if ((rc = ensure_device(ctx, &ctx->d_radii, &ctx->d_radii_elems, 1))) return rc;
-    RG_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->d_radii, &R, sizeof(double), cudaMemcpyHostToDevice, st));
-    if ((rc = ensure_device(ctx, &ctx->wtab, &ctx->wtab_elems, (size_t)(n2max + 1)))) return rc;
-    if ((rc = window_table(ctx, p->BoxSize, ctx->d_radii, 1, ftype, ctx->wtab, n2max, st))) return rc;
     if ((rc = ensure_device(ctx, &ctx->wplanes, &ctx->wplanes_elems, wplane_size(N)))) return rc;
-    if ((rc = window_planes(ctx, N, ctx->wtab, 1, ctx->wplanes, st))) return rc;
+    prof_begin(ctx, "window_planes", st);
+    k_window_plane<<<dim3(N / 2 + 1, N / 2 + 1), 64, 0, st>>>(2.0 * M_PI / p->BoxSize, R, ftype, N, ctx->wplanes);
+    prof_end(ctx, 4.0 * wplane_size(N), st);
+    RG_CUDA_TRY(ctx, cudaGetLastError());
     wplane = ctx->wplanes;
   }
   if ((rc = debug_inverse(ctx, N, wplane, d_out, st))) return rc;
