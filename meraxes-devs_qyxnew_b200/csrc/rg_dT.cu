@@ -90,7 +90,9 @@ int delta_T_launch(rg_context* ctx, int n, const float* xH, const float* deltax,
 // peculiar velocities (BrightnessTemperature.c:150-509): with the spin temperature,
 // Flag_IncludePecVelsFor21cm 1 caps the velocity gradient (the 21cmFAST treatment), 2 uses the
 // optical-depth form with the uncapped gradient, 3 adds the line-of-sight re-binning of 50
-// sub-cells per cell (Greig & Mesinger 2018).  Every float/double step is the reference's.
+// sub-cells per cell (Greig & Mesinger 2018).  The values are floats where the reference's are, and each
+// step is taken in double as there, with products by reciprocals in place of its divisions by constants
+// (an ulp of double) and the re-binning in closed form (k_rsd).
 
 // velocity in the tree code's units -> comoving velocity (BrightnessTemperature.c:173-196); the
 // padding of each row is not touched (the r2c transform ignores it).  f0 is the factor of the tree

@@ -5,11 +5,12 @@
 //   x and y passes (rg_hii_xy.cu) into KB x G work grids
 //   z pass : per block of rows, for each radius of the batch in order: c2r of the G grids, then the
 //            aliasing clamp and the barrier test per cell (k_hii_zr in rg_hii_z.cuh; here the
-//            row-buffer form for Pop III sources, k_hii_z).
-// Until the last radius the per-cell state is two bits (ionized this snapshot; z_at_ionization
-// still < 0), kept in registers within a batch and in one byte per cell between batches;
-// z_at_ionization and J_21 are written only where a cell first ionizes.  The last radius also
-// computes the partial xH and runs the closing pass (temperatures and FP64 global sums).
+//            row-buffer form for Pop III sources and the boxes below 64^3, k_hii_z).
+// A cell's state over the radii is two bits (ionized this snapshot; z_at_ionization still < 0), kept in
+// registers within a batch; between batches k_hii_zr keeps them as two words a thread, k_hii_z as a
+// byte per cell.  z_at_ionization and J_21 are written only where a cell first ionizes.  The last radius
+// also writes xH, with the sign of "neutral at every radius"; the closing pass (k_hii_close) then takes
+// xH and the temperatures to their final values and sums the box averages in FP64.
 #include <cuda_runtime.h>
 #include <math.h>
 
@@ -51,7 +52,7 @@ __device__ __forceinline__ float window_value(double delta_k, int n2, double R, 
 
 // For the sharp-k filter (ftype 1) the row is a step in n2 (kR grows with n2); wcut[r], when
 // given, receives the last n2 of the step (written by that entry alone), so
-// W[r][n2] == (n2 <= wcut[r]).
+// W[r][n2] == (n2 <= wcut[r]), and the row is not written.
 __global__ void k_window_table(float* wtab, int n2max, const double* __restrict__ radii, int nr, double delta_k,
                                int ftype, int* wcut) {
   const int r = blockIdx.y;
@@ -59,8 +60,11 @@ __global__ void k_window_table(float* wtab, int n2max, const double* __restrict_
   const double R = radii[r];
   for (int n2 = blockIdx.x * blockDim.x + threadIdx.x; n2 <= n2max; n2 += gridDim.x * blockDim.x) {
     const float w = window_value(delta_k, n2, R, ftype);
-    wtab[(size_t)r * (n2max + 1) + n2] = w;
-    if (ftype == 1 && wcut && w == 1.f && (n2 == n2max || sharpk_zero(delta_k, n2 + 1, R))) wcut[r] = n2;
+    if (ftype != 1 || !wcut) {
+      wtab[(size_t)r * (n2max + 1) + n2] = w;
+    } else if (w == 1.f && (n2 == n2max || sharpk_zero(delta_k, n2 + 1, R))) {
+      wcut[r] = n2;
+    }
   }
 }
 
@@ -99,13 +103,6 @@ __global__ void __launch_bounds__(64) k_window_plane(double delta_k, double R, i
 
 // ---------------------------------------------------------------------------
 // temperatures
-
-__device__ __forceinline__ float partial_T(float t_hi, float res_xh) {
-  // ComputePartiallyIoinizedTemperature (find_HII_bubbles.c:76-84)
-  if (res_xh <= 0.f) return (float)T_RE;
-  if (res_xh >= 1.f) return t_hi;
-  return (float)((double)(t_hi * res_xh) + T_RE * (1.0 - (double)res_xh));
-}
 
 // ComputeFullyIoinizedTemperature (find_HII_bubbles.c:48-74), with its float/double mix.  The powers
 // of constants and of the redshift alone come from the host (HiiConst); the per-cell ones are

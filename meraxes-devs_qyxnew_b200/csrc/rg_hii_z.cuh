@@ -19,7 +19,7 @@ struct HiiBatch {
   int nr;             // radii in this batch
   int first;          // the batch starts the snapshot (state comes from z_at_ionization)
   int last;           // the batch ends with the snapshot's last (unfiltered) radius
-  int ng;             // grids per radius (read by the instantiation for 5 to 7 grids)
+  int ng;             // grids per radius (k_hii_zr and the plain forms of k_hii_z know it at compile time)
   double fcoll_pref[KB_MAX];
   float J_aux[KB_MAX], J_aux_bh[KB_MAX];
   float G_pref[KB_MAX], G_pref_bh[KB_MAX], R[KB_MAX];   // recombination branch
