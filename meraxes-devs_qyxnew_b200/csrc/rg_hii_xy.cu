@@ -49,16 +49,19 @@ int launch_inverse_xy(rg_context* ctx, const cf* spec, int ng, int ngu, cf* work
 #define RG_XY(PLAN, BL) launch_xy_fused<N, PLAN<N>, BL>(ctx, op, spec, ng, nr, "inv_xy_c2c_window", bytes, st)
     // Where 3 divides N, the plan over more threads a line (PlanZ: 12 values a thread at most; PlanW: 24): always
     // while its lines take up to 8 threads; with up to 32 (a warp) from 4 grids an item on, at three blocks
-    // an SM, which PlanW's registers do not allow (they spill); with 64, blocks of 512, never.  us for
-    // 2, 3, 4, 6, 12 grids an item, PlanW then PlanZ:
-    //   24^3    44 52 61 78 130        40 44 47 60 81
-    //   48^3    101 129 168 246 459    74 87 104 134 246
-    //   96^3    288 410 545 901 1909   330 425 524 720 1481   (at two blocks 405 509 616 827 1494)
-    //   192^3   1.84 2.72 4.78 7.92 16.4   2.61 3.44 4.30 6.09 12.4 (ms; 6 snapshots take the 12)
-    //   384^3   14.1 21.4 33.6 51.4 -      29.3 39.0 48.8 69.0 -   (ms)
+    // an SM (PlanW's registers spill there), or two where the planes that three have in flight would not stay
+    // in L2; with 64, blocks of 512, never.  2, 3, 4, 6, 8, 12 grids an item, PlanW then PlanZ:
+    //   24^3    44 52 61 78 94 130          40 44 47 60 65 81 us
+    //   48^3    101 129 168 246 323 459     74 87 104 134 167 246 us
+    //   96^3    288 410 545 901 1225 1909   at two blocks 405 509 616 827 1042 1494, at three 330 425 524 720 939 1481 us
+    //   192^3   1.84 2.72 4.78 7.92 10.8 16.4   3.14 4.01 4.89 6.67 8.50 12.3, 2.61 3.44 4.30 6.09 8.05 12.4 ms
+    //   384^3   14.1 21.4 33.6 51.4         29.3 39.0 48.8 69.0 ms
+    // and with the sharp-k window, 8 and 12 grids at two and three blocks: 96^3 983 902, 1432 1489 us; 192^3 8.07 7.85,
+    // 11.8 12.8 ms.
     if constexpr (N % 3 == 0 && PlanZ<N>::T <= 32) {
       if constexpr (PlanZ<N>::T <= 8) return RG_XY(PlanZ, 2);
-      if (ng >= 4) return RG_XY(PlanZ, 3);
+      if (ng >= 4)
+        return xy_least_planes<N, PlanZ<N>, 3>(ctx, ng) <= XY_PLANES ? RG_XY(PlanZ, 3) : RG_XY(PlanZ, 2);
     }
     // Powers of two: three blocks an SM for 2 grids an item, two for more, whose planes in flight do not stay in
     // L2 with the third.  us for 2, 3, 4, 6 grids, two blocks then three:

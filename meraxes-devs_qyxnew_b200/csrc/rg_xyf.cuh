@@ -266,6 +266,19 @@ __global__ void __launch_bounds__(XYF<N, PL_, BL>::NTH, XYF<N, PL_, BL>::MINB)
   if (!waited && threadIdx.x % 32 == 0) atomicExch(sch.err, 1u);
 }
 
+// bytes of planes in flight that stay in L2 (written by X, read and written by Y: half of it)
+constexpr size_t XY_PLANES = 64u << 20;
+
+// the lag at which Y(j) is handed out about when X(j) completes, with `grid` blocks in flight
+template <class F>
+int xy_lag(int grid) { return (grid + 2 * F::M - 1) / (2 * F::M); }
+
+// bytes of planes that BL blocks an SM have in flight at the least lag, ng grids an item
+template <int N, class PL, int BL>
+size_t xy_least_planes(const rg_context* ctx, int ng) {
+  return 2 * (size_t)(xy_lag<XYF<N, PL, BL>>(BL * ctx->num_sms) + 1) * sizeof(cf) * N * N * ng;
+}
+
 // Launch the fused pass of one batch of nr radii (or shells); the control words must have been
 // sized by xy_ctrl_reset for at least (N/2 + 1) nr jobs.
 template <int N, class PL, int BL, class Op>
@@ -298,9 +311,9 @@ int launch_xy_fused(rg_context* ctx, const Op& op, const cf* spec, int nspec, in
   // the 2L planes written in between (64 MB of them: a plane is written by X, read and written by Y)
   // stay in L2.  Measured (ms of a snapshot's passes) at L = grid / (2M), 1.5, 2 and 3 times that:
   // 192^3 3.50, 2.83, 2.91, 3.29; 256^3 3.47, 3.04, 2.95, 3.03; 512^3 65.6, 65.8, 66.7, 70.4.
-  const int base = (grid + 2 * F::M - 1) / (2 * F::M);
+  const int base = xy_lag<F>(grid);
   const size_t job_bytes = sizeof(cf) * (size_t)N * N * op.ng;
-  s.L = std::min(J, std::max(base + 1, std::min(2 * base + 1, (int)((64u << 20) / (2 * job_bytes)))));
+  s.L = std::min(J, std::max(base + 1, std::min(2 * base + 1, (int)(XY_PLANES / (2 * job_bytes)))));
   // a batch that does not stay in L2 until its z pass leaves by evict-first stores: its finished planes
   // go before the ones that Y items still read (192^3: 3.31 -> 2.83 ms)
   s.stream = (size_t)J * job_bytes > (48u << 20);
