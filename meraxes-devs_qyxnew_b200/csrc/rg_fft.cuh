@@ -186,6 +186,7 @@ RG_PLAN(Plan8, 512, 64, 8, 8, 8)
 // the z pass of find_HII_bubbles, which keeps every grid's values of a thread in registers: the
 // default plans' stages (the same arithmetic), over more threads where 3 divides N, so that a thread
 // ends with 6 values instead of 24.  A quarter of the threads idle in the radix-8 stages.
+// (The fused x/y pass takes them too, by the rule in rg_hii_xy.cu.)
 template <int N>
 struct PlanZ : Plan<N> {};
 RG_PLAN(PlanZ, 24, 4, 8, 3)
