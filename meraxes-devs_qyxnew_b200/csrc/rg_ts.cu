@@ -543,17 +543,19 @@ struct TsZev {
   double inv_scale[4];            // undo the FP32 scaling
 };
 
-// LOOK: a pass with look-ups and sums per cell and shell (X-ray by shells, or AGN units).  It takes 8 values a
-// thread (two blocks of 256 threads); without (X-ray by nodes, no AGN) the default plan where that has one
-// exchange at 16 values a thread (128, 256; three blocks of 128 threads, up to 168 registers).  The passes over 40
-// shells, sharp-k or top-hat, us at 8 values a thread and in the one-exchange plan:
-//   by nodes            128^3, 4 nodes 195 190; 9 nodes 293 271     256^3, 2 nodes 1260 1140; 9 nodes 2129 1831
-//   by shells           128^3 303 315                               256^3 2358 2360; top-hat 2917 2848
-//   AGN, by nodes       128^3, 4 nodes 568 675                      256^3, 2 nodes 4277 4858; 9 nodes 5692 6040
-//   AGN, by shells      128^3 659 783                               256^3 5330 6011
-template <int N, bool LOOK>
+// LOOK: the pass's look-ups and sums per cell and shell: 0 none (X-ray by nodes, no AGN), 1 X-ray by shells, 2 AGN
+// units. The default plan has one exchange at 16 values a thread at 128 and 256 (three blocks of 128
+// threads, up to 168 registers); it is taken without look-ups, and by shells where a line takes 16 threads (256).
+// Else 8 values a thread (two blocks of 256).  The passes over 40 shells, sharp-k unless it says top-hat, us at 8
+// values a thread and in the one-exchange plan:
+//   by nodes            128^3, 4 nodes 195 190; top-hat, 9 nodes 293 271     256^3, 2 nodes 1260 1140; top-hat, 9 2129 1831
+//   by shells           128^3 303 315                                        256^3 2358 2360; top-hat 2917 2848
+//   AGN, by nodes       128^3, 4 nodes 568 675                               256^3, 2 nodes 4277 4858; top-hat, 9 5692 6040
+//   AGN, by shells      128^3 659 783                                        256^3 5330 6011
+template <int N, int LOOK>
 struct TsZ {
-  using PL = std::conditional_t<!LOOK && Plan<N>::S == 2 && N / Plan<N>::T == 16, Plan<N>, Plan8<N>>;
+  static constexpr bool ONE = Plan<N>::S == 2 && N / Plan<N>::T == 16 && (LOOK == 0 || (LOOK == 1 && Plan<N>::T >= 16));
+  using PL = std::conditional_t<ONE, Plan<N>, Plan8<N>>;
   static constexpr int T = PL::T;
   static constexpr int V = N / T;            // 8 or 16
   static constexpr int R0 = PL::R[0];
@@ -599,11 +601,11 @@ __device__ __forceinline__ cf ts_tile_input(const cf* tile, int q, int p, int ka
 // innermost, then x, then kz of spectrum s at s (N/2 + 1) + kz), STAGES tiles in flight, one
 // mbarrier each; a spectrum's planes beyond its cut are not loaded.
 template <int N, bool XS, int NA>
-__global__ void __launch_bounds__((TsZ<N, XS || NA != 0>::NTH), (TsZ<N, XS || NA != 0>::MINB))
+__global__ void __launch_bounds__((TsZ<N, NA != 0 ? 2 : XS>::NTH), (TsZ<N, NA != 0 ? 2 : XS>::MINB))
     k_ts_zsum(const __grid_constant__ CUtensorMap tmap, const cf* __restrict__ g_tw,
               const TsShellCoef* __restrict__ gco, TsZev zv, const float* __restrict__ xe_prev,
               float4* __restrict__ sums, float2* __restrict__ agn_heat, uint32_t* err) {
-  using Z = TsZ<N, XS || NA != 0>;
+  using Z = TsZ<N, NA != 0 ? 2 : XS>;
   using PL = typename Z::PL;
   constexpr int Q = Z::Q, V = Z::V, NZ = Z::NZ;
   constexpr int G = 1 + XS + NA;
@@ -1085,7 +1087,7 @@ static int launch_ts_zsum_g(rg_context* ctx, const cf* work, size_t stride, cons
   const cf* tw;
   int rc = twiddles_for(ctx, N, &tw);
   if (rc) return rc;
-  using Z = TsZ<N, XS || NA != 0>;
+  using Z = TsZ<N, NA != 0 ? 2 : XS>;
   const double n3 = (double)N * N * N;
   if (stride != (size_t)Z::NZ * N * N) return set_error(ctx, RG_EINVAL, "Ts z pass: shell spectra must be contiguous");
   // every spectrum (S[kz][x][y], one after another) as a 3-D float tensor

@@ -1,5 +1,5 @@
-"""The two plans of ComputeTs' z pass at 128^3, with the X-ray sums by nodes and by shells, with and without AGN
-bands, against the oracle.  The 128^3 box is an 8^3 field repeated 16 times, whose result is the 8^3 one
+"""The two plans of ComputeTs' z pass, with the X-ray sums by nodes and by shells, with and without AGN
+bands, against the oracle.  The box is an 8^3 field repeated 16 (32) times, whose result is the 8^3 one
 repeated (test_gpu_tiled.py); tolerances as there (1e-5)."""
 
 from types import SimpleNamespace
@@ -21,11 +21,10 @@ def ts_tables():
     return to.TsTables()
 
 
-@pytest.mark.parametrize("nodes,flag", [(3, 0), (0, 0), (3, 1), (0, 1)])
-def test_z_pass_plans_at_128(ts_tables, nodes, flag):
-    """128^3 as an 8^3 field repeated 16 times (test_gpu_tiled.py): by nodes without AGN bands the
-    one-exchange plan, else the one of 8 values a thread."""
-    n, reps = 8, 16
+# the one-exchange plan by nodes without AGN bands, and by shells at 256^3; else 8 values a thread
+@pytest.mark.parametrize("reps,nodes,flag", [(16, 3, 0), (16, 0, 0), (16, 3, 1), (16, 0, 1), (32, 0, 0)])
+def test_z_pass_plans(ts_tables, reps, nodes, flag):
+    n = 8
     zz, idx = wl.snapshot_redshifts(15.0)
     src = wl.make_sources(n, 8.0, 1300)
     ti = wl.make_ts_inputs(src, zz, idx, 16, 1301)
