@@ -974,6 +974,7 @@ static int hii_buffers(rg_context* ctx, size_t nc, int ng, int nr, int nu, bool 
     *elems = 0;
   };
   int rc;
+  const size_t fitted = ctx->hii_fit;
   if (ctx->radius_batch > 0 && (rc = ensure_device(ctx, &ctx->work, &ctx->work_elems, nc * ng * *kb))) return rc;
   for (;;) {
     *npl = plane_radii(N, *kb, nr);
@@ -982,6 +983,7 @@ static int hii_buffers(rg_context* ctx, size_t nc, int ng, int nr, int nu, bool 
       *npl = *kb;
       rc = all();
     }
+    if (rc == RG_ENOMEM && *kb == 1) ctx->hii_fit = fitted;   // nothing fitted: a later call tries anew
     if (rc != RG_ENOMEM || *kb == 1) return rc;
     release(&ctx->work, &ctx->work_elems);
     release(&ctx->wplanes, &ctx->wplanes_elems);

@@ -81,8 +81,12 @@ def test_no_room_is_enomem_and_the_context_stays_usable():
         with pytest.raises(rg.RGError) as e:
             call(ctx, a, p)
         assert e.value.status == rg.RG_ENOMEM
+    ctx.profile(True)
     assert call(ctx, a, p).as_dict() == o.as_dict()
+    # with the default batch again, not one that was tried where nothing fitted
+    passes = {s["name"]: s["launches"] for s in ctx.kernel_stats()}["inv_xy_c2c_window"]
     ctx.close()
+    assert passes == -(-o.n_radii // 16)
     for k in tp.OUT:
         assert np.array_equal(a.get(k), want.get(k)), k
 
